@@ -3,6 +3,7 @@
 // stream and scratch; handles are independent (the reference keeps its diagonal
 // buckets and U3 descriptors in process-global statics, kernel_cuda.cu:91-142).
 #include "../../include/zxh_b200.h"
+#include "permute.h"
 #include "sim.h"
 
 #include <cuda_runtime.h>
@@ -648,15 +649,18 @@ static int state_to_device(zxh_sim *s, void *dst, int order)
     const int N = int(s->n);
     const uint64_t nv = 1ULL << N;
     if (s->ws.m < N) CK(s, cudaMemsetAsync(dst, 0, size_t(nv) * size_t(s->elem_bytes), s->stream), "zero state");
-    static thread_local uint64_t tab[8][256];
-    column_tables(s->ws.map, tab);
-    void *dtab = nullptr;
-    CK(s, cudaMallocAsync(&dtab, sizeof(tab), s->stream), "cudaMallocAsync(table)");
-    CK(s, cudaMemcpyAsync(dtab, tab, sizeof(tab), cudaMemcpyHostToDevice, s->stream), "upload table");
-    CK(s, zxh::run_scatter(s->d_state, 1ULL << s->ws.m, static_cast<uint64_t *>(dtab), s->ws.map.b(), N, order,
-                           s->ws.gphase.real(), s->ws.gphase.imag(), dst, s->elem_bytes, s->sms, s->stream),
-       "scatter");
-    CK(s, cudaFreeAsync(dtab, s->stream), "cudaFreeAsync(table)");
+    // columns of the map, rows reversed for the reference's order
+    zxh::PermCols cols = {};
+    const zxh::AffineMap &A = s->ws.map;
+    auto place = [&](int q) { return order == ZXH_ORDER_REFERENCE ? N - 1 - q : q; };
+    cols.m = s->ws.m;
+    for (int q = 0; q < N; q++) {
+        for (int j = 0; j < cols.m; j++) cols.col[j] |= ((A.row(q) >> j) & 1) << place(q);
+        cols.b |= ((A.b() >> q) & 1) << place(q);
+    }
+    CK(s, zxh::run_permute(s->d_state, cols, s->ws.gphase.real(), s->ws.gphase.imag(), dst, s->elem_bytes, s->sms,
+                           s->stream),
+       "get_state");
     return ZXH_OK;
 }
 

@@ -12,8 +12,6 @@
 //                   stores it back once. Replaces u3_block_batch_kernel_cuda (one grid
 //                   sweep per descriptor, kernel_cuda.cu:390-423) and
 //                   diag_block_kernel_cuda (kernel_cuda.cu:505-614).
-//   scatter_kernel  get_state: real -> virtual index, bit reversal, global phase
-//                   (zxh.cpp:579-636).
 #include "core.h"
 #include "dev.cuh"
 #include "host.h"
@@ -457,32 +455,6 @@ __global__ void __launch_bounds__(kThreads) tile_kernel(const uint8_t *__restric
 }
 
 // ---------------------------------------------------------------------------
-// get_state scatter
-
-template <typename E>
-__global__ void __launch_bounds__(kThreads) scatter_kernel(const E *__restrict__ state, uint64_t n_real,
-                                                           const uint64_t *__restrict__ coltab, uint64_t b, int N,
-                                                           int order, double gre, double gim, E *__restrict__ out)
-{
-    using R = typename ET<E>::R;
-    __shared__ uint64_t tab[8][256];
-    for (int i = threadIdx.x; i < 8 * 256; i += kThreads) tab[i >> 8][i & 255] = coltab[i];
-    __syncthreads();
-    const R gr = R(gre), gi = R(gim);
-    for (uint64_t r = uint64_t(blockIdx.x) * kThreads + threadIdx.x; r < n_real; r += uint64_t(gridDim.x) * kThreads) {
-        uint64_t v = b;
-#pragma unroll
-        for (int k = 0; k < 8; k++) v ^= tab[k][(r >> (8 * k)) & 255];
-        const uint64_t idx = order == 0 ? (__brevll(v) >> (64 - N)) : v;
-        const E a = state[r];
-        E o;
-        o.x = a.x * gr - a.y * gi;
-        o.y = a.x * gi + a.y * gr;
-        out[idx] = o;
-    }
-}
-
-// ---------------------------------------------------------------------------
 // launchers
 
 template <typename E>
@@ -590,20 +562,6 @@ cudaError_t run_passes(const std::vector<Pass> &passes, const uint8_t *dblob, vo
         kernels++;
     }
     return cudaSuccess;
-}
-
-cudaError_t run_scatter(const void *state, uint64_t n_real, const uint64_t *dcoltab, uint64_t b, int N, int order,
-                        double gre, double gim, void *out, int elem_bytes, int sms, cudaStream_t st)
-{
-    const unsigned grid = unsigned(std::max<uint64_t>(1, std::min<uint64_t>((n_real + kThreads - 1) / kThreads,
-                                                                            uint64_t(sms) * 16)));
-    if (elem_bytes == 8)
-        scatter_kernel<float2><<<grid, kThreads, 0, st>>>(static_cast<const float2 *>(state), n_real, dcoltab, b, N,
-                                                          order, gre, gim, static_cast<float2 *>(out));
-    else
-        scatter_kernel<double2><<<grid, kThreads, 0, st>>>(static_cast<const double2 *>(state), n_real, dcoltab, b, N,
-                                                           order, gre, gim, static_cast<double2 *>(out));
-    return cudaGetLastError();
 }
 
 }  // namespace zxh

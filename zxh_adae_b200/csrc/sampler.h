@@ -89,7 +89,5 @@ cudaError_t run_grow(const uint8_t *dblob, uint64_t poff, uint64_t toff, int R, 
 int grow_reg_bits(int elem_bytes, bool adjoint);
 int grow_fixed_bits(int elem_bytes);
 int grow_adjoint_gates();
-cudaError_t run_scatter(const void *state, uint64_t n_real, const uint64_t *dcoltab, uint64_t b, int N, int order,
-                        double gre, double gim, void *out, int elem_bytes, int sms, cudaStream_t st);
 
 }  // namespace zxh
