@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <vector>
 
 namespace zxh {
 
@@ -47,6 +48,23 @@ struct AdjDiagGate {
 // <psi|H|psi> to *energy.
 cudaError_t run_lambda(const void *psi, void *lam, int m, int elem_bytes, const TermDev *dterms, uint32_t nterms,
                        double *energy, int sms, cudaStream_t st);
+
+// One pass of the tiled form (lambda_tile.cu): the tile's basis vectors, the flips it
+// applies (coordinate k of xmask, coefficient xc[k]), the real vectors of the tile bits,
+// and in the first pass the Z / ZZ terms diag0 .. diag0 + nd, sorted by the parity of
+// their masks with basis[4..7] (part g is goff[g] .. goff[g + 1]).
+struct LamPassDev {
+    uint64_t ntiles;
+    uint64_t basis[12], tr[64];
+    double xc[12];
+    uint32_t xmask, nd, diag0, goff[17];
+};
+// Passes for H over 2^m amplitudes, none below 2^12 (run_lambda then). Reorders the Z and
+// ZZ terms; call it before the terms are uploaded.
+std::vector<LamPassDev> plan_lambda(std::vector<TermDev> &terms, int m);
+// run_lambda by the planned passes.
+cudaError_t run_lambda_tiles(const void *psi, void *lam, int elem_bytes, const std::vector<LamPassDev> &passes,
+                             const TermDev *dterms, double *energy, int sms, cudaStream_t st);
 // Adds Im<lam|G|psi> to *grad (gen != 0), then psi <- U^dagger psi, lam <- U^dagger lam.
 cudaError_t run_adj_pair(void *psi, void *lam, int elem_bytes, const AdjPairDev &g, double *grad, int sms,
                          cudaStream_t st);

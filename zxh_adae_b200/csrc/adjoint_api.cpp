@@ -259,6 +259,14 @@ int forward_segments(zxh_sim *s, const std::vector<size_t> &ends, double &ms, ui
     return ZXH_OK;
 }
 
+// H psi (lam null: its expectation only) in the form planned for the state's size.
+cudaError_t run_h(const void *psi, void *lam, int m, int elem_bytes, const std::vector<LamPassDev> &passes,
+                  const TermDev *dterms, uint32_t nterms, double *energy, int sms, cudaStream_t st)
+{
+    if (passes.empty()) return run_lambda(psi, lam, m, elem_bytes, dterms, nterms, energy, sms, st);
+    return run_lambda_tiles(psi, lam, elem_bytes, passes, dterms, energy, sms, st);
+}
+
 // The reverse program: gates walked backwards from the forward output's map.
 int reverse_program(zxh_sim *s, const std::vector<size_t> &ends, AffineMap A, std::vector<RevStep> &steps,
                     std::vector<AdjDiagGate> &dgates, std::vector<uint32_t> &dslots, int diag_max)
@@ -451,6 +459,7 @@ int zxh_expectation(zxh_sim *s, const zxh_term *terms, size_t nterms, double *va
     if (int rc = flush_pending(s)) return rc;
     std::vector<TermDev> dt;
     if (int rc = compile_terms(s, terms, nterms, s->ws.map, s->ws.m, true, dt)) return rc;
+    const std::vector<zxh::LamPassDev> hpasses = zxh::plan_lambda(dt, s->ws.m);
     const AdjLayout L(0, dt.size());
     if (int rc = ensure_dev(s, reinterpret_cast<void **>(&s->d_adj), s->adj_cap, L.total, "cudaMalloc(adjoint)"))
         return rc;
@@ -461,15 +470,15 @@ int zxh_expectation(zxh_sim *s, const zxh_term *terms, size_t nterms, double *va
         CK(s, cudaMemcpyAsync(d_terms, dt.data(), dt.size() * sizeof(TermDev), cudaMemcpyHostToDevice, s->stream),
            "upload terms");
     CK(s, cudaEventRecord(s->ev0, s->stream), "event");
-    CK(s, zxh::run_lambda(s->d_state, nullptr, s->ws.m, s->elem_bytes, d_terms, uint32_t(dt.size()), d_energy, s->sms,
-                          s->stream),
+    CK(s, run_h(s->d_state, nullptr, s->ws.m, s->elem_bytes, hpasses, d_terms, uint32_t(dt.size()), d_energy, s->sms,
+                s->stream),
        "expectation launch");
     CK(s, cudaEventRecord(s->ev1, s->stream), "event");
     CK(s, cudaMemcpyAsync(value, d_energy, sizeof(double), cudaMemcpyDeviceToHost, s->stream), "read energy");
     CK(s, cudaStreamSynchronize(s->stream), "expectation");
     CK(s, cudaEventElapsedTime(&s->last_ms, s->ev0, s->ev1), "event time");
-    s->stat_kernels = 1;
-    s->stat_passes = 1;
+    s->stat_kernels = std::max<size_t>(1, hpasses.size());
+    s->stat_passes = s->stat_kernels;
     return ZXH_OK;
 }
 
@@ -514,6 +523,7 @@ int zxh_adjoint_gradient(zxh_sim *s, const zxh_term *terms, size_t nterms, size_
     AffineMap A = s->ws.map;
     std::vector<TermDev> dt;
     if (int rc = compile_terms(s, terms, nterms, A, N, false, dt)) return rc;
+    const std::vector<zxh::LamPassDev> hpasses = zxh::plan_lambda(dt, N);
     std::vector<RevStep> steps;
     std::vector<AdjDiagGate> dgates;
     std::vector<uint32_t> dslots;
@@ -547,14 +557,14 @@ int zxh_adjoint_gradient(zxh_sim *s, const zxh_term *terms, size_t nterms, size_
     // reverse sweep (the status word was reset before the forward passes and
     // keeps a forward failure)
     CK(s, cudaEventRecord(s->ev0, s->stream), "event");
-    CK(s, cudaMemcpyAsync(s->d_psi, s->d_state, bytes, cudaMemcpyDeviceToDevice, s->stream), "copy state");
-    CK(s, zxh::run_lambda(s->d_psi, s->d_lam, N, s->elem_bytes, d_terms, uint32_t(dt.size()), d_energy, s->sms,
-                          s->stream),
+    CK(s, run_h(s->d_state, s->d_lam, N, s->elem_bytes, hpasses, d_terms, uint32_t(dt.size()), d_energy, s->sms,
+                s->stream),
        "lambda launch");
-    kernels++;
-    // A checkpoint is not copied back into psi: the next general strided pass
-    // reads psi from it (and writes psi); any other kernel gets the copy first.
-    const void *psi_from = nullptr;
+    kernels += std::max<size_t>(1, hpasses.size());
+    // Neither the forward output nor a checkpoint is copied into psi: the next general
+    // strided pass reads psi from it (and writes psi); any other kernel gets the copy
+    // first.
+    const void *psi_from = s->d_state;
     auto settle_restore = [&]() -> int {
         if (psi_from) {
             CK(s, cudaMemcpyAsync(s->d_psi, psi_from, bytes, cudaMemcpyDeviceToDevice, s->stream),
@@ -567,8 +577,7 @@ int zxh_adjoint_gradient(zxh_sim *s, const zxh_term *terms, size_t nterms, size_
         if (r.kind != RevStep::GROW && r.kind != RevStep::RESTORE)
             if (int rc = settle_restore()) return rc;
         switch (r.kind) {
-        case RevStep::RESTORE:
-            if (int rc = settle_restore()) return rc;
+        case RevStep::RESTORE:  // replaces psi, read or not
             psi_from = static_cast<uint8_t *>(s->d_ckpt) + r.ckpt * bytes;
             break;
         case RevStep::PAIR:
@@ -611,7 +620,7 @@ int zxh_adjoint_gradient(zxh_sim *s, const zxh_term *terms, size_t nterms, size_
     fwd_ms = double(f_ms);
     s->last_ms = float(fwd_ms + double(rev_ms));
     s->stat_kernels = kernels;
-    s->stat_passes = steps.size() + 1;
+    s->stat_passes = steps.size() + std::max<size_t>(1, hpasses.size());
     return ZXH_OK;
 }
 

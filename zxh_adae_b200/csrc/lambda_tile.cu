@@ -1,0 +1,314 @@
+// lambda_tile.cu -- lambda = H psi and <psi|H|psi> over tiles held in shared memory
+// (sm_100a), for states of at least 2^12 amplitudes.
+//
+// H is a sum of Z, ZZ and X terms (lambda_dev.cuh has the real-address forms). An X term
+// reads psi[r ^ delta]; done as one gather per term over the whole state that is one more
+// read of the state each: 24 terms on 2^24 complex64 amplitudes took 0.49 ms where one
+// read of the state takes 0.02 (bound by L2), and 9.7 ms at 2^28 (bound by DRAM). Here a
+// CTA holds a tile closed under the flips it applies: 2^12 amplitudes r0 ^ span(basis),
+// the basis vectors being a basis of the low 4 real bits (runs of 16 contiguous
+// amplitudes) and up to 8 flips that are independent modulo them (any real bits, as after
+// CX transport). One read of the state then serves up to 12 X terms, so a chain of 24
+// takes 3 passes; the Z and ZZ terms ride in the first.
+//
+// Tile coordinates 0..3: lanes 0..3; 4..7: a thread's 16 registers; 8: lane bit 4; 9..11:
+// the warp. A flip of a register coordinate is another register; of the others, a read of
+// the tile in shared memory, whose 16 lanes cover one 128-byte row either way, so every
+// access is conflict-free. A pass is bound by the shared-memory reads (8 per amplitude of a
+// full low pass) or by DRAM.
+//
+// The diagonal sum at a thread's 16 amplitudes is the Walsh-Hadamard transform over the
+// register bits of the coefficients summed by register part (the host sorts the terms by
+// it); a term's sign outside the registers is one bit per tile (one parity per term) XOR
+// one per thread.
+#include "adjoint.h"
+#include "core.h"
+#include "dev.cuh"
+
+#include <algorithm>
+#include <cuda_runtime.h>
+#include <vector>
+
+namespace zxh {
+
+namespace {
+
+constexpr int kLamT = 12, kLamRun = 4, kLamRegs = 16;
+
+template <typename E>
+struct LamSmem {
+    using R = typename ET<E>::R;
+    E slab[1 << kLamT];
+    uint64_t mask[kMaxTerms];
+    R coef[kMaxTerms];
+    uint32_t thread_sign[kMaxTerms / 32][kThreads];
+    uint32_t tile_sign[2][kMaxTerms / 32];
+    double red[kThreads / 32];
+};
+
+// MODE 0: energy only; 1: lam is written; 2: lam is added to.
+template <typename E, int MODE>
+__global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 2 : 1)
+    lambda_tile_kernel(const E *__restrict__ psi, E *lam, const __grid_constant__ LamPassDev p,
+                       const TermDev *__restrict__ terms, double *energy)
+{
+    using R = typename ET<E>::R;
+    extern __shared__ __align__(128) unsigned char s_raw[];
+    LamSmem<E> &sm = *reinterpret_cast<LamSmem<E> *>(s_raw);
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t nd = p.nd;
+
+    // this thread's part of the address and of the tile index
+    uint64_t rt = 0;
+#pragma unroll
+    for (int b = 0; b < 5; b++)
+        if ((lane >> b) & 1u) rt ^= p.basis[b < 4 ? b : 8];
+#pragma unroll
+    for (int b = 0; b < 3; b++)
+        if ((warp >> b) & 1u) rt ^= p.basis[9 + b];
+    const uint32_t it = (lane & 15u) | ((lane >> 4) << 8) | (warp << 9);
+    const uint64_t tr0 = p.tr[lane], tr1 = p.tr[lane + 32u];
+
+    if (tid < nd) {
+        const TermDev t = terms[p.diag0 + tid];
+        const bool zz = t.kind == 2;
+        sm.mask[tid] = zz ? t.a0 ^ t.a1 : t.a0;
+        sm.coef[tid] = ((zz ? t.b0 ^ t.b1 : t.b0) & 1u) ? -R(t.coef) : R(t.coef);
+    }
+    __syncthreads();
+    for (uint32_t w = 0; w * 32u < nd; w++) {
+        uint32_t bits = 0;
+        for (uint32_t k = 0; k < 32u && w * 32u + k < nd; k++) bits |= uint32_t(par64(sm.mask[w * 32u + k] & rt)) << k;
+        sm.thread_sign[w][tid] = bits;
+    }
+
+    double en = 0.0;
+    uint32_t turn = 0;
+    for (uint64_t t = blockIdx.x; t < p.ntiles; t += gridDim.x, turn ^= 1u) {
+        const uint64_t rl = (((t >> lane) & 1u) ? tr0 : 0) ^ (((t >> (lane + 32u)) & 1u) ? tr1 : 0);
+        const uint64_t r0 = (uint64_t(__reduce_xor_sync(0xffffffffu, uint32_t(rl >> 32))) << 32) |
+                            __reduce_xor_sync(0xffffffffu, uint32_t(rl));
+        const uint64_t ra = r0 ^ rt;
+        auto addr = [&](int j) {
+            uint64_t r = ra;
+#pragma unroll
+            for (int b = 0; b < 4; b++)
+                if ((j >> b) & 1) r ^= p.basis[4 + b];
+            return r;
+        };
+        E x[kLamRegs];
+#pragma unroll
+        for (int j = 0; j < kLamRegs; j++) x[j] = __ldg(psi + addr(j));
+        if (warp * 32u < nd) {
+            const uint32_t k = tid;
+            const uint32_t bits = __ballot_sync(0xffffffffu, k < nd && par64(sm.mask[k] & r0));
+            if (lane == 0) sm.tile_sign[turn][warp] = bits;
+        }
+        __syncthreads();  // the slab's previous reads are done
+#pragma unroll
+        for (int j = 0; j < kLamRegs; j++) sm.slab[it | uint32_t(j << 4)] = x[j];
+        __syncthreads();
+
+        // diagonal part: coefficients by register part, then the transform
+        E l[kLamRegs];
+        if (nd) {
+            R u[kLamRegs];
+#pragma unroll
+            for (int g = 0; g < kLamRegs; g++) {
+                R a = 0;
+                for (uint32_t k = p.goff[g]; k < p.goff[g + 1]; k++) {
+                    const uint32_t s = (sm.tile_sign[turn][k >> 5] ^ sm.thread_sign[k >> 5][tid]) >> (k & 31u);
+                    const R c = sm.coef[k];
+                    a += (s & 1u) ? -c : c;
+                }
+                u[g] = a;
+            }
+#pragma unroll
+            for (int b = 1; b < kLamRegs; b <<= 1)
+#pragma unroll
+                for (int g = 0; g < kLamRegs; g++)
+                    if (!(g & b)) {
+                        const R lo = u[g], hi = u[g | b];
+                        u[g] = lo + hi;
+                        u[g | b] = lo - hi;
+                    }
+#pragma unroll
+            for (int j = 0; j < kLamRegs; j++) {
+                l[j].x = u[j] * x[j].x;
+                l[j].y = u[j] * x[j].y;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < kLamRegs; j++) l[j].x = l[j].y = R(0);
+        }
+        // flips of register coordinates
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            if (!((p.xmask >> (4 + b)) & 1u)) continue;
+            const R c = R(p.xc[4 + b]);
+#pragma unroll
+            for (int j = 0; j < kLamRegs; j++) {
+                l[j].x += c * x[j ^ (1 << b)].x;
+                l[j].y += c * x[j ^ (1 << b)].y;
+            }
+        }
+        // flips of lane and warp coordinates
+#pragma unroll
+        for (int k = 0; k < kLamT; k++) {
+            if ((k >= 4 && k < 8) || !((p.xmask >> k) & 1u)) continue;
+            const R c = R(p.xc[k]);
+            const E *row = sm.slab + (it ^ (1u << k));
+#pragma unroll
+            for (int j = 0; j < kLamRegs; j++) {
+                const E q = row[j << 4];
+                l[j].x += c * q.x;
+                l[j].y += c * q.y;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kLamRegs; j++) {
+            en += double(x[j].x) * double(l[j].x) + double(x[j].y) * double(l[j].y);  // Re(conj(psi) lambda)
+            if constexpr (MODE != 0) {
+                E *dst = lam + addr(j);
+                if constexpr (MODE == 2) {
+                    const E old = *dst;
+                    l[j].x += old.x;
+                    l[j].y += old.y;
+                }
+                *dst = l[j];
+            }
+        }
+    }
+    en = warp_sum_f64(en);
+    if (lane == 0) sm.red[warp] = en;
+    __syncthreads();
+    if (tid == 0) {
+        double s = 0.0;
+        for (int w = 0; w < kThreads / 32; w++) s += sm.red[w];
+        atomicAdd(energy, s);
+    }
+}
+
+template <typename E, int MODE>
+cudaError_t launch_pass(const E *psi, E *lam, const LamPassDev &p, const TermDev *terms, double *energy, int sms,
+                        cudaStream_t st)
+{
+    auto kern = lambda_tile_kernel<E, MODE>;
+    const int smem = int(sizeof(LamSmem<E>));
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    int per_sm = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, size_t(smem));
+    const unsigned grid = unsigned(std::min<uint64_t>(p.ntiles, uint64_t(sms) * uint64_t(std::max(1, per_sm))));
+    kern<<<grid, kThreads, size_t(smem), st>>>(psi, lam, p, terms, energy);
+    return cudaGetLastError();
+}
+
+template <typename E>
+cudaError_t lambda_tiles_typed(const E *psi, E *lam, const std::vector<LamPassDev> &passes, const TermDev *terms,
+                               double *energy, int sms, cudaStream_t st)
+{
+    for (size_t i = 0; i < passes.size(); i++) {
+        const cudaError_t e = !lam   ? launch_pass<E, 0>(psi, lam, passes[i], terms, energy, sms, st)
+                              : i ? launch_pass<E, 2>(psi, lam, passes[i], terms, energy, sms, st)
+                                  : launch_pass<E, 1>(psi, lam, passes[i], terms, energy, sms, st);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+int top_bit(uint64_t x) { return 63 - __builtin_clzll(x); }
+
+}  // namespace
+
+std::vector<LamPassDev> plan_lambda(std::vector<TermDev> &terms, int m)
+{
+    std::vector<LamPassDev> out;
+    if (m < kLamT) return out;  // lambda_kernel: no tile fits
+    struct Flip { uint64_t delta; double coef; };
+    std::vector<Flip> flips;
+    size_t nx = 0;
+    while (nx < terms.size() && terms[nx].kind == 3) {
+        const TermDev &t = terms[nx++];
+        auto same = std::find_if(flips.begin(), flips.end(), [&](const Flip &f) { return f.delta == t.delta; });
+        if (same != flips.end()) same->coef += t.coef;
+        else flips.push_back({t.delta, t.coef});
+    }
+    // flips of low bits first: the first tiles are then whole runs of memory
+    std::stable_sort(flips.begin(), flips.end(), [](const Flip &a, const Flip &b) { return a.delta < b.delta; });
+
+    auto reduced = [](uint64_t v, const std::vector<uint64_t> &ech) {
+        for (uint64_t b : ech)
+            if ((v >> top_bit(b)) & 1) v ^= b;
+        return v;
+    };
+    auto insert = [](uint64_t v, std::vector<uint64_t> &ech) {
+        ech.push_back(v);
+        std::sort(ech.rbegin(), ech.rend());
+    };
+    do {
+        LamPassDev p = {};
+        std::vector<uint64_t> low, high;  // echelon forms of the low parts and of the high parts
+        int nlow = 0, nhigh = 0;
+        std::vector<Flip> rest;
+        for (const Flip &f : flips) {
+            const bool inside = (f.delta >> kLamRun) == 0;
+            std::vector<uint64_t> &ech = inside ? low : high;
+            const uint64_t v = reduced(inside ? f.delta : f.delta >> kLamRun, ech);
+            const bool room = inside ? nlow < kLamRun : nhigh < kLamT - kLamRun;
+            if (!v || !room) {
+                rest.push_back(f);
+                continue;
+            }
+            insert(v, ech);
+            const int k = inside ? nlow++ : kLamRun + nhigh++;
+            p.basis[k] = f.delta;
+            p.xc[k] = f.coef;
+            p.xmask |= 1u << k;
+        }
+        flips.swap(rest);
+        for (int b = 0; b < m; b++) {  // complete the basis by single bits, the lowest first
+            const bool inside = b < kLamRun;
+            std::vector<uint64_t> &ech = inside ? low : high;
+            if (inside ? nlow == kLamRun : nhigh == kLamT - kLamRun) continue;
+            const uint64_t v = reduced(inside ? 1ULL << b : 1ULL << (b - kLamRun), ech);
+            if (!v) continue;
+            insert(v, ech);
+            p.basis[inside ? nlow++ : kLamRun + nhigh++] = 1ULL << b;
+        }
+        uint64_t piv = low_mask(kLamRun);
+        for (uint64_t v : high) piv |= 1ULL << (top_bit(v) + kLamRun);
+        int t = 0;
+        for (int b = 0; b < m; b++)
+            if (!((piv >> b) & 1)) p.tr[t++] = 1ULL << b;
+        p.ntiles = 1ULL << t;
+        if (out.empty()) {
+            p.diag0 = uint32_t(nx);
+            p.nd = uint32_t(terms.size() - nx);
+            auto part = [&](const TermDev &d) {
+                const uint64_t mask = d.kind == 2 ? d.a0 ^ d.a1 : d.a0;
+                uint32_t g = 0;
+                for (int b = 0; b < 4; b++) g |= uint32_t(parity64(mask & p.basis[4 + b])) << b;
+                return g;
+            };
+            std::stable_sort(terms.begin() + long(nx), terms.end(),
+                             [&](const TermDev &a, const TermDev &b) { return part(a) < part(b); });
+            for (size_t i = nx; i < terms.size(); i++) p.goff[part(terms[i]) + 1]++;
+            for (int g = 0; g < kLamRegs; g++) p.goff[g + 1] += p.goff[g];
+        }
+        out.push_back(p);
+    } while (!flips.empty());
+    return out;
+}
+
+cudaError_t run_lambda_tiles(const void *psi, void *lam, int elem_bytes, const std::vector<LamPassDev> &passes,
+                             const TermDev *dterms, double *energy, int sms, cudaStream_t st)
+{
+    if (elem_bytes == 8)
+        return lambda_tiles_typed(static_cast<const float2 *>(psi), static_cast<float2 *>(lam), passes, dterms, energy,
+                                  sms, st);
+    return lambda_tiles_typed(static_cast<const double2 *>(psi), static_cast<double2 *>(lam), passes, dterms, energy, sms,
+                              st);
+}
+
+}  // namespace zxh
