@@ -337,7 +337,9 @@ int zxh_optimize_gates(size_t n, int level, const zxh_gate *gates, size_t count,
  * tiles a warp of the diagonal pass walks in Gray-code order; -1 = automatic),
  * diag_row_bits_c64, diag_row_bits_c128 (log2 rows of its warp tile), grow (1:
  * U3 batches whose pair deltas span several bits use the general strided pass,
- * 0: the TMA tile / global pair passes), grow_regs (1..4: gates with high deltas per
+ * 0: the TMA tile / global pair passes), affine (1: such batches, and the adjoint
+ * sweep, run as affine tile passes on states of at least 2^12 amplitudes with
+ * every qubit expanded, 0: the register-row form of the general strided pass), grow_regs (1..4: gates with high deltas per
  * general strided pass), grow_only (1: plan every batch and window as general
  * strided passes after a |0...0> init, the pass set of the batched launch; needs
  * eager_expand_all), adj_windows (1: the adjoint sweep undoes diagonal gates

@@ -1,0 +1,144 @@
+"""Affine tile passes: gates with any pair deltas in tiles of 2^12 amplitudes, at the
+smallest states that take them (12 qubits: one tile), and above; deltas inside the runs,
+dependent modulo the runs and spread over all bits; real and complex matrices; windows of
+single and paired selectors; the adjoint form with checkpoints. Against the oracle, its dense
+adjoint and the general strided passes (knob affine = 0)."""
+import math
+
+import numpy as np
+import pytest
+
+from oracle import observables as ob
+from oracle.bridge import Oracle
+from zxh_adae_b200 import ZXH, workloads
+from zxh_adae_b200 import adjoint as ad
+from zxh_adae_b200._core import plan_stats
+from zxh_adae_b200.records import CP, CX, H, P, RX, RZ, U3, X, Z, as_records
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"complex64": 1e-6, "complex128": 1e-12}  # the parity suite's bounds on amplitudes
+
+
+def layer(n, rng, gates, window):
+    qs = rng.permutation(n)[: int(rng.integers(1, n + 1))]
+    if gates == "real":
+        recs = [(U3, 0, int(q), rng.uniform(0, 6), 0.0, 0.0) for q in qs]
+    elif gates == "h":
+        recs = [(H, 0, int(q)) for q in qs]
+    else:
+        recs = [(U3, 0, int(q), *rng.uniform(0, 6, 3)) for q in qs]
+    if window == "linear":
+        recs += [(int(rng.choice([RZ, P, Z])), 0, int(q), rng.uniform(0, 6)) for q in rng.permutation(n)[: n // 2]]
+    elif window == "chain":
+        recs += [(CP, i, i + 1, rng.uniform(0, 6)) for i in range(n - 1)]
+    elif window == "dense":  # pairs of every kind, a pair of a qubit with itself, repeats
+        for _ in range(40):
+            a, b = (int(v) for v in rng.integers(0, n, 2))
+            recs.append((CP, a, b, rng.uniform(0, 6)))
+    return recs
+
+
+def circuit(n, links, gates, window, seed, layers=4):
+    rng = np.random.default_rng(seed)
+    recs = [(H, 0, q) for q in range(n)]
+    for _ in range(layers):
+        if links == "chain":
+            recs += [(CX, i, i + 1) for i in range(n - 1)]
+        elif links == "back":  # from the high qubits down: deltas inside the runs mix
+            recs += [(CX, i + 1, i) for i in range(n - 1)]
+        else:
+            recs += [(CX, int(a), int(b)) for a, b in rng.integers(0, n, (3 * n, 2)) if a != b]
+        recs += [(X, 0, int(q)) for q in rng.permutation(n)[:3]]
+        recs += layer(n, rng, gates, window)
+    return as_records(recs)
+
+
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+@pytest.mark.parametrize("window", ["none", "linear", "chain", "dense"])
+@pytest.mark.parametrize("n,links,gates", [(12, "chain", "complex"), (12, "random", "real"), (13, "back", "complex"),
+                                           (14, "chain", "h"), (15, "random", "complex"), (16, "back", "real")])
+def test_affine_passes_against_oracle(n, links, gates, window, dtype):
+    g = circuit(n, links, gates, window, seed=n)
+    assert plan_stats(n, g, dtype=dtype)["grow"] > 0
+    o = Oracle(n)
+    o.push(g)
+    o.execute()
+    for affine in (1, 0):
+        s = ZXH(n, dtype=dtype)
+        s.set_param("affine", affine)
+        s.push_gates(g)
+        s.execute()
+        assert np.max(np.abs(s.get_state(0).astype(np.complex128) - o.get_state(0))) <= TOL[dtype], affine
+        s.close()
+
+
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+def test_affine_layers_applied_one_by_one(dtype):
+    # phases an apply leaves over meet a batch of affine passes as its first window
+    n = 13
+    rng = np.random.default_rng(4)
+    parts = [workloads.h_all(n), workloads.u3_layer(n, 1), workloads.cx_chain(n),
+             as_records(layer(n, rng, "complex", "chain")), workloads.u3_layer(n, 2), workloads.cx_chain(n),
+             as_records(layer(n, rng, "real", "linear"))]
+    s = ZXH(n, dtype=dtype)
+    s.push_gates(parts[0])
+    s.execute()
+    for p in parts[1:]:
+        s.apply(p)
+    o = Oracle(n)
+    o.push(np.concatenate(parts))
+    o.execute()
+    assert np.max(np.abs(s.get_state(0).astype(np.complex128) - o.get_state(0))) <= TOL[dtype]
+    s.close()
+
+
+def ansatz(n, links, window, seed):
+    rng = np.random.default_rng(seed)
+    recs, par = [], []
+
+    def add(rec, parameter):
+        recs.append(rec)
+        par.append(sum(p >= 0 for p in par) if parameter else -1)
+
+    for _ in range(3):
+        for q in rng.permutation(n):
+            add((U3, 0, int(q), 0.0, 0.0, 0.0) if rng.random() < 0.7 else (RX, 0, int(q), 0.0), True)
+        add((H, 0, int(rng.integers(n))), False)
+        if window == "dense":
+            for a, b in rng.integers(0, n, (20, 2)):
+                if a != b:
+                    add((CP, int(a), int(b), 0.0), True)
+            add((Z, 0, 2), False)
+        for q in rng.permutation(n)[: n - 2]:
+            add((RZ if rng.random() < 0.5 else P, 0, int(q), 0.0), True)
+        if links == "chain":
+            for i in range(n - 1):
+                add((CX, i, i + 1), False)
+        else:
+            for a, b in rng.integers(0, n, (2 * n, 2)):
+                if a != b:
+                    add((CX, int(a), int(b)), False)
+        add((X, 0, int(rng.integers(n))), False)
+    return ad.Circuit(n, as_records(recs), par)
+
+
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+@pytest.mark.parametrize("n,links,window", [(12, "chain", "linear"), (12, "random", "dense"), (13, "random", "linear"),
+                                            (15, "chain", "dense")])
+def test_affine_gradients_against_dense_adjoint(n, links, window, dtype):
+    circ = ansatz(n, links, window, seed=n)
+    terms = ad.tfim_terms(n, h=0.6)
+    p = np.random.default_rng(n).uniform(-math.pi, math.pi, circ.nparams)
+    e_ref, g_ref = ob.dense_adjoint(n, circ.records(p), terms)
+    s = ZXH(n, dtype=dtype)
+    s.push_gates(circ.records(p))
+    # energies and gradients are sums of 2 n unit terms of the state's relative error
+    tol = 2 * n * (1e-12 if dtype == "complex128" else 1e-6)
+    for every in (0, 7):
+        e, g = s.adjoint_gradient(terms, every)
+        assert abs(e - e_ref) <= tol
+        assert np.max(np.abs(g - g_ref)) <= tol
+    want = ob.oracle_state(n, circ.records(p))
+    assert np.max(np.abs(ob.qubit_order(s.get_state(), n) - want)) <= TOL[dtype]  # the forward output stays
+    s.close()

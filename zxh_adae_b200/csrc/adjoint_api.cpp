@@ -123,7 +123,7 @@ struct AdjLayout {
     }
 };
 
-// Descriptors of the general strided adjoint passes, packed into one blob.
+// Descriptors of the general strided and affine tile adjoint passes, packed into one blob.
 std::vector<uint8_t> pack_grow(std::vector<RevStep> &steps)
 {
     std::vector<uint8_t> blob;
@@ -135,15 +135,23 @@ std::vector<uint8_t> pack_grow(std::vector<RevStep> &steps)
     };
     uint64_t toff = 0;
     bool have_tab = false;
+    auto table = [&](int elem_bytes) {  // the phase table of the windows
+        if (have_tab) return;
+        std::vector<uint8_t> t;
+        zxh::exp_table(elem_bytes, t);
+        toff = put(t.data(), t.size());
+        have_tab = true;
+    };
     for (RevStep &r : steps) {
+        if (r.kind == RevStep::AFFINE) {
+            if (r.aff->dev.win[0].nterms) table(r.aff->elem_bytes);
+            r.toff = toff;
+            r.off = zxh::pack_affine(*r.aff, put);
+            continue;
+        }
         if (r.kind != RevStep::GROW) continue;
         zxh::GrowBuild &gb = r.gb;
-        if (gb.dev.ncls[1][2] && !have_tab) {  // the phase table of the windows
-            std::vector<uint8_t> t;
-            zxh::exp_table(gb.elem_bytes, t);
-            toff = put(t.data(), t.size());
-            have_tab = true;
-        }
+        if (gb.dev.ncls[1][2]) table(gb.elem_bytes);
         r.toff = toff;
         gb.dev.nsel = uint32_t(gb.sels.size());
         gb.dev.off_gates = put(gb.gates.data(), gb.gates.size() * sizeof(zxh::GrowGateDev));
@@ -228,10 +236,11 @@ int forward_segments(zxh_sim *s, const std::vector<size_t> &ends, double &ms, ui
         if (!P.empty()) {
             const void *src = nullptr;
             if (cur != s->d_state) {
-                if (P.front().kind == zxh::Pass::GROW) src = cur;
+                if (P.front().kind == zxh::Pass::GROW || P.front().kind == zxh::Pass::AFFINE) src = cur;
                 else if (int rc = to_state()) return rc;
             }
-            void *dst = (k < nck && P.back().kind == zxh::Pass::GROW) ? ckpt(k) : nullptr;
+            const bool strided = P.back().kind == zxh::Pass::GROW || P.back().kind == zxh::Pass::AFFINE;
+            void *dst = (k < nck && strided) ? ckpt(k) : nullptr;
             if (dst == src && dst) dst = nullptr;  // never in place on a slot it reads whole
             CK(s, zxh::run_passes(P, s->d_blob + boff[k], s->d_state, s->elem_bytes, s->d_status, s->sms, s->stream,
                                   kernels, src, dst),
@@ -279,6 +288,13 @@ int reverse_program(zxh_sim *s, const std::vector<size_t> &ends, AffineMap A, st
     const int R = std::max(1, std::min(s->pp.adj_regs, zxh::grow_reg_bits(s->elem_bytes, true)));
     const int maxg = zxh::grow_adjoint_gates();
     const bool fuse = N >= F && s->pp.adj_windows;  // diagonal gates ride in the general strided passes
+    // affine tile passes; grow_only is the batch kernel's set, which has none
+    const bool tiles = fuse && s->pp.affine && !s->pp.grow_only && N >= zxh::kAffBits;
+    auto all_deltas = [&]() {
+        std::vector<uint64_t> d(static_cast<size_t>(N), 0);
+        for (int q = 0; q < N; q++) A.solve(q, d[size_t(q)]);
+        return d;
+    };
     PairGroup pg;
     // Diagonal gates met since the last pair group: in forward order they follow the
     // gates of the group collected next, so that group's pass undoes them first.
@@ -319,6 +335,29 @@ int reverse_program(zxh_sim *s, const std::vector<size_t> &ends, AffineMap A, st
     };
     auto close_group = [&]() -> int {
         if (pg.gates.empty() && pw.empty()) return ZXH_OK;
+        if (tiles) {
+            RevStep r;
+            r.kind = RevStep::AFFINE;
+            r.aff = std::make_shared<zxh::AffBuild>();
+            std::vector<zxh::U3Op> ops;
+            std::vector<uint32_t> gens, slots;
+            for (const PairGroup::G &g : pg.gates) {
+                ops.push_back(g.op);
+                gens.push_back(g.gen);
+                slots.push_back(g.slot);
+            }
+            const bool ok = r.aff->init(s->elem_bytes, N, ops, all_deltas(), true, &gens, &slots);
+            const bool fused = ok && (pw.empty() || r.aff->add_window(0, pw, &pwk, &pws, true));
+            if (!fused && !pw.empty() && !window_steps())
+                return fail(s, ZXH_ERR_STATE, "adjoint sweep: window not placeable");
+            if (ok && (fused || !pg.gates.empty())) steps.push_back(r);
+            else if (!ok) pair_steps();
+            pg = PairGroup();
+            pw.clear();
+            pwk.clear();
+            pws.clear();
+            return ZXH_OK;
+        }
         std::vector<uint64_t> regs;
         for (const PairGroup::G &g : pg.gates)
             if (g.op.delta >> F) regs.push_back(g.op.delta);
@@ -422,6 +461,13 @@ int reverse_program(zxh_sim *s, const std::vector<size_t> &ends, AffineMap A, st
             pgt.gen = pair_generator(g);
             pgt.slot = uint32_t(gi);
             pgt.q = int(g.q);
+            if (tiles) {
+                if (!pg.join_affine(pgt)) {
+                    if (int rc = close_group()) return rc;
+                    pg.join_affine(pgt);
+                }
+                break;
+            }
             if (!pg.fits(pgt, F, R, N, maxg))
                 if (int rc = close_group()) return rc;
             pg.add(pgt, F);
@@ -574,7 +620,7 @@ int zxh_adjoint_gradient(zxh_sim *s, const zxh_term *terms, size_t nterms, size_
         return ZXH_OK;
     };
     for (const RevStep &r : steps) {
-        if (r.kind != RevStep::GROW && r.kind != RevStep::RESTORE)
+        if (r.kind != RevStep::GROW && r.kind != RevStep::AFFINE && r.kind != RevStep::RESTORE)
             if (int rc = settle_restore()) return rc;
         switch (r.kind) {
         case RevStep::RESTORE:  // replaces psi, read or not
@@ -591,6 +637,13 @@ int zxh_adjoint_gradient(zxh_sim *s, const zxh_term *terms, size_t nterms, size_
                                 (s->pp.grow_staged & (s->elem_bytes == 8 ? 1 : 4)) != 0,
                                 s->d_status, s->sms, s->stream, psi_from),
                "adjoint strided launch");
+            psi_from = nullptr;
+            kernels++;
+            break;
+        case RevStep::AFFINE:
+            CK(s, zxh::run_affine(s->d_adj + L.grow, r.off, r.toff, r.aff->dev.ntiles, s->elem_bytes, r.aff->real,
+                                  s->d_psi, psi_from, s->d_lam, d_grads, s->sms, s->stream),
+               "adjoint tile launch");
             psi_from = nullptr;
             kernels++;
             break;

@@ -25,15 +25,16 @@ int compile_terms(zxh_sim *s, const zxh_term *terms, size_t nterms, AffineMap &A
                   std::vector<TermDev> &out);
 
 struct RevStep {
-    enum Kind { PAIR, DIAG, RESTORE, GROW } kind;
+    enum Kind { PAIR, DIAG, RESTORE, GROW, AFFINE } kind;
     AdjPairDev pair;
     size_t slot = 0;   // PAIR: gradient slot
     size_t first = 0;  // DIAG: first gate in the uploaded group array
     uint32_t ng = 0;   // DIAG: gates in the group
     size_t ckpt = 0;   // RESTORE: checkpoint index
     zxh::GrowBuild gb; // GROW: commuting 2x2 gates on distinct qubits, adjoint form
-    uint64_t off = 0;  // GROW: descriptor offset in the uploaded blob
-    uint64_t toff = 0; // GROW: phase-table offset in the uploaded blob
+    std::shared_ptr<AffBuild> aff;  // AFFINE: the same as an affine tile pass
+    uint64_t off = 0;  // GROW, AFFINE: descriptor offset in the uploaded blob
+    uint64_t toff = 0; // GROW, AFFINE: phase-table offset in the uploaded blob
 };
 
 // A run of 2x2 gates on distinct qubits with no CX between them, collected in
@@ -49,6 +50,16 @@ struct PairGroup {
     std::vector<G> gates;
     std::vector<uint64_t> basis;  // reduced high parts of the register deltas
     int nreg = 0;
+    AffBuild::Room room;          // affine tile passes
+    // The same as fits and add, for an affine tile pass.
+    bool join_affine(const G &g)
+    {
+        for (const G &h : gates)
+            if (h.q == g.q) return false;
+        if (!room.add(g.op.delta)) return false;
+        gates.push_back(g);
+        return true;
+    }
     // Whether g can join (distinct qubit, room, independent high part).
     bool fits(const G &g, int F, int R, int m, int maxg) const
     {

@@ -768,6 +768,11 @@ int zxh_plan_stats(size_t n, int disable_x, int eager_expand_all, int dtype, con
             out[10]++;
             continue;
         }
+        if (p.kind == zxh::Pass::AFFINE) {  // a form of the general strided pass
+            out[9]++;
+            out[10]++;
+            continue;
+        }
         if (p.kind > zxh::Pass::GROW) continue;
         out[2 + int(p.kind)]++;
         if (p.kind != zxh::Pass::PRODUCT) out[10]++;
@@ -808,6 +813,7 @@ int zxh_set_param(zxh_sim *s, const char *name, int value)
         {"span_mixed", &s->pp.span_mixed, 0, 1},
         {"diag_chunk_bits", &s->pp.diag_chunk_bits, -1, 8},
         {"grow", &s->pp.grow, 0, 1},
+        {"affine", &s->pp.affine, 0, 1},
         {"grow_regs", &s->pp.grow_regs, 1, 4},
         {"grow_only", &s->pp.grow_only, 0, 1},
         {"adj_windows", &s->pp.adj_windows, 0, 1},

@@ -10,6 +10,7 @@
 #include <complex>
 #include <cstdint>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -112,6 +113,8 @@ struct Op {
     int m = 0;                   // state bits when the op runs (after growth for EXPAND)
     std::vector<U3Op> u3;
     std::vector<DiagTerm> diag;
+    // U3BATCH: the pair delta of every qubit, where every qubit has one (all expanded)
+    std::shared_ptr<const std::vector<uint64_t>> deltas;
 };
 
 // ---------------------------------------------------------------------------

@@ -178,11 +178,21 @@ int walk(const Gate *gates, size_t count, bool disable_x, int M, WalkState &ws, 
         window.clear();
     };
 
+    // every qubit's delta, where the map has one for each
+    auto all_deltas = [&]() -> std::shared_ptr<const std::vector<uint64_t>> {
+        if (A.m() != N) return nullptr;
+        auto d = std::make_shared<std::vector<uint64_t>>(size_t(N), 0);
+        for (int q = 0; q < N; q++)
+            if (!A.solve(q, (*d)[size_t(q)])) return nullptr;
+        return d;
+    };
+
     auto flush_u3_batch = [&]() {
         if (pend_count == 0) return;
         Op op;
         op.kind = Op::U3BATCH;
         op.m = ws.m;
+        op.deltas = all_deltas();
         for (int q = 0; q < N; q++) {
             if (!pend[q].active) continue;
             U3Op u;
@@ -1289,6 +1299,35 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
         return true;
     };
 
+    // Affine tile passes for one batch: the gates in order of their deltas (low bits first:
+    // longer runs), each in the first pass with room for it.
+    auto emit_affine = [&](const Op &op) -> bool {
+        std::vector<const U3Op *> gs;
+        for (const U3Op &u : op.u3) gs.push_back(&u);
+        std::sort(gs.begin(), gs.end(), [](const U3Op *a, const U3Op *b) { return a->delta < b->delta; });
+        std::vector<AffBuild::Room> rooms;
+        std::vector<std::vector<U3Op>> groups;
+        for (const U3Op *u : gs) {
+            size_t k = 0;
+            while (k < rooms.size() && !rooms[k].add(u->delta)) k++;
+            if (k == rooms.size()) {
+                rooms.emplace_back();
+                groups.emplace_back();
+                if (!rooms[k].add(u->delta)) return false;
+            }
+            groups[k].push_back(*u);
+        }
+        for (const std::vector<U3Op> &g : groups) {
+            Pass ps;
+            ps.kind = Pass::AFFINE;
+            ps.m = op.m;
+            ps.aff = std::make_shared<AffBuild>();
+            if (!ps.aff->init(elem_bytes, op.m, g, *op.deltas)) return false;
+            out.passes.push_back(ps);
+        }
+        return true;
+    };
+
     for (; i < ops.size(); i++) {
         const Op &op = ops[i];
         const std::vector<DiagTerm> *wd = op.kind == Op::DIAG ? &op.diag : nullptr;  // this op's window
@@ -1562,6 +1601,12 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
                 ensure_exp();
                 out.passes[last_tile_pass].off2 = exp_off;
                 last_tile_pass = -1;
+            } else if (last_tile_pass >= 0 && out.passes[last_tile_pass].kind == Pass::AFFINE &&
+                       out.passes[last_tile_pass].m == op.m && out.passes[last_tile_pass].aff->dev.win[1].nterms == 0 &&
+                       out.passes[last_tile_pass].aff->add_window(1, *wd)) {
+                ensure_exp();
+                out.passes[last_tile_pass].off2 = exp_off;
+                last_tile_pass = -1;
             } else if (last_tile_pass >= 0 && out.passes[last_tile_pass].kind == Pass::TILE &&
                        out.passes[last_tile_pass].m == op.m &&
                        out.passes[last_tile_pass].steps.size() < size_t(pp.max_steps) && count_general(*wd) <= 32) {
@@ -1599,14 +1644,21 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
             last_tile_pass = -1;
             continue;
         }
-        // U3BATCH with multi-bit deltas: general strided passes (grow.cu)
+        // U3BATCH with multi-bit deltas: affine tile passes (affine.cu), or general strided
+        // passes (grow.cu) for small states and while qubits are unexpanded
         if ((pp.grow || pp.grow_only) && grow_ok(op)) {
             const int mm = op.m;
             const size_t first = out.passes.size();
-            if (emit_grow(op)) {
+            const bool tiles = pp.affine && !pp.grow_only && op.deltas && mm >= kAffBits;
+            bool done = tiles && emit_affine(op);
+            if (!done) {
+                out.passes.resize(first);
+                done = emit_grow(op);
+            }
+            if (done) {
                 if (held) {
-                    GrowBuild &gb = out.passes[first].gb;
-                    if (gb.add_window(0, *held)) {
+                    Pass &p0 = out.passes[first];
+                    if (p0.kind == Pass::AFFINE ? p0.aff->add_window(0, *held) : p0.gb.add_window(0, *held)) {
                         ensure_exp();
                         out.passes[first].off2 = exp_off;
                     } else {
@@ -1722,6 +1774,13 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
             gb.dev.off_terms[1] = put_vec(out.blob, gb.terms[1]);
             ps.off = put(out.blob, gb.dev);
             ps.prefetch = (pp.grow_staged & 2) ? 1 : 0;
+            continue;
+        }
+        if (ps.kind == Pass::AFFINE) {
+            ps.off = pack_affine(*ps.aff, [&](const void *p, size_t n) {
+                const uint8_t *b = static_cast<const uint8_t *>(p);
+                return put_vec(out.blob, std::vector<uint8_t>(b, b + n));
+            });
             continue;
         }
         if (ps.kind == Pass::ROW) {

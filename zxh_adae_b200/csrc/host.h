@@ -1,6 +1,7 @@
 // host.h -- walk and planner interfaces (implemented in host.cpp).
 #pragma once
 
+#include "affine.h"
 #include "core.h"
 
 namespace zxh {
@@ -55,6 +56,8 @@ struct PlanParams {
                                 // 2 KiB; with 32 KiB chunks 1.00 of measured HBM at 30-32 qubits on B200)
     int diag_row_bits_c128 = 3; // same for complex128 (tile = 32 amplitudes x rows: 4 KiB)
     int grow = 1;               // 1: U3 batches with multi-bit deltas use the general strided pass (grow.cu)
+    int affine = 1;             // 1: such batches, and the adjoint sweep, use affine tile passes (affine.cu) on
+                                // states of at least 2^12 amplitudes whose qubits are all expanded
     int grow_regs = 4;          // register coordinates (gates with high deltas) per general strided pass
     int grow_only = 0;          // 1: only INIT and general strided passes (the persistent batch kernel's set)
     int adj_windows = 1;        // adjoint sweep: diagonal gates ride in the general strided passes as windows
@@ -116,7 +119,7 @@ struct GrowBuild {
 };
 
 struct Pass {
-    enum Kind { PRODUCT, EXPAND, TILE, PAIR, DIAG, FAST, ROW, GROW, INIT, WALSH, SPAN } kind;  // INIT: |0...0> (grow_only)
+    enum Kind { PRODUCT, EXPAND, TILE, PAIR, DIAG, FAST, ROW, GROW, INIT, WALSH, SPAN, AFFINE } kind;  // INIT: |0...0> (grow_only)
     int m = 0;
     uint64_t off = 0;    // blob offset of the pass descriptor
     uint64_t off2 = 0;   // PRODUCT: lookup table; DIAG: exp table
@@ -136,6 +139,7 @@ struct Pass {
                                          // staged form (next item in shared memory); SPAN: the landing form
     std::vector<FastGateDev> fgates;     // FAST
     GrowBuild gb;                        // GROW
+    std::shared_ptr<AffBuild> aff;       // AFFINE
 };
 
 struct Plan {
@@ -160,6 +164,18 @@ int fast_reg_bits(int elem_bytes);
 int row_reg_bits(int elem_bytes, int wide);
 int row_fixed_bits(int elem_bytes, int wide);
 bool row_low_ok(int elem_bytes, int wide);  // the shape's lane bits can swap with its rows (the low pass)
+
+// Writes the pass's tables into a blob through put(pointer, bytes) -> offset; returns the
+// descriptor's offset.
+template <typename Put>
+uint64_t pack_affine(AffBuild &ab, Put put)
+{
+    for (int d = 0; d < 2; d++) {
+        ab.dev.win[d].off_entries = put(ab.entries[d].data(), ab.entries[d].size() * sizeof(AffEntryDev));
+        ab.dev.win[d].off_terms = put(ab.terms[d].data(), ab.terms[d].size() * sizeof(AffTermDev));
+    }
+    return put(&ab.dev, sizeof(AffDev));
+}
 
 // carry_in: phases due on the state before the ops (left over by the previous
 // plan; real-bit selectors, so the affine map's changes since do not touch them);

@@ -532,6 +532,11 @@ cudaError_t run_passes(const std::vector<Pass> &passes, const uint8_t *dblob, vo
             const void *src = (i == 0 && first_src) ? first_src : (dst != state ? state : nullptr);
             e = run_grow(dblob, ps.off, ps.off2, int(ps.gb.regs.size()), ps.gb.dev.nitems, elem_bytes, dst, nullptr,
                          nullptr, ps.gb.all_real(), ps.prefetch != 0, status, sms, st, src);
+        } else if (ps.kind == Pass::AFFINE) {
+            void *dst = (i + 1 == passes.size() && last_dst) ? last_dst : state;
+            const void *src = (i == 0 && first_src) ? first_src : (dst != state ? state : nullptr);
+            e = run_affine(dblob, ps.off, ps.off2, ps.aff->dev.ntiles, elem_bytes, ps.aff->real, dst, src, nullptr,
+                           nullptr, sms, st);
         } else if (ps.kind == Pass::DIAG) {
             e = run_diag(dblob, ps.off, ps.off2, ps.m, elem_bytes, ps.row_bits, ps.chunk_bits, ps.prefetch != 0, state, status,
                          sms, st);
