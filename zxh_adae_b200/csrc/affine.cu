@@ -423,10 +423,20 @@ __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? (ADJ ? 2 : 3) : (AD
     const uint64_t ntiles = p.ntiles;
     const uint64_t lw = sm.lw[lane & 15u], lw0 = sm.lw[0], lwe = sm.lw[tid >> 4];
 
-    for (uint64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    auto tile_base = [&](uint64_t t) {
         const uint64_t rl = (((t >> lane) & 1u) ? tr0 : 0) ^ (((t >> (lane + 32u)) & 1u) ? tr1 : 0);
-        const uint64_t r0 = (uint64_t(__reduce_xor_sync(0xffffffffu, uint32_t(rl >> 32))) << 32) |
-                            __reduce_xor_sync(0xffffffffu, uint32_t(rl));
+        return (uint64_t(__reduce_xor_sync(0xffffffffu, uint32_t(rl >> 32))) << 32) |
+               __reduce_xor_sync(0xffffffffu, uint32_t(rl));
+    };
+    // the run of 16 amplitudes this thread asks L2 for, one tile ahead
+    uint64_t rp = 0;
+#pragma unroll
+    for (int b = 0; b < kAffHigh; b++)
+        if ((tid >> b) & 1u) rp ^= sm.basis[kAffRun + b];
+
+    uint64_t rn = tile_base(blockIdx.x);
+    for (uint64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const uint64_t r0 = rn;
         auto addr = [&](uint64_t base, int k0, int j) {
 #pragma unroll
             for (int b = 0; b < 4; b++)
@@ -439,6 +449,15 @@ __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? (ADJ ? 2 : 3) : (AD
             const uint64_t r = addr(r0 ^ ra, 4, j);
             x[j] = __ldcg(src + r);
             if constexpr (ADJ) y[j] = __ldcg(lam + r);
+        }
+        if (t + gridDim.x < ntiles) {
+            rn = tile_base(t + gridDim.x);
+            const uint64_t r = (rn ^ rp) & ~uint64_t(kRun - 1);
+#pragma unroll
+            for (int i = 0; i < int(sizeof(E)) / 8; i++) {
+                prefetch_l2(src + r + i * (kRun / 2));
+                if constexpr (ADJ) prefetch_l2(lam + r + i * (kRun / 2));
+            }
         }
         // selector bits of the tile: lane s takes selectors s and s + 32
         const bool b0 = lane < nsel && par64(sm.alpha[lane] & r0);

@@ -265,6 +265,12 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void *gsrc, uint32_t byte
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gsrc), "r"(bytes) : "memory");
 }
 
+// Asks L2 for the 128-byte line of gsrc.
+__device__ __forceinline__ void prefetch_l2(const void *gsrc)
+{
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(gsrc) : "memory");
+}
+
 // 16-byte asynchronous copy global -> shared through L2 (cp.async.cg); both
 // addresses 16-byte aligned. A thread's copies complete in commit groups.
 __device__ __forceinline__ void cp_async16(void *sdst, const void *gsrc)

@@ -46,6 +46,20 @@ struct LamSmem {
     double red[kThreads / 32];
 };
 
+// c x + y, one paired FP32 FMA or two FP64 ones
+__device__ __forceinline__ float2 axpy(float c, float2 x, float2 y) { return __ffma2_rn(make_float2(c, c), x, y); }
+__device__ __forceinline__ double2 axpy(double c, double2 x, double2 y)
+{
+    return make_double2(fma(c, x.x, y.x), fma(c, x.y, y.y));
+}
+
+// c, negated where bit 0 of s is set
+__device__ __forceinline__ float flip_sign(float c, uint32_t s) { return __uint_as_float(__float_as_uint(c) ^ (s << 31)); }
+__device__ __forceinline__ double flip_sign(double c, uint32_t s)
+{
+    return __hiloint2double(__double2hiint(c) ^ int(s << 31), __double2loint(c));
+}
+
 // MODE 0: energy only; 1: lam is written; 2: lam is added to.
 template <typename E, int MODE>
 __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 2 : 1)
@@ -82,12 +96,22 @@ __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 2 : 1)
         sm.thread_sign[w][tid] = bits;
     }
 
+    auto tile_base = [&](uint64_t t) {
+        const uint64_t rl = (((t >> lane) & 1u) ? tr0 : 0) ^ (((t >> (lane + 32u)) & 1u) ? tr1 : 0);
+        return (uint64_t(__reduce_xor_sync(0xffffffffu, uint32_t(rl >> 32))) << 32) |
+               __reduce_xor_sync(0xffffffffu, uint32_t(rl));
+    };
+    // the run of 16 amplitudes this thread asks L2 for, one tile ahead
+    uint64_t rp = 0;
+#pragma unroll
+    for (int b = 0; b < kLamT - kLamRun; b++)
+        if ((tid >> b) & 1u) rp ^= p.basis[kLamRun + b];
+
     double en = 0.0;
     uint32_t turn = 0;
+    uint64_t rn = tile_base(blockIdx.x);
     for (uint64_t t = blockIdx.x; t < p.ntiles; t += gridDim.x, turn ^= 1u) {
-        const uint64_t rl = (((t >> lane) & 1u) ? tr0 : 0) ^ (((t >> (lane + 32u)) & 1u) ? tr1 : 0);
-        const uint64_t r0 = (uint64_t(__reduce_xor_sync(0xffffffffu, uint32_t(rl >> 32))) << 32) |
-                            __reduce_xor_sync(0xffffffffu, uint32_t(rl));
+        const uint64_t r0 = rn;
         const uint64_t ra = r0 ^ rt;
         auto addr = [&](int j) {
             uint64_t r = ra;
@@ -99,6 +123,15 @@ __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 2 : 1)
         E x[kLamRegs];
 #pragma unroll
         for (int j = 0; j < kLamRegs; j++) x[j] = __ldg(psi + addr(j));
+        if (t + gridDim.x < p.ntiles) {
+            rn = tile_base(t + gridDim.x);
+            const uint64_t r = (rn ^ rp) & ~uint64_t((1 << kLamRun) - 1);
+#pragma unroll
+            for (int i = 0; i < int(sizeof(E)) / 8; i++) {
+                prefetch_l2(psi + r + i * (1 << kLamRun) / 2);
+                if constexpr (MODE == 2) prefetch_l2(lam + r + i * (1 << kLamRun) / 2);
+            }
+        }
         if (warp * 32u < nd) {
             const uint32_t k = tid;
             const uint32_t bits = __ballot_sync(0xffffffffu, k < nd && par64(sm.mask[k] & r0));
@@ -113,13 +146,16 @@ __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 2 : 1)
         E l[kLamRegs];
         if (nd) {
             R u[kLamRegs];
+            uint32_t word = ~0u, signs = 0;
 #pragma unroll
             for (int g = 0; g < kLamRegs; g++) {
                 R a = 0;
                 for (uint32_t k = p.goff[g]; k < p.goff[g + 1]; k++) {
-                    const uint32_t s = (sm.tile_sign[turn][k >> 5] ^ sm.thread_sign[k >> 5][tid]) >> (k & 31u);
-                    const R c = sm.coef[k];
-                    a += (s & 1u) ? -c : c;
+                    if (k >> 5 != word) {
+                        word = k >> 5;
+                        signs = sm.tile_sign[turn][word] ^ sm.thread_sign[word][tid];
+                    }
+                    a += flip_sign(sm.coef[k], signs >> (k & 31u));
                 }
                 u[g] = a;
             }
@@ -147,10 +183,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 2 : 1)
             if (!((p.xmask >> (4 + b)) & 1u)) continue;
             const R c = R(p.xc[4 + b]);
 #pragma unroll
-            for (int j = 0; j < kLamRegs; j++) {
-                l[j].x += c * x[j ^ (1 << b)].x;
-                l[j].y += c * x[j ^ (1 << b)].y;
-            }
+            for (int j = 0; j < kLamRegs; j++) l[j] = axpy(c, x[j ^ (1 << b)], l[j]);
         }
         // flips of lane and warp coordinates
 #pragma unroll
@@ -159,11 +192,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 2 : 1)
             const R c = R(p.xc[k]);
             const E *row = sm.slab + (it ^ (1u << k));
 #pragma unroll
-            for (int j = 0; j < kLamRegs; j++) {
-                const E q = row[j << 4];
-                l[j].x += c * q.x;
-                l[j].y += c * q.y;
-            }
+            for (int j = 0; j < kLamRegs; j++) l[j] = axpy(c, row[j << 4], l[j]);
         }
 #pragma unroll
         for (int j = 0; j < kLamRegs; j++) {
