@@ -1029,14 +1029,22 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
             err = "product state larger than 2^(2*table bits + 16) amplitudes";
             return 5;
         }
-        // three factor tables over consecutive bit ranges, computed in double
+        // Three factor tables over consecutive bit ranges, computed in double: one bit at a
+        // time, each step doubling the table, so an entry's factors multiply in bit order
+        // at two products per entry (12 per entry, taken one entry at a time, were 110 us of
+        // every execute()'s host time).
         std::vector<double> tab;
         auto add_table = [&](int lo, int bits, cd scale) {
-            for (uint64_t y = 0; y < (1ULL << bits); y++) {
-                cd acc = scale;
-                for (int b = 0; b < bits; b++) acc *= ((y >> b) & 1) ? v[lo + b][1] : v[lo + b][0];
-                tab.push_back(acc.real());
-                tab.push_back(acc.imag());
+            std::vector<cd> t(1, scale);
+            t.reserve(size_t(1) << bits);
+            for (int b = 0; b < bits; b++) {
+                const size_t half = t.size();
+                for (size_t y = 0; y < half; y++) t.push_back(t[y] * v[lo + b][1]);
+                for (size_t y = 0; y < half; y++) t[y] *= v[lo + b][0];
+            }
+            for (const cd &x : t) {
+                tab.push_back(x.real());
+                tab.push_back(x.imag());
             }
         };
         add_table(0, int(pd.c0), cd(1.0, 0.0));
