@@ -161,19 +161,22 @@ int flush_pending(zxh_sim *s)
     return ZXH_OK;
 }
 
-void column_tables(const zxh::AffineMap &A, uint64_t tab[8][256])
+// Columns of the map over the state's real bits, qubit q at bit place(q).
+template <typename Place>
+zxh::PermCols map_columns(const zxh::AffineMap &A, int m, Place place)
 {
-    uint64_t col[64] = {0};
-    for (int q = 0; q < A.n(); q++)
-        for (int c = 0; c < A.m(); c++)
-            if ((A.row(q) >> c) & 1) col[c] |= 1ULL << q;
-    for (int k = 0; k < 8; k++)
-        for (int byte = 0; byte < 256; byte++) {
-            uint64_t v = 0;
-            for (int i = 0; i < 8; i++)
-                if ((byte >> i) & 1) v ^= col[8 * k + i];
-            tab[k][byte] = v;
-        }
+    zxh::PermCols c = {};
+    c.m = m;
+    for (int q = 0; q < A.n(); q++) {
+        for (int j = 0; j < m; j++) c.col[j] |= ((A.row(q) >> j) & 1) << place(q);
+        c.b |= ((A.b() >> q) & 1) << place(q);
+    }
+    return c;
+}
+
+zxh::PermCols word_columns(const zxh_sim *s, int m)
+{
+    return map_columns(s->ws.map, m, [](int q) { return q; });
 }
 
 }  // namespace api
@@ -546,22 +549,17 @@ int zxh_measure(zxh_sim *s, size_t shots)
     if (int rc = ensure_dev(s, reinterpret_cast<void **>(&s->d_samp), s->samp_cap, need, "cudaMalloc(sampler)"))
         return rc;
     s->sc.carve(s->d_samp, nseg, shots, true);
-    static thread_local uint64_t tab[8][256];
-    column_tables(s->ws.map, tab);
-    CK(s, cudaMemsetAsync(s->d_status, 0, sizeof(zxh::DevStatus), s->stream), "reset status");
     uint64_t kernels = 0;
     CK(s, cudaEventRecord(s->ev0, s->stream), "event");
-    CK(s, zxh::run_sampler(s->d_state, s->elem_bytes, m, shots, stream_seed, &tab[0][0], s->ws.map.b(), s->sc,
-                           s->d_status, s->sms, s->stream, kernels),
+    // no step of the draw waits on the device, so there is no status to read back
+    CK(s, zxh::run_sampler(s->d_state, s->elem_bytes, m, shots, stream_seed, word_columns(s, m), s->sc.real, s->sc.words,
+                           s->sc, s->sms, s->stream, kernels),
        "sampler launch");
     CK(s, cudaEventRecord(s->ev1, s->stream), "event");
-    CK(s, cudaMemcpyAsync(s->h_status, s->d_status, sizeof(zxh::DevStatus), cudaMemcpyDeviceToHost, s->stream),
-       "read status");
     CK(s, cudaStreamSynchronize(s->stream), "sampler");
     CK(s, cudaEventElapsedTime(&s->last_ms, s->ev0, s->ev1), "event time");
     s->stat_kernels = kernels;
     s->stat_passes = 2;
-    if (s->h_status->code != 0) return fail(s, int(s->h_status->code), "sampler device wait gave up");
     s->measured = shots;
     s->measured_m = m;
     s->cnt_ready = false;
@@ -605,7 +603,7 @@ int zxh_counts(zxh_sim *s, uint64_t *words, uint64_t *counts, size_t capacity, s
     auto *dhits = reinterpret_cast<uint64_t *>(s->d_cnt + 2 * seg_bytes + 256 + shot_bytes);
     CK(s, cudaEventRecord(s->ev0, s->stream), "event");
     if (!s->cnt_ready) {
-        CK(s, zxh::run_counts(s->sc, m, s->ws.map.b(), nuniq, uoff, total, dwords, dhits, 1, s->sms, s->stream,
+        CK(s, zxh::run_counts(s->sc, m, word_columns(s, m), nuniq, uoff, total, dwords, dhits, 1, s->sms, s->stream,
                               kernels),
            "counts launch");
         CK(s, cudaMemcpyAsync(&s->cnt_total, total, sizeof(uint64_t), cudaMemcpyDeviceToHost, s->stream),
@@ -623,7 +621,7 @@ int zxh_counts(zxh_sim *s, uint64_t *words, uint64_t *counts, size_t capacity, s
         return ZXH_OK;
     }
     if (capacity < s->cnt_total) return fail(s, ZXH_ERR_LIMIT, "counts: capacity below the number of distinct outcomes");
-    CK(s, zxh::run_counts(s->sc, m, s->ws.map.b(), nuniq, uoff, total, dwords, dhits, 2, s->sms, s->stream, kernels),
+    CK(s, zxh::run_counts(s->sc, m, word_columns(s, m), nuniq, uoff, total, dwords, dhits, 2, s->sms, s->stream, kernels),
        "counts launch");
     CK(s, cudaEventRecord(s->ev1, s->stream), "event");
     CK(s, cudaMemcpyAsync(words, dwords, s->cnt_total * sizeof(uint64_t), cudaMemcpyDeviceToHost, s->stream),
@@ -649,15 +647,8 @@ static int state_to_device(zxh_sim *s, void *dst, int order)
     const int N = int(s->n);
     const uint64_t nv = 1ULL << N;
     if (s->ws.m < N) CK(s, cudaMemsetAsync(dst, 0, size_t(nv) * size_t(s->elem_bytes), s->stream), "zero state");
-    // columns of the map, rows reversed for the reference's order
-    zxh::PermCols cols = {};
-    const zxh::AffineMap &A = s->ws.map;
-    auto place = [&](int q) { return order == ZXH_ORDER_REFERENCE ? N - 1 - q : q; };
-    cols.m = s->ws.m;
-    for (int q = 0; q < N; q++) {
-        for (int j = 0; j < cols.m; j++) cols.col[j] |= ((A.row(q) >> j) & 1) << place(q);
-        cols.b |= ((A.b() >> q) & 1) << place(q);
-    }
+    const zxh::PermCols cols = map_columns(
+        s->ws.map, s->ws.m, [&](int q) { return order == ZXH_ORDER_REFERENCE ? N - 1 - q : q; });  // zxh.cpp:627-635
     CK(s, zxh::run_permute(s->d_state, cols, s->ws.gphase.real(), s->ws.gphase.imag(), dst, s->elem_bytes, s->sms,
                            s->stream),
        "get_state");

@@ -24,6 +24,7 @@
 //    after cudaDeviceReset the process must not call this entry point again.
 #include "../../include/zxh_b200.h"
 #include "core.h"
+#include "permute.h"
 #include "sampler.h"
 
 #include <cuda_runtime.h>
@@ -96,16 +97,11 @@ extern "C" int zxh_sample_noalloc(const void *state, int dtype, size_t m_bits, u
     sc.carve(base, nseg, 0);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 
-    // the previous call's contents stay in the array: clear what starts at zero
-    e = cudaMemsetAsync(sc.flags_begin, 0,
-                        size_t(static_cast<uint8_t *>(sc.flags_end) - static_cast<uint8_t *>(sc.flags_begin)), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(sc.counts, 0, nseg * sizeof(unsigned long long), st);
-    if (e != cudaSuccess) return fail(ZXH_ERR_CUDA, std::string("clear scratch: ") + cudaGetErrorString(e));
-
     const uint64_t stream_seed = zxh::mix_seed_host(seed, 0);  // as zxh_measure with a set seed
     // no step of the draw waits on another CTA, so there is no device status to read back
-    e = zxh::run_sampler_real(state, dtype == ZXH_C64 ? 8 : 16, m, shots, stream_seed, real_out, sc, nullptr,
-                              g_scratch_sms[dev], st);
+    uint64_t kernels = 0;
+    e = zxh::run_sampler(state, dtype == ZXH_C64 ? 8 : 16, m, shots, stream_seed, zxh::PermCols(), real_out, nullptr, sc,
+                         g_scratch_sms[dev], st, kernels);
     if (e != cudaSuccess) return fail(ZXH_ERR_CUDA, std::string("sampler launch: ") + cudaGetErrorString(e));
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return fail(ZXH_ERR_CUDA, std::string("sampler: ") + cudaGetErrorString(e));

@@ -13,6 +13,7 @@
 //                        reference runs segment_mass_kernel + a CUB scan).
 //   count_kernel         shot -> segment by binary search, warp-aggregated atomics.
 //   offsets (3 kernels)  exclusive scan of the per-segment counts.
+//   small_draw_kernel    the three steps above in one CTA, for few segments and shots.
 //   resolve_warp_kernel  segments hit by <= 32 shots: one warp streams the segment
 //                        once, lane-scans it and places each shot with a warp-
 //                        cooperative search (ballot over lane prefixes, then over
@@ -21,8 +22,10 @@
 //                        the segment CDF in shared memory and binary-searches it.
 //   map_kernel           real index -> packed virtual bits (measure_cuda.cu:315-338).
 // No kernel waits on another CTA.
+#include "chain.cuh"
 #include "core.h"
 #include "dev.cuh"
+#include "permute.h"
 #include "sampler.h"
 
 #include <algorithm>
@@ -155,6 +158,45 @@ __global__ void __launch_bounds__(kThreads) seg_mass_kernel(const E *__restrict_
     }
 }
 
+// The same masses, one CTA per full segment, for states whose segments are fewer than the
+// chip's warps: a warp alone reads its 32 to 64 KiB in 32 steps one after another (25 us
+// at 20 qubits complex128), eight of them share the ranges. Every range is summed as
+// above, so the numbers are the same.
+template <typename E>
+__global__ void __launch_bounds__(kThreads) seg_mass_cta_kernel(const E *__restrict__ state, uint64_t nseg,
+                                                                double *__restrict__ mass, double *__restrict__ parts)
+{
+    using VT = typename ET<E>::VT;
+    constexpr int G = 4096 / ET<E>::V / 32 / 32, PER = 32 / (kThreads / 32);
+    __shared__ double s_part[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    chain_trigger();
+    for (uint64_t sg = blockIdx.x; sg < nseg; sg += gridDim.x) {
+        const VT *v = reinterpret_cast<const VT *>(state + sg * 4096);
+        VT x[PER][G];
+#pragma unroll
+        for (int r = 0; r < PER; r++)
+#pragma unroll
+            for (int i = 0; i < G; i++) x[r][i] = __ldcs(v + ((warp * PER + r) * G + i) * 32 + lane);
+#pragma unroll
+        for (int r = 0; r < PER; r++) {
+            double t = 0.0;
+#pragma unroll
+            for (int i = 0; i < G; i++) t += vec_mass(x[r][i]);
+            t = warp_sum_f64(t);
+            if (lane == 0) s_part[warp * PER + r] = t;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            const double part = s_part[lane];
+            if (parts) parts[sg * 32 + uint64_t(lane)] = part;
+            const double total = __shfl_sync(0xffffffffu, lane_prefix(part, lane), 31);
+            if (lane == 0) mass[sg] = total;
+        }
+        __syncthreads();
+    }
+}
+
 __device__ __forceinline__ uint64_t upper_index(const double *cdf, uint64_t n, double tau)
 {
     uint64_t lo = 0, hi = n;
@@ -210,15 +252,29 @@ __global__ void __launch_bounds__(kThreads) block_sum_kernel(const T *__restrict
 }
 
 template <typename T>
-__global__ void scan_small_kernel(T *v, uint64_t n)
+__global__ void __launch_bounds__(kThreads) scan_small_kernel(T *v, uint64_t n)
 {
-    // single thread, exclusive; n is at most a few thousand block sums
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    T run = 0;
-    for (uint64_t i = 0; i < n; i++) {
-        const T x = v[i];
-        v[i] = run;
-        run += x;
+    // one CTA, exclusive; n is at most a few thousand block sums. One thread adds them in
+    // order, from shared memory: reading them one by one from global memory cost a round
+    // trip to L2 each (19 us for the 64 of a 30-qubit state)
+    __shared__ T sh[kThreads];
+    __shared__ T s_run;
+    if (threadIdx.x == 0) s_run = 0;
+    for (uint64_t b = 0; b < n; b += kThreads) {
+        if (b + threadIdx.x < n) sh[threadIdx.x] = v[b + threadIdx.x];
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            T run = s_run;
+            for (uint32_t i = 0; i < kThreads && b + i < n; i++) {
+                const T x = sh[i];
+                sh[i] = run;
+                run += x;
+            }
+            s_run = run;
+        }
+        __syncthreads();
+        if (b + threadIdx.x < n) v[b + threadIdx.x] = sh[threadIdx.x];
+        __syncthreads();
     }
 }
 
@@ -254,22 +310,99 @@ __global__ void __launch_bounds__(kThreads) block_scan_kernel(const T *in, uint6
     }
 }
 
-// segments hit by at most kWarpMax shots
+// Segment CDF, shot counts and offsets in one CTA, where the segments fit one scan block
+// and the shots are few (a 20-qubit, 1024-shot draw spent 30 us in the seven launches
+// this replaces). The CDF is scanned as block_scan_kernel does, so the draws are the same.
+constexpr uint64_t kSmallShots = 16384;  // 64 searches a thread: about the launches' time
+
+__global__ void __launch_bounds__(kThreads) small_draw_kernel(const double *mass, uint32_t nseg,
+                                                              uint64_t stream_seed, uint32_t shots,
+                                                              unsigned long long *__restrict__ counts,
+                                                              unsigned long long *__restrict__ offsets,
+                                                              uint32_t *heavy_count)
+{
+    constexpr int PER = kScanBlock / kThreads;
+    __shared__ double cdf[kScanBlock];
+    __shared__ __align__(8) uint32_t hits[kScanBlock];
+    const uint32_t tid = threadIdx.x;
+    chain_trigger();
+    chain_wait();
+    if (tid == 0) *heavy_count = 0;
+    for (uint32_t i = tid; i < kScanBlock; i += kThreads) cdf[i] = i < nseg ? mass[i] : 0.0;
+    __syncthreads();
+    {
+        double *sh = reinterpret_cast<double *>(hits);  // not counting yet
+        double acc = 0.0;
+#pragma unroll
+        for (int k = 0; k < PER; k++) acc += cdf[tid * PER + k];
+        sh[tid] = acc;
+        __syncthreads();
+        for (int o = 1; o < kThreads; o <<= 1) {
+            const double x = tid >= unsigned(o) ? sh[tid - o] : 0.0;
+            __syncthreads();
+            sh[tid] += x;
+            __syncthreads();
+        }
+        double run = 0.0 + (sh[tid] - acc);
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            run += cdf[tid * PER + k];
+            cdf[tid * PER + k] = run;
+        }
+        __syncthreads();
+        for (uint32_t i = tid; i < kScanBlock; i += kThreads) hits[i] = 0;
+        __syncthreads();
+    }
+    const double total = cdf[nseg - 1];
+    if (total > 0.0)
+        for (uint32_t i = tid; i < shots; i += kThreads) {
+            const double u = uniform_open01(stream_seed ^ (kSeedShot + uint64_t(i)));
+            atomicAdd(&hits[upper_index(cdf, nseg, u * total)], 1u);
+        }
+    __syncthreads();
+    uint32_t acc = 0;
+#pragma unroll
+    for (int k = 0; k < PER; k++) acc += hits[tid * PER + k];
+    uint32_t *sh = reinterpret_cast<uint32_t *>(cdf);  // the searches are done
+    sh[tid] = acc;
+    __syncthreads();
+    for (int o = 1; o < kThreads; o <<= 1) {
+        const uint32_t x = tid >= unsigned(o) ? sh[tid - o] : 0u;
+        __syncthreads();
+        sh[tid] += x;
+        __syncthreads();
+    }
+    uint32_t run = sh[tid] - acc;
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        const uint32_t i = tid * PER + k;
+        if (i < nseg) {
+            counts[i] = hits[i];
+            offsets[i] = run;
+        }
+        run += hits[i];
+    }
+}
+
+// segments hit by at most kWarpMax shots; a warp takes `group` (at most 32) consecutive
+// segments. Registers are capped so that 4 CTAs fit an SM in complex64.
 template <typename E>
-__global__ void __launch_bounds__(kThreads) resolve_warp_kernel(const E *__restrict__ state, uint64_t nseg,
+__global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 4 : 3) resolve_warp_kernel(const E *__restrict__ state, uint64_t nseg,
                                                                 uint32_t seglen, const unsigned long long *counts,
                                                                 const unsigned long long *offsets, uint64_t stream2,
                                                                 uint64_t *__restrict__ real_out,
                                                                 uint32_t *heavy_list, uint32_t *heavy_count,
-                                                                const double *__restrict__ parts)
+                                                                const double *parts, uint32_t group)
 {
+    chain_trigger();
+    chain_wait();
     const int lane = threadIdx.x & 31;
     const uint64_t gwarp = (uint64_t(blockIdx.x) * kThreads + threadIdx.x) >> 5;
     const uint64_t nwarps = (uint64_t(gridDim.x) * kThreads) >> 5;
     const uint32_t per_lane = (seglen + 31) / 32;  // amplitudes owned by a lane
-    for (uint64_t g0 = gwarp * 32; g0 < nseg; g0 += nwarps * 32) {
+    for (uint64_t g0 = gwarp * group; g0 < nseg; g0 += nwarps * group) {
         const uint64_t gl = g0 + uint64_t(lane);
-        const unsigned long long cl = gl < nseg ? counts[gl] : 0ULL;
+        const unsigned long long cl = gl < nseg && uint32_t(lane) < group ? counts[gl] : 0ULL;
         unsigned todo = __ballot_sync(0xffffffffu, cl != 0);
         if (cl > kWarpMax) heavy_list[atomicAdd(heavy_count, 1u)] = uint32_t(gl);
         todo &= __ballot_sync(0xffffffffu, cl <= kWarpMax);
@@ -291,6 +424,7 @@ __global__ void __launch_bounds__(kThreads) resolve_warp_kernel(const E *__restr
             const double excl = incl - part;
             // this lane's shot
             double tau = 0.0;
+            uint64_t mine = 0;  // its outcome
             if (uint64_t(lane) < cnt) tau = uniform_open01(stream2 ^ (kSeedOffset + off + uint64_t(lane))) * total;
             if (seglen == 4096) {
                 // full segments: the owner range is 128 amplitudes, 4 per lane; they
@@ -346,15 +480,13 @@ __global__ void __launch_bounds__(kThreads) resolve_warp_kernel(const E *__restr
                         hit = uint64_t(owner) * 128u + (sl < 32 ? uint32_t(sl) * 4u + fs : 128u);
                         if (hit >= seglen) hit = seglen - 1;
                     }
-                    if (lane == 0) real_out[off + uint64_t(j)] = g * seglen + hit;
+                    if (lane == j) mine = g * seglen + hit;
                     t = tn;
                     owner = on;
 #pragma unroll
                     for (int i = 0; i < 4; i++) cur[i] = nxt[i];
                 }
-                continue;
-            }
-            for (int j = 0; j < int(cnt); j++) {
+            } else for (int j = 0; j < int(cnt); j++) {
                 const double t = __shfl_sync(0xffffffffu, tau, j);
                 // owner lane: first lane whose inclusive prefix exceeds t
                 const unsigned le = __ballot_sync(0xffffffffu, incl <= t);
@@ -396,8 +528,9 @@ __global__ void __launch_bounds__(kThreads) resolve_warp_kernel(const E *__restr
                     hit = (sl < 32) ? fs : ohi;
                     if (hit >= seglen) hit = seglen - 1;
                 }
-                if (lane == 0) real_out[off + uint64_t(j)] = g * seglen + hit;
+                if (lane == j) mine = g * seglen + hit;
             }
+            if (uint64_t(lane) < cnt) real_out[off + uint64_t(lane)] = mine;
         }
     }
 }
@@ -427,6 +560,8 @@ __global__ void __launch_bounds__(kThreads) resolve_cta_kernel(const E *__restri
 {
     extern __shared__ double cdf[];  // cdf_slot(seglen) entries
     __shared__ double s_warp[kThreads / 32];
+    chain_trigger();
+    chain_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t nh = *heavy_count;
     // heavy segment h goes to CTA h mod grid, which places all of its shots
@@ -466,20 +601,43 @@ __global__ void __launch_bounds__(kThreads) resolve_cta_kernel(const E *__restri
     }
 }
 
-__global__ void __launch_bounds__(kThreads) map_kernel(const uint64_t *__restrict__ real, uint64_t shots,
-                                                       const uint64_t *__restrict__ coltab, uint64_t b,
+// Virtual words from byte tables (XORs of the map's columns), built by each CTA from the
+// columns in the kernel's parameters.
+struct MapTab {
+    uint64_t t[8][256];
+    uint64_t b;
+    // all threads of the CTA; ends with a barrier
+    __device__ __forceinline__ void build(const PermCols &c)
+    {
+        if (threadIdx.x == 0) b = c.b;
+        for (uint32_t i = threadIdx.x; i < 256; i += kThreads)
+            for (int k = 0; 8 * k < c.m; k++) {
+                uint64_t v = 0;
+#pragma unroll
+                for (int j = 0; j < 8; j++) v ^= ((i >> j) & 1u) ? c.col[8 * k + j] : 0ULL;
+                t[k][i] = v;
+            }
+        m = c.m;
+        __syncthreads();
+    }
+    __device__ __forceinline__ uint64_t word(uint64_t r) const
+    {
+        uint64_t v = b;
+        for (int k = 0; 8 * k < m; k++) v ^= t[k][(r >> (8 * k)) & 255];
+        return v;
+    }
+    int m;
+};
+
+__global__ void __launch_bounds__(kThreads) map_kernel(const uint64_t *real, uint64_t shots,
+                                                       const __grid_constant__ PermCols cols,
                                                        uint64_t *__restrict__ words)
 {
-    __shared__ uint64_t tab[8][256];
-    for (int i = threadIdx.x; i < 8 * 256; i += kThreads) tab[i >> 8][i & 255] = coltab[i];
-    __syncthreads();
-    for (uint64_t i = uint64_t(blockIdx.x) * kThreads + threadIdx.x; i < shots; i += uint64_t(gridDim.x) * kThreads) {
-        const uint64_t r = real[i];
-        uint64_t v = b;
-#pragma unroll
-        for (int k = 0; k < 8; k++) v ^= tab[k][(r >> (8 * k)) & 255];
-        words[i] = v;
-    }
+    __shared__ MapTab tab;
+    tab.build(cols);
+    chain_wait();
+    for (uint64_t i = uint64_t(blockIdx.x) * kThreads + threadIdx.x; i < shots; i += uint64_t(gridDim.x) * kThreads)
+        words[i] = tab.word(real[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -507,29 +665,18 @@ __device__ __forceinline__ uint32_t warp_sort32(uint32_t v, int lane)
     return v;
 }
 
-__device__ __forceinline__ uint64_t map_word(const uint64_t (*tab)[256], uint64_t b, uint64_t r)
-{
-    uint64_t v = b;
-#pragma unroll
-    for (int k = 0; k < 8; k++) v ^= tab[k][(r >> (8 * k)) & 255];
-    return v;
-}
-
 template <bool WRITE>
 __global__ void __launch_bounds__(kThreads) count_light_kernel(const uint64_t *__restrict__ real, uint64_t nseg,
                                                                uint32_t seglen, const unsigned long long *counts,
                                                                const unsigned long long *offsets,
                                                                unsigned long long *nuniq,
                                                                const unsigned long long *uoff,
-                                                               const uint64_t *__restrict__ coltab, uint64_t b,
+                                                               const __grid_constant__ PermCols cols,
                                                                uint64_t *__restrict__ words,
                                                                uint64_t *__restrict__ hits)
 {
-    __shared__ uint64_t tab[WRITE ? 8 : 1][256];
-    if constexpr (WRITE) {
-        for (int i = threadIdx.x; i < 8 * 256; i += kThreads) tab[i >> 8][i & 255] = coltab[i];
-        __syncthreads();
-    }
+    [[maybe_unused]] __shared__ MapTab tab;
+    if constexpr (WRITE) tab.build(cols);
     const int lane = threadIdx.x & 31;
     const uint64_t gwarp = (uint64_t(blockIdx.x) * kThreads + threadIdx.x) >> 5;
     const uint64_t nwarps = (uint64_t(gridDim.x) * kThreads) >> 5;
@@ -557,7 +704,7 @@ __global__ void __launch_bounds__(kThreads) count_light_kernel(const uint64_t *_
                 const unsigned above = starts & ~((2u << lane) - 1u);  // lane 31: 2u << 31 wraps to 0, nothing above
                 const uint32_t next = above ? uint32_t(__ffs(above) - 1) : cnt;
                 const uint64_t slot = uoff[g] + uint64_t(__popc(starts & ((1u << lane) - 1u)));
-                words[slot] = map_word(tab, b, base + key);
+                words[slot] = tab.word(base + key);
                 hits[slot] = next - uint32_t(lane);
             }
         }
@@ -573,16 +720,14 @@ __global__ void __launch_bounds__(kThreads) count_heavy_kernel(const uint64_t *_
                                                                const uint32_t *heavy_count,
                                                                unsigned long long *nuniq,
                                                                const unsigned long long *uoff,
-                                                               const uint64_t *__restrict__ coltab, uint64_t b,
+                                                               const __grid_constant__ PermCols cols,
                                                                uint64_t *__restrict__ words,
                                                                uint64_t *__restrict__ hits)
 {
     __shared__ uint32_t hist[4096];
     __shared__ uint32_t s_warp[kThreads / 32];
-    __shared__ uint64_t tab[WRITE ? 8 : 1][256];
-    if constexpr (WRITE) {
-        for (int i = threadIdx.x; i < 8 * 256; i += kThreads) tab[i >> 8][i & 255] = coltab[i];
-    }
+    [[maybe_unused]] __shared__ MapTab tab;
+    if constexpr (WRITE) tab.build(cols);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t nh = *heavy_count;
     const uint32_t per = (seglen + kThreads - 1) / kThreads;  // bins of a thread (16 for full segments)
@@ -617,7 +762,7 @@ __global__ void __launch_bounds__(kThreads) count_heavy_kernel(const uint64_t *_
             uint64_t slot = uoff[g] + before + incl - mine;
             for (uint32_t k = lo; k < hi; k++)
                 if (hist[k]) {
-                    words[slot] = map_word(tab, b, base + k);
+                    words[slot] = tab.word(base + k);
                     hits[slot] = hist[k];
                     slot++;
                 }
@@ -634,7 +779,7 @@ __global__ void count_total_kernel(const unsigned long long *nuniq, const unsign
 
 }  // namespace
 
-cudaError_t run_counts(const SamplerScratch &sc, int m, uint64_t b, unsigned long long *nuniq,
+cudaError_t run_counts(const SamplerScratch &sc, int m, const PermCols &cols, unsigned long long *nuniq,
                        unsigned long long *uoff, unsigned long long *total, uint64_t *words, uint64_t *hits,
                        int pass, int sms, cudaStream_t st, uint64_t &kernels)
 {
@@ -648,20 +793,20 @@ cudaError_t run_counts(const SamplerScratch &sc, int m, uint64_t b, unsigned lon
     const unsigned gh = unsigned(sms) * 4;
     if (pass == 1) {
         count_light_kernel<false><<<gw, kThreads, 0, st>>>(sc.real, nseg, seglen, sc.counts, sc.offsets, nuniq,
-                                                           nullptr, nullptr, b, nullptr, nullptr);
+                                                           nullptr, cols, nullptr, nullptr);
         count_heavy_kernel<false><<<gh, kThreads, 0, st>>>(sc.real, seglen, sc.counts, sc.offsets, sc.heavy_list,
-                                                           sc.heavy_count, nuniq, nullptr, nullptr, b, nullptr,
+                                                           sc.heavy_count, nuniq, nullptr, cols, nullptr,
                                                            nullptr);
         block_sum_kernel<unsigned long long><<<unsigned(nblk), kThreads, 0, st>>>(nuniq, nseg, sc.bsum);
-        scan_small_kernel<unsigned long long><<<1, 32, 0, st>>>(sc.bsum, nblk);
+        scan_small_kernel<unsigned long long><<<1, kThreads, 0, st>>>(sc.bsum, nblk);
         block_scan_kernel<unsigned long long, false><<<unsigned(nblk), kThreads, 0, st>>>(nuniq, nseg, sc.bsum, uoff);
         count_total_kernel<<<1, 1, 0, st>>>(nuniq, uoff, nseg, total);
         kernels += 6;
     } else {
         count_light_kernel<true><<<gw, kThreads, 0, st>>>(sc.real, nseg, seglen, sc.counts, sc.offsets, nuniq, uoff,
-                                                          sc.coltab, b, words, hits);
+                                                          cols, words, hits);
         count_heavy_kernel<true><<<gh, kThreads, 0, st>>>(sc.real, seglen, sc.counts, sc.offsets, sc.heavy_list,
-                                                          sc.heavy_count, nuniq, uoff, sc.coltab, b, words, hits);
+                                                          sc.heavy_count, nuniq, uoff, cols, words, hits);
         kernels += 2;
     }
     return cudaGetLastError();
@@ -679,30 +824,24 @@ static size_t layout(SamplerScratch *sc, uint8_t *base, uint64_t nseg, uint64_t 
         return p;
     };
     uint8_t *segcdf = take(nseg * 8);
-    uint8_t *fb = base ? base + b : nullptr;
     uint8_t *heavy_count = take(16);
-    uint8_t *fe = base ? base + b : nullptr;
     uint8_t *counts = take(nseg * 8);
     uint8_t *offsets = take(nseg * 8);
     uint8_t *bsum = take(nblk * 8);
     uint8_t *heavy = take(nseg * 4);
     uint8_t *real = take(shots * 8);
     uint8_t *words = take(shots * 8);
-    uint8_t *coltab = take(8 * 256 * 8);
     uint8_t *parts = with_parts ? take(nseg * 32 * 8) : nullptr;
     if (sc) {
         sc->parts = reinterpret_cast<double *>(parts);
         sc->segcdf = reinterpret_cast<double *>(segcdf);
-        sc->flags_begin = fb;
         sc->heavy_count = reinterpret_cast<uint32_t *>(heavy_count);
-        sc->flags_end = fe;
         sc->counts = reinterpret_cast<unsigned long long *>(counts);
         sc->offsets = reinterpret_cast<unsigned long long *>(offsets);
         sc->bsum = reinterpret_cast<unsigned long long *>(bsum);
         sc->heavy_list = reinterpret_cast<uint32_t *>(heavy);
         sc->real = reinterpret_cast<uint64_t *>(real);
         sc->words = reinterpret_cast<uint64_t *>(words);
-        sc->coltab = reinterpret_cast<uint64_t *>(coltab);
     }
     return b;
 }
@@ -717,120 +856,80 @@ void SamplerScratch::carve(uint8_t *base, uint64_t nseg, uint64_t shots, bool pa
     layout(this, base, nseg, shots, parts);
 }
 
-cudaError_t run_sampler(const void *state, int elem_bytes, int m, uint64_t shots, uint64_t stream_seed,
-                        const uint64_t *host_coltab, uint64_t b, SamplerScratch &sc, DevStatus *status, int sms,
-                        cudaStream_t st, uint64_t &kernels)
+namespace {
+
+template <typename E>
+cudaError_t draw(const E *state, int m, uint64_t shots, uint64_t stream_seed, uint64_t *real_out, const PermCols &cols,
+                 uint64_t *words, SamplerScratch &sc, int sms, cudaStream_t st, uint64_t &kernels)
 {
     const uint64_t local = 1ULL << m;
     const uint32_t seglen = uint32_t(std::min<uint64_t>(4096, local));
     const uint64_t nseg = local / seglen;
     const uint64_t nblk = (nseg + kScanBlock - 1) / kScanBlock;
     const uint64_t stream2 = mix_seed_host(stream_seed, 1);
-    cudaError_t e;
-    e = cudaMemsetAsync(sc.flags_begin, 0, size_t(static_cast<uint8_t *>(sc.flags_end) - static_cast<uint8_t *>(sc.flags_begin)), st);
-    if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(sc.counts, 0, nseg * 8, st);
-    if (e != cudaSuccess) return e;
-    e = cudaMemcpyAsync(sc.coltab, host_coltab, 8 * 256 * 8, cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return e;
-    const unsigned gmass = unsigned(std::max<uint64_t>(1, std::min<uint64_t>((nseg * 32 + kThreads - 1) / kThreads,
-                                                                             uint64_t(sms) * 8)));
-    if (elem_bytes == 8)
-        seg_mass_kernel<float2><<<gmass, kThreads, 0, st>>>(static_cast<const float2 *>(state), nseg, seglen, sc.segcdf,
-                                                            sc.parts);
+    const uint64_t slots = uint64_t(sms) * 8;  // CTAs at most
+    auto grid = [&](uint64_t ctas) { return unsigned(std::max<uint64_t>(1, std::min(ctas, slots))); };
+    // a CTA per segment while that leaves no more CTAs than fit
+    if (seglen == 4096 && nseg <= slots)
+        seg_mass_cta_kernel<E><<<grid(nseg), kThreads, 0, st>>>(state, nseg, sc.segcdf, sc.parts);
     else
-        seg_mass_kernel<double2><<<gmass, kThreads, 0, st>>>(static_cast<const double2 *>(state), nseg, seglen,
-                                                            sc.segcdf, sc.parts);
-    double *bsum_d = reinterpret_cast<double *>(sc.bsum);  // the counts' scan reuses it afterwards
-    block_sum_kernel<double><<<unsigned(nblk), kThreads, 0, st>>>(sc.segcdf, nseg, bsum_d);
-    scan_small_kernel<double><<<1, 32, 0, st>>>(bsum_d, nblk);
-    block_scan_kernel<double, true><<<unsigned(nblk), kThreads, 0, st>>>(sc.segcdf, nseg, bsum_d, sc.segcdf);
-    const unsigned gc = unsigned(std::max<uint64_t>(1, std::min<uint64_t>((shots + kThreads - 1) / kThreads, uint64_t(sms) * 8)));
-    count_kernel<<<gc, kThreads, 0, st>>>(sc.segcdf, nseg, stream_seed, shots, sc.counts);
-    block_sum_kernel<unsigned long long><<<unsigned(nblk), kThreads, 0, st>>>(sc.counts, nseg, sc.bsum);
-    scan_small_kernel<unsigned long long><<<1, 32, 0, st>>>(sc.bsum, nblk);
-    block_scan_kernel<unsigned long long, false><<<unsigned(nblk), kThreads, 0, st>>>(sc.counts, nseg, sc.bsum,
-                                                                                     sc.offsets);
-    const uint64_t warps_needed = (nseg + 31) / 32;
-    const unsigned gw = unsigned(std::max<uint64_t>(1, std::min<uint64_t>((warps_needed * 32 + kThreads - 1) / kThreads,
-                                                                          uint64_t(sms) * 8)));
-    if (elem_bytes == 8)
-        resolve_warp_kernel<float2><<<gw, kThreads, 0, st>>>(static_cast<const float2 *>(state), nseg, seglen, sc.counts,
-                                                            sc.offsets, stream2, sc.real, sc.heavy_list, sc.heavy_count,
-                                                            sc.parts);
-    else
-        resolve_warp_kernel<double2><<<gw, kThreads, 0, st>>>(static_cast<const double2 *>(state), nseg, seglen,
-                                                             sc.counts, sc.offsets, stream2, sc.real, sc.heavy_list,
-                                                             sc.heavy_count, sc.parts);
-    const size_t smem = size_t(seglen + seglen / 16 + 1) * 8;
-    const unsigned gh = unsigned(sms) * 2;
-    if (elem_bytes == 8)
-        resolve_cta_kernel<float2><<<gh, kThreads, smem, st>>>(static_cast<const float2 *>(state), seglen, sc.counts,
-                                                              sc.offsets, stream2, sc.real, sc.heavy_list,
-                                                              sc.heavy_count);
-    else
-        resolve_cta_kernel<double2><<<gh, kThreads, smem, st>>>(static_cast<const double2 *>(state), seglen, sc.counts,
-                                                               sc.offsets, stream2, sc.real, sc.heavy_list,
-                                                               sc.heavy_count);
-    const unsigned gm = unsigned(std::max<uint64_t>(1, std::min<uint64_t>((shots + kThreads - 1) / kThreads, uint64_t(sms) * 8)));
-    map_kernel<<<gm, kThreads, 0, st>>>(sc.real, shots, sc.coltab, b, sc.words);
-    kernels += 11;
-    (void)status;  // no step of the draw waits on another CTA
-    return cudaGetLastError();
+        seg_mass_kernel<E><<<grid((nseg * 32 + kThreads - 1) / kThreads), kThreads, 0, st>>>(state, nseg, seglen, sc.segcdf,
+                                                                                          sc.parts);
+    kernels++;
+    if (nblk == 1 && shots <= kSmallShots) {
+        const cudaError_t e = launch_chained(true, small_draw_kernel, 1, kThreads, 0, st, sc.segcdf, nseg, stream_seed,
+                                             shots, sc.counts, sc.offsets, sc.heavy_count);
+        if (e != cudaSuccess) return e;
+        kernels++;
+    } else {
+        cudaError_t e = cudaMemsetAsync(sc.heavy_count, 0, sizeof(uint32_t), st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(sc.counts, 0, nseg * 8, st);
+        if (e != cudaSuccess) return e;
+        double *bsum_d = reinterpret_cast<double *>(sc.bsum);  // the counts' scan reuses it afterwards
+        block_sum_kernel<double><<<unsigned(nblk), kThreads, 0, st>>>(sc.segcdf, nseg, bsum_d);
+        scan_small_kernel<double><<<1, kThreads, 0, st>>>(bsum_d, nblk);
+        block_scan_kernel<double, true><<<unsigned(nblk), kThreads, 0, st>>>(sc.segcdf, nseg, bsum_d, sc.segcdf);
+        count_kernel<<<grid((shots + kThreads - 1) / kThreads), kThreads, 0, st>>>(sc.segcdf, nseg, stream_seed, shots,
+                                                                                 sc.counts);
+        block_sum_kernel<unsigned long long><<<unsigned(nblk), kThreads, 0, st>>>(sc.counts, nseg, sc.bsum);
+        scan_small_kernel<unsigned long long><<<1, kThreads, 0, st>>>(sc.bsum, nblk);
+        block_scan_kernel<unsigned long long, false><<<unsigned(nblk), kThreads, 0, st>>>(sc.counts, nseg, sc.bsum,
+                                                                                         sc.offsets);
+        kernels += 7;
+    }
+    // Segments per warp: as few as give every warp that fits on the chip (4 CTAs an SM) one
+    // group, so that a small state's segments are not queued behind one another (20 qubits:
+    // 256 segments on 8 warps, 120 us) and a large one's fill the chip.
+    const uint64_t warps = uint64_t(sms) * 4 * (kThreads / 32);
+    const uint32_t group = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(32, (nseg + warps - 1) / warps)));
+    const uint64_t groups = (nseg + group - 1) / group;
+    cudaError_t e = launch_chained(true, resolve_warp_kernel<E>, grid((groups * 32 + kThreads - 1) / kThreads), kThreads, 0,
+                                   st, state, nseg, seglen, sc.counts, sc.offsets, stream2, real_out, sc.heavy_list,
+                                   sc.heavy_count, sc.parts, group);
+    kernels++;
+    if (e == cudaSuccess && shots > kWarpMax) {  // fewer cannot make a segment heavy
+        const size_t smem = size_t(seglen + seglen / 16 + 1) * 8;
+        e = launch_chained(true, resolve_cta_kernel<E>, grid(std::min<uint64_t>(nseg, uint64_t(sms) * 2)), kThreads, smem, st,
+                           state, seglen, sc.counts, sc.offsets, stream2, real_out, sc.heavy_list, sc.heavy_count);
+        kernels++;
+    }
+    if (e == cudaSuccess && words) {
+        e = launch_chained(true, map_kernel, grid((shots + kThreads - 1) / kThreads), kThreads, 0, st, real_out, shots, cols,
+                           words);
+        kernels++;
+    }
+    return e;
 }
 
-// The same draw as run_sampler up to the real indices, written to a caller buffer;
-// used by the allocation-free entry point (noalloc.cu). Scratch comes from sc,
-// whose flag region, counts and heavy count the caller has cleared.
-cudaError_t run_sampler_real(const void *state, int elem_bytes, int m, uint64_t shots, uint64_t stream_seed,
-                             uint64_t *real_out, SamplerScratch &sc, DevStatus *status, int sms, cudaStream_t st)
+}  // namespace
+
+cudaError_t run_sampler(const void *state, int elem_bytes, int m, uint64_t shots, uint64_t stream_seed,
+                        const PermCols &cols, uint64_t *real_out, uint64_t *words, SamplerScratch &sc, int sms,
+                        cudaStream_t st, uint64_t &kernels)
 {
-    const uint64_t local = 1ULL << m;
-    const uint32_t seglen = uint32_t(std::min<uint64_t>(4096, local));
-    const uint64_t nseg = local / seglen;
-    const uint64_t nblk = (nseg + kScanBlock - 1) / kScanBlock;
-    const uint64_t stream2 = mix_seed_host(stream_seed, 1);
-    const unsigned gmass = unsigned(std::max<uint64_t>(1, std::min<uint64_t>((nseg * 32 + kThreads - 1) / kThreads,
-                                                                             uint64_t(sms) * 8)));
     if (elem_bytes == 8)
-        seg_mass_kernel<float2><<<gmass, kThreads, 0, st>>>(static_cast<const float2 *>(state), nseg, seglen, sc.segcdf,
-                                                            sc.parts);
-    else
-        seg_mass_kernel<double2><<<gmass, kThreads, 0, st>>>(static_cast<const double2 *>(state), nseg, seglen,
-                                                            sc.segcdf, sc.parts);
-    double *bsum_d = reinterpret_cast<double *>(sc.bsum);  // the counts' scan reuses it afterwards
-    block_sum_kernel<double><<<unsigned(nblk), kThreads, 0, st>>>(sc.segcdf, nseg, bsum_d);
-    scan_small_kernel<double><<<1, 32, 0, st>>>(bsum_d, nblk);
-    block_scan_kernel<double, true><<<unsigned(nblk), kThreads, 0, st>>>(sc.segcdf, nseg, bsum_d, sc.segcdf);
-    const unsigned gc = unsigned(std::max<uint64_t>(1, std::min<uint64_t>((shots + kThreads - 1) / kThreads, uint64_t(sms) * 8)));
-    count_kernel<<<gc, kThreads, 0, st>>>(sc.segcdf, nseg, stream_seed, shots, sc.counts);
-    block_sum_kernel<unsigned long long><<<unsigned(nblk), kThreads, 0, st>>>(sc.counts, nseg, sc.bsum);
-    scan_small_kernel<unsigned long long><<<1, 32, 0, st>>>(sc.bsum, nblk);
-    block_scan_kernel<unsigned long long, false><<<unsigned(nblk), kThreads, 0, st>>>(sc.counts, nseg, sc.bsum,
-                                                                                     sc.offsets);
-    const uint64_t warps_needed = (nseg + 31) / 32;
-    const unsigned gw = unsigned(std::max<uint64_t>(1, std::min<uint64_t>((warps_needed * 32 + kThreads - 1) / kThreads,
-                                                                          uint64_t(sms) * 8)));
-    if (elem_bytes == 8)
-        resolve_warp_kernel<float2><<<gw, kThreads, 0, st>>>(static_cast<const float2 *>(state), nseg, seglen, sc.counts,
-                                                            sc.offsets, stream2, real_out, sc.heavy_list, sc.heavy_count,
-                                                            sc.parts);
-    else
-        resolve_warp_kernel<double2><<<gw, kThreads, 0, st>>>(static_cast<const double2 *>(state), nseg, seglen,
-                                                             sc.counts, sc.offsets, stream2, real_out, sc.heavy_list,
-                                                             sc.heavy_count, sc.parts);
-    const size_t smem = size_t(seglen + seglen / 16 + 1) * 8;
-    const unsigned gh = unsigned(sms) * 2;
-    if (elem_bytes == 8)
-        resolve_cta_kernel<float2><<<gh, kThreads, smem, st>>>(static_cast<const float2 *>(state), seglen, sc.counts,
-                                                              sc.offsets, stream2, real_out, sc.heavy_list,
-                                                              sc.heavy_count);
-    else
-        resolve_cta_kernel<double2><<<gh, kThreads, smem, st>>>(static_cast<const double2 *>(state), seglen, sc.counts,
-                                                               sc.offsets, stream2, real_out, sc.heavy_list,
-                                                               sc.heavy_count);
-    (void)status;  // no step of the draw waits on another CTA
-    return cudaGetLastError();
+        return draw(static_cast<const float2 *>(state), m, shots, stream_seed, real_out, cols, words, sc, sms, st, kernels);
+    return draw(static_cast<const double2 *>(state), m, shots, stream_seed, real_out, cols, words, sc, sms, st, kernels);
 }
 
 uint64_t mix_seed_host(uint64_t base, uint64_t salt)

@@ -10,11 +10,9 @@ namespace zxh {
 struct SamplerScratch {
     double *segcdf = nullptr;
     uint32_t *heavy_count = nullptr;
-    void *flags_begin = nullptr, *flags_end = nullptr;  // region zeroed before every draw
     unsigned long long *counts = nullptr, *offsets = nullptr, *bsum = nullptr;
     uint32_t *heavy_list = nullptr;
     uint64_t *real = nullptr, *words = nullptr;
-    uint64_t *coltab = nullptr;
     double *parts = nullptr;  // optional: the 32 lane-range masses of every segment
 
     static size_t need_bytes(uint64_t nseg, uint64_t shots, bool parts = false);
@@ -23,25 +21,24 @@ struct SamplerScratch {
 
 uint64_t mix_seed_host(uint64_t base, uint64_t salt);
 
-// Draws shots outcomes from the 2^m-amplitude state into sc.real (real indices,
-// grouped by segment) and sc.words (virtual bits, one word per shot for n <= 63).
+struct PermCols;  // permute.h: the affine map's columns
+
+// Draws shots outcomes from the 2^m-amplitude state into real_out (real indices, grouped
+// by segment) and, where words is given, their virtual bits through the map's columns
+// (one word per shot for n <= 63).
 cudaError_t run_sampler(const void *state, int elem_bytes, int m, uint64_t shots, uint64_t stream_seed,
-                        const uint64_t *host_coltab, uint64_t b, SamplerScratch &sc, DevStatus *status, int sms,
+                        const PermCols &cols, uint64_t *real_out, uint64_t *words, SamplerScratch &sc, int sms,
                         cudaStream_t st, uint64_t &kernels);
 
 // Counts of the draw left in sc by run_sampler on a 2^m-amplitude state (map
-// offset b): pass 1 writes every segment's number of distinct outcomes (nuniq),
+// columns cols): pass 1 writes every segment's number of distinct outcomes (nuniq),
 // their exclusive scan (uoff) and the total; pass 2 writes the distinct outcomes'
 // virtual words and counts at uoff, in increasing real index.
-cudaError_t run_counts(const SamplerScratch &sc, int m, uint64_t b, unsigned long long *nuniq,
+cudaError_t run_counts(const SamplerScratch &sc, int m, const PermCols &cols, unsigned long long *nuniq,
                        unsigned long long *uoff, unsigned long long *total, uint64_t *words, uint64_t *hits,
                        int pass, int sms, cudaStream_t st, uint64_t &kernels);
 
-// run_sampler's draw up to real indices, into a caller buffer (noalloc.cu).
-cudaError_t run_sampler_real(const void *state, int elem_bytes, int m, uint64_t shots, uint64_t stream_seed,
-                             uint64_t *real_out, SamplerScratch &sc, DevStatus *status, int sms, cudaStream_t st);
-
-// Pass runner and get_state scatter (kernels.cu).
+// Pass runner (kernels.cu).
 struct Pass;
 // first_src / last_dst (only where the first / last pass is a general strided
 // pass): that pass reads psi from first_src / writes it to last_dst instead of
