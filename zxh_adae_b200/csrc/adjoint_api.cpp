@@ -611,8 +611,10 @@ int zxh_adjoint_gradient(zxh_sim *s, const zxh_term *terms, size_t nterms, size_
     // strided pass reads psi from it (and writes psi); any other kernel gets the copy
     // first.
     const void *psi_from = s->d_state;
+    bool chained = true;  // the last thing queued is a kernel
     auto settle_restore = [&]() -> int {
         if (psi_from) {
+            chained = false;
             CK(s, cudaMemcpyAsync(s->d_psi, psi_from, bytes, cudaMemcpyDeviceToDevice, s->stream),
                "restore checkpoint");
             psi_from = nullptr;
@@ -638,13 +640,15 @@ int zxh_adjoint_gradient(zxh_sim *s, const zxh_term *terms, size_t nterms, size_
                                 s->d_status, s->sms, s->stream, psi_from),
                "adjoint strided launch");
             psi_from = nullptr;
+            chained = true;
             kernels++;
             break;
         case RevStep::AFFINE:
             CK(s, zxh::run_affine(s->d_adj + L.grow, r.off, r.toff, r.aff->dev.ntiles, s->elem_bytes, r.aff->real,
-                                  s->d_psi, psi_from, s->d_lam, d_grads, s->sms, s->stream),
+                                  s->d_psi, psi_from, s->d_lam, d_grads, chained, s->sms, s->stream),
                "adjoint tile launch");
             psi_from = nullptr;
+            chained = true;
             kernels++;
             break;
         case RevStep::DIAG:

@@ -56,7 +56,7 @@ struct PairGroup {
     {
         for (const G &h : gates)
             if (h.q == g.q) return false;
-        if (!room.add(g.op.delta)) return false;
+        if (room.add(g.op.delta) < 0) return false;
         gates.push_back(g);
         return true;
     }

@@ -23,9 +23,7 @@
 // memory. Gradients of window terms come from the marginals of w = Im(conj(lambda) psi) over
 // the same bits, reduced once per tile. The slot of tile index i is i ^ (bits 4..7 of i): in
 // every layout the lanes that share a bank cycle cover one 128-byte row.
-#include "affine.h"
-#include "core.h"
-#include "dev.cuh"
+#include "affine_dev.cuh"
 
 #include <algorithm>
 #include <cuda_runtime.h>
@@ -34,487 +32,22 @@ namespace zxh {
 
 namespace {
 
-constexpr int kNR = 16;   // amplitudes per thread
-constexpr int kRun = 1 << kAffRun;
-constexpr int kSums = 11;  // w summed over a thread's registers: all, 4 bits, 6 pairs of bits
-
-template <typename E, bool ADJ>
-struct AffSmem {
-    using RT = typename ET<E>::R;
-    static constexpr int NW = ADJ ? 1 : 2;  // windows
-    E slab[ADJ ? 2 : 1][1 << kAffBits];      // adjoint passes: also the sums and marginals of w
-    E exp[1 << kExpTableBits];
-    RT u[kAffBits][2][8];  // [1]: the |1> member first
-    uint32_t sel[kAffBits], gen[kAffBits];
-    uint64_t alpha[kAffMaxSel], lw[kRun], basis[kAffBits];
-    AffWinDev win[NW];
-    AffEntryDev ent[NW][kAffMaxEntries];
-    int64_t K[NW][kRun], w[NW][kRun][kAffHigh], q[NW][kRun][kAffPairs];
-    AffTermDev term[ADJ ? kAffMaxTerms : 1];
-    uint8_t plist[kAffPairs];
-    double tacc[ADJ ? kAffMaxTerms : 1];
-    double gacc[ADJ ? kAffBits : 1][ADJ ? kThreads : 1];
-};
-
-__device__ __forceinline__ uint32_t slot_of(uint32_t i) { return i ^ ((i >> 4) & 15u); }
-
-// Registers j of layout L (0 A, 1 B, 2 C) in tile index bits.
-template <int L>
-__host__ __device__ constexpr uint32_t reg_bits(int j) { return L == 0 ? uint32_t(j) << 4 : L == 1 ? uint32_t(j) << 8 : uint32_t(j); }
-template <int L>
-__device__ __forceinline__ uint32_t fixed_bits(uint32_t lane, uint32_t warp)
-{
-    if constexpr (L == 0) return (lane & 15u) | ((lane >> 4) << 8) | (warp << 9);
-    if constexpr (L == 1) return lane | (warp << 5);
-    return (lane << 4) | (warp << 9);
-}
-
-template <int LA, int LB, int NS, typename E>
-__device__ __forceinline__ void exchange(E (&x)[kNR], E (&y)[kNR], E (*slab)[1 << kAffBits], uint32_t lane, uint32_t warp)
-{
-    const uint32_t a = slot_of(fixed_bits<LA>(lane, warp)), b = slot_of(fixed_bits<LB>(lane, warp));
-    __syncthreads();  // the slab's previous reads are done
-#pragma unroll
-    for (int j = 0; j < kNR; j++) {
-        const uint32_t s = a ^ (reg_bits<LA>(j) ^ ((reg_bits<LA>(j) >> 4) & 15u));
-        slab[0][s] = x[j];
-        if constexpr (NS == 2) slab[1][s] = y[j];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < kNR; j++) {
-        const uint32_t s = b ^ (reg_bits<LB>(j) ^ ((reg_bits<LB>(j) >> 4) & 15u));
-        x[j] = slab[0][s];
-        if constexpr (NS == 2) y[j] = slab[1][s];
-    }
-}
-
-template <typename E, typename RT>
-__device__ __forceinline__ E cmad2(RT ar, RT ai, E a, RT br, RT bi, E b)  // a-coefficient * a + b-coefficient * b
-{
-    E o;
-    o.x = ar * a.x - ai * a.y + br * b.x - bi * b.y;
-    o.y = ar * a.y + ai * a.x + br * b.y + bi * b.x;
-    return o;
-}
-
-// The gate on register bit RR, m its matrix in the thread's orientation; adjoint passes
-// first add the gradient's share (FP32 over 8 pairs for complex64) to acc.
-template <int RR, bool ADJ, bool REAL, typename E, typename RT>
-__device__ __forceinline__ void gate(E (&x)[kNR], E (&y)[kNR], const RT *m, bool flip, uint32_t gen, double *acc)
-{
-    RT part = 0;
-    const RT m0 = m[0], m2 = m[2], m4 = m[4], m6 = m[6];
-    const RT m1 = REAL ? RT(0) : m[1], m3 = REAL ? RT(0) : m[3], m5 = REAL ? RT(0) : m[5], m7 = REAL ? RT(0) : m[7];
-#pragma unroll
-    for (int j = 0; j < kNR; j++) {
-        if ((j >> RR) & 1) continue;
-        constexpr int B = 1 << RR;
-        const E lo = x[j], hi = x[j | B];
-        if constexpr (ADJ) {
-            const E llo = y[j], lhi = y[j | B];
-            if (gen == 1) {  // Im<l|Y|p> = Re(conj(l1) p0) - Re(conj(l0) p1)
-                part += (lhi.x * lo.x + lhi.y * lo.y) - (llo.x * hi.x + llo.y * hi.y);
-            } else if (gen == 2) {  // Im<l|X|p> = Im(conj(l0) p1 + conj(l1) p0)
-                part += (llo.x * hi.y - llo.y * hi.x) + (lhi.x * lo.y - lhi.y * lo.x);
-            }
-            if constexpr (REAL) {
-                y[j] = rmad2(m0, llo, m2, lhi);
-                y[j | B] = rmad2(m4, llo, m6, lhi);
-            } else {
-                y[j] = cmad2(m0, m1, llo, m2, m3, lhi);
-                y[j | B] = cmad2(m4, m5, llo, m6, m7, lhi);
-            }
-        }
-        if constexpr (REAL) {
-            x[j] = rmad2(m0, lo, m2, hi);
-            x[j | B] = rmad2(m4, lo, m6, hi);
-        } else {
-            x[j] = cmad2(m0, m1, lo, m2, m3, hi);
-            x[j | B] = cmad2(m4, m5, lo, m6, m7, hi);
-        }
-    }
-    if constexpr (ADJ) {
-        if (gen) *acc += double(gen == 1 && flip ? -part : part);
-    }
-}
-
-// The gates on coordinates K0 .. K0 + 3, the layout's registers; c: the selector bits of
-// the thread (of the tile, in layout C).
-template <int K0, bool ADJ, bool REAL, typename E, typename SM>
-__device__ __forceinline__ void gates(E (&x)[kNR], E (&y)[kNR], uint32_t mask, uint64_t c, SM &sm, uint32_t tid)
-{
-    auto one = [&](auto rr) {
-        constexpr int RR = decltype(rr)::value, k = K0 + RR;
-        if (!((mask >> k) & 1u)) return;
-        const bool flip = (c >> sm.sel[k]) & 1;
-        gate<RR, ADJ, REAL>(x, y, sm.u[k][flip], flip, sm.gen[k], ADJ ? &sm.gacc[ADJ ? k : 0][ADJ ? tid : 0] : nullptr);
-    };
-    one(std::integral_constant<int, 0>());
-    one(std::integral_constant<int, 1>());
-    one(std::integral_constant<int, 2>());
-    one(std::integral_constant<int, 3>());
-}
-
-// Window d's polynomial at run position l, by the 16 threads part = 0..15 of that position:
-// all take shares of the entries without a coordinate, thread k < 8 those of coordinate k.
-template <typename SM>
-__device__ __forceinline__ void window_eval(SM &sm, const AffWinDev &wd, int d, uint64_t c, uint32_t part, uint32_t l)
-{
-    int64_t K = 0;
-    for (uint32_t e = part; e < wd.n0; e += 16u) {
-        const AffEntryDev t = sm.ent[d][e];
-        const bool on = ((c >> t.s0) & 1) && (t.s1 == 0xff || ((c >> t.s1) & 1));
-        if (on) K += t.coef;
-    }
-    if (part < uint32_t(kAffHigh)) {
-        int64_t w = 0;
-        for (uint32_t e = wd.ck[part]; e < wd.ck[part + 1]; e++) {
-            const AffEntryDev t = sm.ent[d][e];
-            const bool f0 = (c >> t.s0) & 1, f1 = t.s1 != 0xff && ((c >> t.s1) & 1);
-            const int64_t slope = f0 ? -t.coef : t.coef;  // S = f + y (1 - 2 f)
-            if (t.kind == 3) {
-                if (f0 && f1) K += t.coef;
-                if (f1) w += slope;
-                const int64_t q = f0 != f1 ? -t.coef : t.coef;
-                sm.q[d][l][t.pair] = t.first ? q : sm.q[d][l][t.pair] + q;
-            } else if (t.kind == 4) {
-                if (f1) w += slope;
-            } else if (t.kind == 1 || (t.kind == 2 ? f1 : f0 == f1)) {
-                if (f0) K += t.coef;
-                w += slope;
-            }
-        }
-        sm.w[d][l][part] = w;
-    }
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) K += __shfl_xor_sync(0xffffffffu, K, o);
-    if (part == 0) sm.K[d][l] = K;
-}
-
-template <typename E>
-struct Turn;  // turns of a phase in the state's precision
-template <>
-struct Turn<float2> {
-    using T = uint32_t;
-    static __device__ __forceinline__ T of(int64_t t) { return turns32(t); }
-    static __device__ __forceinline__ float2 factor(const float2 *tab, T t) { return phase_factor32(tab, t); }
-};
-template <>
-struct Turn<double2> {
-    using T = int64_t;
-    static __device__ __forceinline__ T of(int64_t t) { return t; }
-    static __device__ __forceinline__ double2 factor(const double2 *tab, T t) { return phase_factor(tab, t); }
-};
-
-// Window d applied in layout L (A: registers are high coordinates 0..3 and the thread
-// fixes 4..7; B: the other way round).
-template <int L, bool ADJ, typename E, typename SM>
-__device__ __forceinline__ void window_apply(E (&x)[kNR], E (&y)[kNR], SM &sm, uint32_t pairs, int d, uint32_t lane,
-                                             uint32_t warp)
-{
-    constexpr int RK = L == 0 ? 0 : 4, FK = 4 - RK;  // first register / fixed high coordinate
-    const uint32_t l = lane & 15u, fix = (lane >> 4) | (warp << 1);
-    int64_t a = sm.K[d][l], w[4], q[6] = {0, 0, 0, 0, 0, 0};
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        if ((fix >> i) & 1u) a += sm.w[d][l][FK + i];
-        w[i] = sm.w[d][l][RK + i];
-    }
-    if (pairs) {
-#pragma unroll
-        for (int i = 0; i < kAffHigh; i++)
-#pragma unroll
-            for (int j = i + 1; j < kAffHigh; j++) {
-                if (!((pairs >> aff_pair(i, j)) & 1u)) continue;
-                const int64_t v = sm.q[d][l][aff_pair(i, j)];
-                const bool ri = i >= RK && i < RK + 4, rj = j >= RK && j < RK + 4;
-                if (ri && rj) {
-                    constexpr int base[4] = {0, 3, 5, 6};
-                    q[base[i & 3] + (j & 3) - (i & 3) - 1] = v;
-                } else if (!ri && !rj) {
-                    if ((fix >> (i & 3)) & (fix >> (j & 3)) & 1u) a += v;
-                } else if ((fix >> ((ri ? j : i) & 3)) & 1u) {
-                    w[(ri ? i : j) & 3] += v;
-                }
-            }
-    }
-    using TT = typename Turn<E>::T;
-    const TT ta = Turn<E>::of(a);
-    TT tw[4], tq[6];
-#pragma unroll
-    for (int i = 0; i < 4; i++) tw[i] = Turn<E>::of(w[i]);
-#pragma unroll
-    for (int i = 0; i < 6; i++) tq[i] = Turn<E>::of(q[i]);
-#pragma unroll
-    for (int j = 0; j < kNR; j++) {
-        TT t = ta;
-#pragma unroll
-        for (int b = 0; b < 4; b++)
-            if ((j >> b) & 1) t += tw[b];
-        int n = 0;
-#pragma unroll
-        for (int b = 0; b < 4; b++)
-#pragma unroll
-            for (int e = b + 1; e < 4; e++, n++)
-                if (((j >> b) & 1) && ((j >> e) & 1)) t += tq[n];
-        const E ph = Turn<E>::factor(sm.exp, t);
-        x[j] = cmul(x[j], ph);
-        if constexpr (ADJ) y[j] = cmul(y[j], ph);
-    }
-}
-
-// The window's gradients, in layout A before its phases are undone: per run position the
-// sum of w and its marginals over the high coordinates and their pairs, then each term's
-// sum_r w (S ? m1 : m0) from them. P: the tile's selector bits.
-template <typename E, typename SM>
-__device__ __forceinline__ void window_grad(const E (&x)[kNR], const E (&y)[kNR], SM &sm, const AffWinDev &wd, uint64_t P,
-                                            uint32_t tid)
-{
-    double *V = reinterpret_cast<double *>(&sm.slab[0][0]);  // [kSums][16 fixed][16 run]
-    double *M = V + kSums * kThreads;                         // [1 + 8 + pairs][16 run]
-    const uint32_t lane = tid & 31u, warp = tid >> 5;
-    const uint32_t pairs = wd.pairs;
-    {
-        double v[kSums];
-#pragma unroll
-        for (int i = 0; i < kSums; i++) v[i] = 0.0;
-#pragma unroll
-        for (int j = 0; j < kNR; j++) {
-            const double w = double(y[j].x * x[j].y - y[j].y * x[j].x);  // Im(conj(lambda) psi)
-            v[0] += w;
-            int n = 5;
-#pragma unroll
-            for (int b = 0; b < 4; b++) {
-                if ((j >> b) & 1) v[1 + b] += w;
-#pragma unroll
-                for (int e = b + 1; e < 4; e++, n++)
-                    if (((j >> b) & 1) && ((j >> e) & 1)) v[n] += w;
-            }
-        }
-        const uint32_t at = (((lane >> 4) | (warp << 1)) << 4) | (lane & 15u);
-#pragma unroll
-        for (int i = 0; i < kSums; i++)
-            if (i < 5 || pairs) V[i * kThreads + at] = v[i];
-    }
-    __syncthreads();
-    const uint32_t l = tid & 15u, part = tid >> 4;
-    const uint32_t rows = 9u + uint32_t(__popc(pairs));
-    for (uint32_t r = part; r < rows; r += 16u) {
-        uint32_t src = 0, need = 0;  // row of V, fixed bits that must be set
-        if (r >= 1 && r < 9) {
-            if (r < 5) src = r;
-            else need = 1u << (r - 5);
-        } else if (r >= 9) {
-            const uint32_t p = sm.plist[r - 9];
-            const uint32_t i = p & 15u, j = p >> 4;
-            if (j < 4) src = 5u + (i == 0 ? j - 1 : i == 1 ? j + 1 : 5u);  // (0,1) (0,2) (0,3) (1,2) (1,3) (2,3)
-            else if (i < 4) src = 1u + i, need = 1u << (j - 4);
-            else need = (1u << (i - 4)) | (1u << (j - 4));
-        }
-        double s = 0.0;
-#pragma unroll
-        for (uint32_t f = 0; f < 16; f++)
-            if ((f & need) == need) s += V[src * kThreads + (f << 4) + l];
-        M[r * kRun + l] = s;
-    }
-    __syncthreads();
-    const uint64_t c = P ^ sm.lw[l];
-    const double W = M[l];
-    for (uint32_t t0 = 0; t0 < wd.nterms; t0 += 16u) {
-        const uint32_t t = t0 + part;
-        const bool live = t < wd.nterms;
-        const AffTermDev tm = sm.term[live ? t : 0];
-        const bool f0 = (c >> tm.s0) & 1, two = tm.s1 != 0xff, f1 = two && ((c >> tm.s1) & 1);
-        double s;
-        if (tm.k0 == 0xff) {
-            s = f0 && (!two || f1) ? W : 0.0;
-        } else {
-            const double M0 = M[(1u + tm.k0) * kRun + l], S0 = f0 ? W - M0 : M0;
-            if (!two) s = S0;
-            else if (tm.k1 == 0xff) s = f1 ? S0 : 0.0;
-            else if (tm.k1 == tm.k0) s = f0 == f1 ? S0 : 0.0;
-            else {
-                const double M1 = M[(1u + tm.k1) * kRun + l], M01 = M[(9u + tm.pair) * kRun + l];
-                s = f0 ? (f1 ? W - M0 - M1 + M01 : M1 - M01) : (f1 ? M0 - M01 : M01);
-            }
-        }
-        const double g0 = tm.gk == 1 ? 1.0 : 0.0, g1 = tm.gk == 1 ? -1.0 : -2.0;
-        double g = live && tm.gk ? g0 * W + (g1 - g0) * s : 0.0;
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
-        if (live && l == 0) sm.tacc[t] += g;
-    }
-}
+using namespace adev;
 
 template <typename E, bool ADJ, bool REAL>
 __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? (ADJ ? 2 : 3) : (ADJ ? 1 : 2))
     affine_kernel(const uint8_t *__restrict__ blob, uint64_t poff, uint64_t toff, E *psi, const E *src, E *lam,
-                  double *grads)
+                  double *grads, uint64_t ntiles)
 {
-    using SM = AffSmem<E, ADJ>;
-    using RT = typename ET<E>::R;
     extern __shared__ __align__(128) unsigned char s_raw[];
-    SM &sm = *reinterpret_cast<SM *>(s_raw);
-    const AffDev &p = *reinterpret_cast<const AffDev *>(blob + poff);
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t mask = p.gates, nsel = p.nsel;
-    const AffWinDev &w0 = sm.win[0], &w1 = sm.win[SM::NW - 1];
-    const bool win0 = p.win[0].nterms != 0, win1 = !ADJ && p.win[1].nterms != 0;
-
-    // tables
-    if (tid < SM::NW) sm.win[tid] = p.win[tid];
-    __syncthreads();
-    if (win0 || win1) {
-        const E *tab = reinterpret_cast<const E *>(blob + toff);
-        for (uint32_t i = tid; i < (1u << kExpTableBits); i += kThreads) sm.exp[i] = tab[i];
-        for (int d = 0; d < SM::NW; d++) {
-            const AffWinDev &wd = sm.win[d];
-            const AffEntryDev *e = reinterpret_cast<const AffEntryDev *>(blob + wd.off_entries);
-            for (uint32_t i = tid; i < wd.ck[kAffHigh]; i += kThreads) sm.ent[d][i] = e[i];
-        }
-    }
-    if (tid < kAffBits) {
-        const AffGateDev &g = p.gate[tid];
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            sm.u[tid][0][i] = RT(g.u[i]);
-            sm.u[tid][1][i] = RT(g.u[i ^ 6]);  // [[u11, u10], [u01, u00]]
-        }
-        sm.sel[tid] = g.sel;
-        sm.gen[tid] = g.gen;
-        sm.basis[tid] = p.basis[tid];
-    }
-    if (tid >= 32 && tid < 32 + kAffMaxSel) sm.alpha[tid - 32] = p.alpha[tid - 32];
-    if (tid >= 96 && tid < 96 + kRun) sm.lw[tid - 96] = p.lw[tid - 96];
-    if constexpr (ADJ) {
-        const AffTermDev *t = reinterpret_cast<const AffTermDev *>(blob + w0.off_terms);
-        for (uint32_t i = tid; i < w0.nterms; i += kThreads) {
-            sm.term[i] = t[i];
-            sm.tacc[i] = 0.0;
-        }
-#pragma unroll
-        for (int k = 0; k < kAffBits; k++) sm.gacc[k][tid] = 0.0;
-        if (tid == 128) {
-            int n = 0;
-            for (int i = 0; i < kAffHigh; i++)
-                for (int j = i + 1; j < kAffHigh; j++)
-                    if ((w0.pairs >> aff_pair(i, j)) & 1u) sm.plist[n++] = uint8_t(i | (j << 4));
-        }
-    }
-    __syncthreads();
-
-    // the thread's part of the address in layouts A and B
-    uint64_t ra = 0, rb = 0;
-#pragma unroll
-    for (int b = 0; b < 5; b++)
-        if ((lane >> b) & 1u) {
-            ra ^= sm.basis[b < 4 ? b : 8];
-            rb ^= sm.basis[b];
-        }
-#pragma unroll
-    for (int b = 0; b < 3; b++)
-        if ((warp >> b) & 1u) {
-            ra ^= sm.basis[9 + b];
-            rb ^= sm.basis[5 + b];
-        }
-    const uint64_t tr0 = p.tr[lane], tr1 = p.tr[lane + 32u];
-    const bool need_c = (mask & 0x00fu) != 0, need_b = need_c || (mask & 0xf00u) != 0 || win1;
-    const uint64_t ntiles = p.ntiles;
-    const uint64_t lw = sm.lw[lane & 15u], lw0 = sm.lw[0], lwe = sm.lw[tid >> 4];
-
-    auto tile_base = [&](uint64_t t) {
-        const uint64_t rl = (((t >> lane) & 1u) ? tr0 : 0) ^ (((t >> (lane + 32u)) & 1u) ? tr1 : 0);
-        return (uint64_t(__reduce_xor_sync(0xffffffffu, uint32_t(rl >> 32))) << 32) |
-               __reduce_xor_sync(0xffffffffu, uint32_t(rl));
-    };
-    // the run of 16 amplitudes this thread asks L2 for, one tile ahead
-    uint64_t rp = 0;
-#pragma unroll
-    for (int b = 0; b < kAffHigh; b++)
-        if ((tid >> b) & 1u) rp ^= sm.basis[kAffRun + b];
-
-    uint64_t rn = tile_base(blockIdx.x);
-    for (uint64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const uint64_t r0 = rn;
-        auto addr = [&](uint64_t base, int k0, int j) {
-#pragma unroll
-            for (int b = 0; b < 4; b++)
-                if ((j >> b) & 1) base ^= sm.basis[k0 + b];
-            return base;
-        };
-        E x[kNR], y[kNR];
-#pragma unroll
-        for (int j = 0; j < kNR; j++) {
-            const uint64_t r = addr(r0 ^ ra, 4, j);
-            x[j] = __ldcg(src + r);
-            if constexpr (ADJ) y[j] = __ldcg(lam + r);
-        }
-        if (t + gridDim.x < ntiles) {
-            rn = tile_base(t + gridDim.x);
-            const uint64_t r = (rn ^ rp) & ~uint64_t(kRun - 1);
-#pragma unroll
-            for (int i = 0; i < int(sizeof(E)) / 8; i++) {
-                prefetch_l2(src + r + i * (kRun / 2));
-                if constexpr (ADJ) prefetch_l2(lam + r + i * (kRun / 2));
-            }
-        }
-        // selector bits of the tile: lane s takes selectors s and s + 32
-        const bool b0 = lane < nsel && par64(sm.alpha[lane] & r0);
-        const bool b1 = lane + 32u < nsel && par64(sm.alpha[lane + 32u] & r0);
-        const uint64_t P = uint64_t(__ballot_sync(0xffffffffu, b0)) | (uint64_t(__ballot_sync(0xffffffffu, b1)) << 32);
-        const uint64_t c = P ^ lw;
-        if (win0 || win1) {
-            __syncthreads();  // the previous tile's polynomials and sums are read
-            if (win0) window_eval(sm, w0, 0, P ^ lwe, tid & 15u, tid >> 4);
-            if constexpr (!ADJ) {
-                if (win1) window_eval(sm, w1, 1, P ^ lwe, tid & 15u, tid >> 4);
-            }
-            __syncthreads();
-        }
-        if (win0) {
-            if constexpr (ADJ) window_grad(x, y, sm, w0, P, tid);
-            window_apply<0, ADJ>(x, y, sm, w0.pairs, 0, lane, warp);
-        }
-        gates<4, ADJ, REAL>(x, y, mask, c, sm, tid);
-        if (need_c) {
-            exchange<0, 2, ADJ ? 2 : 1>(x, y, sm.slab, lane, warp);
-            gates<0, ADJ, REAL>(x, y, mask, P ^ lw0, sm, tid);
-            exchange<2, 1, ADJ ? 2 : 1>(x, y, sm.slab, lane, warp);
-        } else if (need_b) {
-            exchange<0, 1, ADJ ? 2 : 1>(x, y, sm.slab, lane, warp);
-        }
-        if (need_b) gates<8, ADJ, REAL>(x, y, mask, c, sm, tid);
-        if constexpr (!ADJ) {
-            if (win1) window_apply<1, false>(x, y, sm, w1.pairs, 1, lane, warp);
-        }
-        const uint64_t rs = r0 ^ (need_b ? rb : ra);
-        const int ks = need_b ? 8 : 4;
-#pragma unroll
-        for (int j = 0; j < kNR; j++) {
-            const uint64_t r = addr(rs, ks, j);
-            __stcg(psi + r, x[j]);
-            if constexpr (ADJ) __stcg(lam + r, y[j]);
-        }
-    }
-    if constexpr (ADJ) {
-        __syncthreads();
-        for (uint32_t i = tid; i < w0.nterms; i += kThreads)
-            if (sm.term[i].gk) atomicAdd(&grads[sm.term[i].slot], sm.tacc[i]);
-        // warp w sums gates w and w + 8
-        for (uint32_t k = warp; k < uint32_t(kAffBits); k += kThreads / 32) {
-            if (!((mask >> k) & 1u) || !sm.gen[k]) continue;
-            double s = 0.0;
-            for (int i = 0; i < kThreads / 32; i++) s += sm.gacc[k][i * 32 + int(lane)];
-            s = warp_sum_f64(s);
-            if (lane == 0) atomicAdd(&grads[p.gate[k].slot], s);
-        }
-    }
+    chain_trigger();
+    affine_body<E, ADJ, REAL>(*reinterpret_cast<AffSmem<E, ADJ> *>(s_raw), blob, poff, toff, psi, src, lam, grads,
+                              blockIdx.x, gridDim.x, ntiles);
 }
 
 template <typename E, bool ADJ, bool REAL>
 cudaError_t launch_affine(const uint8_t *blob, uint64_t poff, uint64_t toff, uint64_t ntiles, E *psi, const E *src, E *lam,
-                          double *grads, int sms, cudaStream_t st)
+                          double *grads, bool chained, int sms, cudaStream_t st)
 {
     auto kern = affine_kernel<E, ADJ, REAL>;
     const int smem = int(sizeof(AffSmem<E, ADJ>));
@@ -523,31 +56,31 @@ cudaError_t launch_affine(const uint8_t *blob, uint64_t poff, uint64_t toff, uin
     int per_sm = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, size_t(smem));
     const unsigned grid = unsigned(std::min<uint64_t>(ntiles, uint64_t(sms) * uint64_t(std::max(1, per_sm))));
-    kern<<<grid, kThreads, size_t(smem), st>>>(blob, poff, toff, psi, src ? src : psi, lam, grads);
-    return cudaGetLastError();
+    return launch_chained(chained, kern, grid, kThreads, size_t(smem), st, blob, poff, toff, psi,
+                          src ? src : static_cast<const E *>(psi), lam, grads, ntiles);
 }
 
 template <typename E>
 cudaError_t affine_typed(bool real, const uint8_t *blob, uint64_t poff, uint64_t toff, uint64_t ntiles, E *psi, const E *src,
-                         E *lam, double *grads, int sms, cudaStream_t st)
+                         E *lam, double *grads, bool chained, int sms, cudaStream_t st)
 {
     if (lam)
-        return real ? launch_affine<E, true, true>(blob, poff, toff, ntiles, psi, src, lam, grads, sms, st)
-                    : launch_affine<E, true, false>(blob, poff, toff, ntiles, psi, src, lam, grads, sms, st);
-    return real ? launch_affine<E, false, true>(blob, poff, toff, ntiles, psi, src, lam, grads, sms, st)
-                : launch_affine<E, false, false>(blob, poff, toff, ntiles, psi, src, lam, grads, sms, st);
+        return real ? launch_affine<E, true, true>(blob, poff, toff, ntiles, psi, src, lam, grads, chained, sms, st)
+                    : launch_affine<E, true, false>(blob, poff, toff, ntiles, psi, src, lam, grads, chained, sms, st);
+    return real ? launch_affine<E, false, true>(blob, poff, toff, ntiles, psi, src, lam, grads, chained, sms, st)
+                : launch_affine<E, false, false>(blob, poff, toff, ntiles, psi, src, lam, grads, chained, sms, st);
 }
 
 }  // namespace
 
 cudaError_t run_affine(const uint8_t *dblob, uint64_t poff, uint64_t toff, uint64_t ntiles, int elem_bytes, bool real,
-                       void *psi, const void *psi_src, void *lam, double *grads, int sms, cudaStream_t st)
+                       void *psi, const void *psi_src, void *lam, double *grads, bool chained, int sms, cudaStream_t st)
 {
     if (elem_bytes == 8)
         return affine_typed(real, dblob, poff, toff, ntiles, static_cast<float2 *>(psi),
-                            static_cast<const float2 *>(psi_src), static_cast<float2 *>(lam), grads, sms, st);
+                            static_cast<const float2 *>(psi_src), static_cast<float2 *>(lam), grads, chained, sms, st);
     return affine_typed(real, dblob, poff, toff, ntiles, static_cast<double2 *>(psi),
-                        static_cast<const double2 *>(psi_src), static_cast<double2 *>(lam), grads, sms, st);
+                        static_cast<const double2 *>(psi_src), static_cast<double2 *>(lam), grads, chained, sms, st);
 }
 
 }  // namespace zxh

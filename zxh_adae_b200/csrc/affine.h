@@ -94,8 +94,8 @@ struct AffBuild {
 
 // The pass at poff of the blob over psi (read from psi_src where given); lam != nullptr:
 // the adjoint form, gradients added to grads[slot]. toff: the phase table (unused without
-// windows).
+// windows). chained: directly after another kernel of the run (chain.cuh).
 cudaError_t run_affine(const uint8_t *dblob, uint64_t poff, uint64_t toff, uint64_t ntiles, int elem_bytes, bool real,
-                       void *psi, const void *psi_src, void *lam, double *grads, int sms, cudaStream_t st);
+                       void *psi, const void *psi_src, void *lam, double *grads, bool chained, int sms, cudaStream_t st);
 
 }  // namespace zxh

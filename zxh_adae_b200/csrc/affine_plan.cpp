@@ -27,15 +27,22 @@ void insert(uint64_t v, std::vector<uint64_t> &ech)
 
 }  // namespace
 
-bool AffBuild::Room::add(uint64_t delta)
+int AffBuild::Room::add(uint64_t delta)
 {
-    const uint64_t high = delta >> kAffRun;
-    if (!high) return delta != 0;  // deltas of distinct qubits are independent: at most 4 lie in the run
-    if (ech.size() >= size_t(kAffHigh)) return false;
-    const uint64_t v = reduced(high, ech);
-    if (!v) return false;
-    insert(v, ech);
-    return true;
+    uint64_t v = delta;  // delta modulo the high deltas, their parts' leading bits cleared
+    for (const High &h : high)
+        if ((v >> (kAffRun + top_bit(h.part))) & 1) v ^= h.delta;
+    if (v >> kAffRun) {
+        if (high.size() >= size_t(kAffHigh)) return -1;
+        high.push_back({v >> kAffRun, v});
+        std::sort(high.begin(), high.end(), [](const High &x, const High &y) { return x.part > y.part; });
+        return 1;
+    }
+    if (low.size() >= size_t(kAffRun)) return -1;
+    v = reduced(v, low);
+    if (!v) return -1;
+    insert(v, low);
+    return 0;
 }
 
 bool AffBuild::init(int eb, int mm, const std::vector<U3Op> &gates, const std::vector<uint64_t> &deltas, bool adjoint_matrix,
@@ -51,25 +58,22 @@ bool AffBuild::init(int eb, int mm, const std::vector<U3Op> &gates, const std::v
     real = true;
     if (m < kAffBits) return false;
     dev.m = uint32_t(m);
-    std::vector<uint64_t> low, high;
+    Room room;
     int nlow = 0, nhigh = 0;
     std::vector<int> at;
     for (const U3Op &g : gates) {
         if (g.has_ctrl || !g.delta) return false;
-        const bool inside = (g.delta >> kAffRun) == 0;
-        std::vector<uint64_t> &ech = inside ? low : high;
-        const uint64_t v = reduced(inside ? g.delta : g.delta >> kAffRun, ech);
-        if (!v || (inside ? nlow == kAffRun : nhigh == kAffHigh)) return false;
-        insert(v, ech);
-        at.push_back(inside ? nlow++ : kAffRun + nhigh++);
+        const int kind = room.add(g.delta);
+        if (kind < 0) return false;
+        at.push_back(kind ? kAffRun + nhigh++ : nlow++);
         dev.basis[at.back()] = g.delta;
     }
-    // The run's other basis vectors are single bits, moved by the run's gates' deltas so that
+    // The run's other basis vectors are single bits, moved by the low gates' deltas so that
     // no selector of those gates sees them.
     for (int b = 0; b < kAffRun && nlow < kAffRun; b++) {
-        const uint64_t r = reduced(1ULL << b, low);
+        const uint64_t r = reduced(1ULL << b, room.low);
         if (!r) continue;
-        insert(r, low);
+        insert(r, room.low);
         uint64_t v = 1ULL << b;
         for (size_t i = 0; i < gates.size(); i++)
             if (at[i] < kAffRun && parity64(gates[i].sel.alpha & (1ULL << b))) v ^= gates[i].delta;
@@ -82,14 +86,11 @@ bool AffBuild::init(int eb, int mm, const std::vector<U3Op> &gates, const std::v
     std::sort(others.begin(), others.end());
     for (uint64_t d : others) {
         if (nhigh == kAffHigh) break;
-        const uint64_t v = reduced(d >> kAffRun, high);
-        if (!v) continue;
-        insert(v, high);
-        dev.basis[kAffRun + nhigh++] = d;
+        if (room.add(d) == 1) dev.basis[kAffRun + nhigh++] = d;
     }
     if (nlow != kAffRun || nhigh != kAffHigh) return false;
     uint64_t piv = low_mask(kAffRun);
-    for (uint64_t v : high) piv |= 1ULL << (top_bit(v) + kAffRun);
+    for (const Room::High &h : room.high) piv |= 1ULL << (top_bit(h.part) + kAffRun);
     int t = 0;
     for (int b = 0; b < m; b++)
         if (!((piv >> b) & 1)) dev.tr[t++] = 1ULL << b;

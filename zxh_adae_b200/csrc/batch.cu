@@ -10,6 +10,7 @@
 // depends on, so the tasks a CTA waits for were taken earlier by CTAs that are
 // running: no co-residency is needed. State loads and stores go through L2
 // (.cg), and each task fences its stores before it is counted.
+#include "affine_dev.cuh"
 #include "batch.h"
 #include "dev.cuh"
 #include "grow_dev.cuh"
@@ -132,12 +133,24 @@ __device__ __forceinline__ void diag_adj_body(E *psi, E *lam, uint64_t b, uint64
 template <typename E, bool REAL, int NT>
 __device__ __forceinline__ void run_op_slice(const BatchOp &op, const uint8_t *blob, E *arena, double *grads,
                                              double *energies, uint64_t b, uint64_t e, uint64_t first, uint64_t step,
-                                             BatchShared<E, NT> &sm)
+                                             BatchShared<E, NT> &sm, unsigned char *tile)
 {
     const uint8_t *ob = blob + op.base;
     E *psi = arena + op.psi;
     E *lam = arena + op.lam;
     double *gr = grads + op.grad_base;
+    if constexpr (NT == kThreads) {  // tile: dynamic shared memory of the affine passes
+        if (op.kind == BOP_AFFINE) {
+            adev::affine_body<E, false, REAL>(*reinterpret_cast<adev::AffSmem<E, false> *>(tile), ob, op.off0, op.off1, psi,
+                                              psi, nullptr, nullptr, b, 1, e);
+            return;
+        }
+        if (op.kind == BOP_AFFINE_ADJ) {
+            adev::affine_body<E, true, REAL>(*reinterpret_cast<adev::AffSmem<E, true> *>(tile), ob, op.off0, op.off1, psi,
+                                             psi, lam, gr, b, 1, e);
+            return;
+        }
+    }
     switch (op.kind) {
     case BOP_INIT: init_body<E, NT>(psi, b, e); break;
     case BOP_GROW:
@@ -172,10 +185,11 @@ __device__ __forceinline__ void run_op_slice(const BatchOp &op, const uint8_t *b
     }
 }
 
-// NT threads per CTA, 2048 / NT... resident CTAs per SM at 128 registers: 16 warps
-// per SM whatever NT is.
+// NT threads per CTA, 512 / NT resident CTAs per SM at 128 registers: 16 warps per SM
+// whatever NT is. The 256-thread complex128 form runs affine passes whose two states fill
+// an SM's shared memory: one CTA per SM, at twice the registers.
 template <typename E, bool REAL, int NT>
-__global__ void __launch_bounds__(NT, 512 / NT) batch_kernel(const uint8_t *__restrict__ blob,
+__global__ void __launch_bounds__(NT, NT == kThreads && sizeof(E) == 16 ? 1 : 512 / NT) batch_kernel(const uint8_t *__restrict__ blob,
                                                              const BatchOp *__restrict__ ops,
                                                              const BatchTask *__restrict__ tasks, uint32_t ntasks,
                                                              uint32_t *next, uint32_t *remaining, E *arena,
@@ -183,6 +197,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) batch_kernel(const uint8_t *__re
                                                              long long spin_limit)
 {
     __shared__ BatchShared<E, NT> sm;
+    extern __shared__ __align__(128) unsigned char s_tile[];
     __shared__ uint32_t s_task, s_abort;
     for (;;) {
         __syncthreads();
@@ -211,7 +226,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) batch_kernel(const uint8_t *__re
         if (s_abort) break;
         const bool grow = op.kind == BOP_GROW || op.kind == BOP_GROW_ADJ;
         run_op_slice<E, REAL, NT>(op, blob, arena, grads, energies, task.begin, task.end, grow ? task.begin : 0,
-                                  grow ? uint64_t(NT / 32) : 0, sm);
+                                  grow ? uint64_t(NT / 32) : 0, sm, s_tile);
         __threadfence();
         __syncthreads();
         if (threadIdx.x == 0) atomicSub(&remaining[task.op], 1u);
@@ -224,9 +239,16 @@ cudaError_t persistent_typed(const uint8_t *blob, const BatchOp *ops, const Batc
                              DevStatus *status, long long spin_limit, int sms, cudaStream_t st)
 {
     int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel<E, REAL, NT>, NT, 0);
+    size_t smem = 0;
+    if (NT == kThreads) {
+        smem = sizeof(adev::AffSmem<E, true>);
+        const cudaError_t e = cudaFuncSetAttribute(batch_kernel<E, REAL, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   int(smem));
+        if (e != cudaSuccess) return e;
+    }
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel<E, REAL, NT>, NT, smem);
     if (per_sm < 1) per_sm = 1;
-    batch_kernel<E, REAL, NT><<<unsigned(sms * per_sm), NT, 0, st>>>(blob, ops, tasks, ntasks, next, remaining, arena,
+    batch_kernel<E, REAL, NT><<<unsigned(sms * per_sm), NT, smem, st>>>(blob, ops, tasks, ntasks, next, remaining, arena,
                                                                      grads, energies, status, spin_limit);
     return cudaGetLastError();
 }

@@ -19,6 +19,8 @@ enum BatchOpKind : uint32_t {
     BOP_LAMBDA = 2,    // lambda := H psi, energy += <psi|H|psi>
     BOP_GROW_ADJ = 3,  // general strided adjoint pass on psi and lambda, gradients
     BOP_DIAG_ADJ = 4,  // adjoint diagonal group on psi and lambda, gradients
+    BOP_AFFINE = 5,    // affine tile pass on psi (256-thread CTAs)
+    BOP_AFFINE_ADJ = 6,  // affine tile pass on psi and lambda, gradients
 };
 
 constexpr uint32_t kNoDep = 0xffffffffu;
@@ -26,11 +28,11 @@ constexpr int kBatchDiagMax = 16;  // diagonal gates per adjoint group in the ba
 
 struct BatchOp {
     uint32_t kind, R, circuit, dep;  // dep: index of the op this one waits for
-    uint64_t units;                  // items (grow passes) or amplitudes
+    uint64_t units;                  // items (grow passes), tiles (affine passes) or amplitudes
     uint64_t base;                   // this op's descriptors start at blob + base
-    uint64_t off0, off1, off2;       // GROW*: pass descriptor, phase table; LAMBDA: terms;
+    uint64_t off0, off1, off2;       // GROW*, AFFINE*: pass descriptor, phase table; LAMBDA: terms;
                                      // DIAG_ADJ: gates, slots, phase table (all from base)
-    uint32_t aux, m;                 // LAMBDA: terms; DIAG_ADJ: gates; GROW*: 1 if every gate is real; m: state bits
+    uint32_t aux, m;                 // LAMBDA: terms; DIAG_ADJ: gates; GROW*, AFFINE*: 1 if every gate is real; m: state bits
     uint64_t psi, lam;               // element offsets of the circuit's states in the arena
     uint32_t grad_base, energy;      // the circuit's first gradient slot and its energy slot
 };

@@ -132,6 +132,7 @@ int compile(zxh_batch *b)
     b->arena_elems = 0;
     zxh::PlanParams pp;
     pp.grow_only = 1;
+    pp.grow_tiles = b->threads == 256;  // the affine tile passes' CTA
     pp.grow_regs = b->grow_regs;
     pp.adj_regs = b->adj_regs;  // the persistent kernel runs reverse passes of at most 3 register coordinates
     std::vector<uint8_t> etab;
@@ -171,7 +172,8 @@ int compile(zxh_batch *b)
             op.energy = uint32_t(c);
             op.dep = b->chain[c].empty() ? zxh::kNoDep : b->chain[c].back();
             const uint64_t sb = uint64_t(b->eb) << N;  // one state
-            b->bytes += op.kind == zxh::BOP_INIT ? sb : (op.kind == zxh::BOP_GROW || op.kind == zxh::BOP_LAMBDA) ? 2 * sb : 4 * sb;
+            const bool one = op.kind == zxh::BOP_GROW || op.kind == zxh::BOP_AFFINE || op.kind == zxh::BOP_LAMBDA;
+            b->bytes += op.kind == zxh::BOP_INIT ? sb : one ? 2 * sb : 4 * sb;
             b->chain[c].push_back(uint32_t(b->ops.size()));
             b->ops.push_back(op);
         };
@@ -189,6 +191,13 @@ int compile(zxh_batch *b)
                 op.off0 = ps.off;
                 op.off1 = ps.off2;
                 op.aux = ps.gb.all_real() ? 1u : 0u;
+            } else if (ps.kind == zxh::Pass::AFFINE) {
+                op.kind = zxh::BOP_AFFINE;
+                op.units = ps.aff->dev.ntiles;
+                op.base = base;
+                op.off0 = ps.off;
+                op.off1 = ps.off2;
+                op.aux = ps.aff->real ? 1u : 0u;
             } else {
                 return bfail(b, ZXH_ERR_ARG, "circuit " + std::to_string(c) +
                                                  " needs a pass the batched launch does not run (n >= 6 required)");
@@ -228,6 +237,13 @@ int compile(zxh_batch *b)
                 op.off0 = r.off;
                 op.off1 = r.toff;
                 op.aux = r.gb.all_real() ? 1u : 0u;
+            } else if (r.kind == zxh::adj::RevStep::AFFINE) {
+                op.kind = zxh::BOP_AFFINE_ADJ;
+                op.units = r.aff->dev.ntiles;
+                op.base = gbase;
+                op.off0 = r.off;
+                op.off1 = r.toff;
+                op.aux = r.aff->real ? 1u : 0u;
             } else if (r.kind == zxh::adj::RevStep::DIAG) {
                 op.kind = zxh::BOP_DIAG_ADJ;
                 op.units = uint64_t(1) << N;
@@ -257,7 +273,12 @@ void make_tasks(zxh_batch *b)
             const uint32_t oi = b->chain[c][L];
             const BatchOp &op = b->ops[oi];
             const bool grow = op.kind == zxh::BOP_GROW || op.kind == zxh::BOP_GROW_ADJ;
-            const uint64_t per = grow ? uint64_t(b->task_items) : uint64_t(b->task_elems);
+            const bool tiles = op.kind == zxh::BOP_AFFINE || op.kind == zxh::BOP_AFFINE_ADJ;
+            // a tile is four strided items' amplitudes (complex64, 16 rows); a quarter of their
+            // task keeps a circuit's tiles on more CTAs
+            const uint64_t per = grow    ? uint64_t(b->task_items)
+                                 : tiles ? uint64_t(std::max(1, b->task_items / 16))
+                                         : uint64_t(b->task_elems);
             for (uint64_t s = 0; s < op.units; s += per) {
                 BatchTask t;
                 t.op = oi;
@@ -341,6 +362,14 @@ int launch_op(zxh_batch *b, const BatchOp &op)
         e = zxh::run_grow(b->d_blob + op.base, op.off0, op.off1, int(op.R), op.units, b->eb, psi, nullptr, nullptr,
                           op.aux != 0, (zxh::PlanParams().grow_staged & 2) != 0, b->d_status, b->sms, b->stream);
         break;
+    case zxh::BOP_AFFINE:
+        e = zxh::run_affine(b->d_blob + op.base, op.off0, op.off1, op.units, b->eb, op.aux != 0, psi, nullptr, nullptr,
+                            nullptr, false, b->sms, b->stream);
+        break;
+    case zxh::BOP_AFFINE_ADJ:
+        e = zxh::run_affine(b->d_blob + op.base, op.off0, op.off1, op.units, b->eb, op.aux != 0, psi, nullptr, lam, gr,
+                            false, b->sms, b->stream);
+        break;
     case zxh::BOP_LAMBDA:
         e = zxh::run_lambda(psi, lam, int(op.m), b->eb, reinterpret_cast<const zxh::TermDev *>(b->d_blob + op.off0),
                             op.aux, b->d_energy + op.energy, b->sms, b->stream);
@@ -367,7 +396,8 @@ int build(zxh_batch *b)
     if (int rc = compile(b)) return rc;
     b->real = true;
     for (const BatchOp &op : b->ops)
-        if ((op.kind == zxh::BOP_GROW || op.kind == zxh::BOP_GROW_ADJ) && !op.aux) b->real = false;
+        if ((op.kind == zxh::BOP_GROW || op.kind == zxh::BOP_GROW_ADJ || op.kind == zxh::BOP_AFFINE ||
+             op.kind == zxh::BOP_AFFINE_ADJ) && !op.aux) b->real = false;
     make_tasks(b);
     return upload(b);
 }
@@ -528,15 +558,17 @@ int zxh_batch_set(zxh_batch *b, const char *name, int value)
         return bfail(b, ZXH_ERR_ARG, std::string(name) + " must be in [" + std::to_string(lo) + ", " +
                                          std::to_string(hi) + "]" +
                                          (field == &b->threads ? " and one of 64, 128, 256" : ""));
+    // only 256-thread CTAs run affine tile passes: another pass set on either side
+    const bool other_passes = field == &b->threads && (b->threads == 256) != (value == 256);
     *field = value;
     BCK(b, cudaSetDevice(b->device), "cudaSetDevice");
-    if (field == &b->wait_limit_log2 || field == &b->threads) {
+    if (field == &b->wait_limit_log2 || (field == &b->threads && !other_passes)) {
         // launch parameters: only the captured graph holds the old value
         BCK(b, cudaStreamSynchronize(b->stream), "sync");
         drop_graph(b);
         return ZXH_OK;
     }
-    return (field == &b->grow_regs || field == &b->adj_regs) ? build(b) : retask(b);
+    return (field == &b->grow_regs || field == &b->adj_regs || other_passes) ? build(b) : retask(b);
 }
 
 int zxh_batch_get(const zxh_batch *b, const char *name, int *value)
@@ -606,12 +638,14 @@ int zxh_batch_tune(zxh_batch *b, int reps)
         if (nt == best_n) continue;
         const int keep = b->threads;
         b->threads = nt;
+        if (int rc = build(b)) return rc;  // the pass set depends on it
         double t;
         if (int rc = timed(t)) return rc;
         if (t < best) best = t, best_n = nt;
         b->threads = keep;
     }
     b->threads = best_n;
+    if (int rc = build(b)) return rc;
     // 3. register coordinates per reverse pass (fewer: more passes, less register pressure)
     int best_a = b->adj_regs;
     for (int a = 1; a <= 3; a++) {

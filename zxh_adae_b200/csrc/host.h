@@ -60,6 +60,7 @@ struct PlanParams {
                                 // states of at least 2^12 amplitudes whose qubits are all expanded
     int grow_regs = 4;          // register coordinates (gates with high deltas) per general strided pass
     int grow_only = 0;          // 1: only INIT and general strided passes (the persistent batch kernel's set)
+    int grow_tiles = 0;         // 1: grow_only plans may use affine tile passes
     int adj_windows = 1;        // adjoint sweep: diagonal gates ride in the general strided passes as windows
     int adj_regs = 4;           // adjoint sweep: gates with high deltas per strided pass (4 runs at one CTA per SM)
     int grow_staged = 1;        // general strided passes whose warps stage their next item in shared memory

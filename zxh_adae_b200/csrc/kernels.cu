@@ -12,6 +12,7 @@
 //                   stores it back once. Replaces u3_block_batch_kernel_cuda (one grid
 //                   sweep per descriptor, kernel_cuda.cu:390-423) and
 //                   diag_block_kernel_cuda (kernel_cuda.cu:505-614).
+#include "chain.cuh"
 #include "core.h"
 #include "dev.cuh"
 #include "host.h"
@@ -32,6 +33,7 @@ __global__ void __launch_bounds__(kThreads) product_kernel(const uint8_t *__rest
 {
     using VT = typename ET<E>::VT;
     constexpr int V = ET<E>::V;
+    chain_trigger();
     const ProductDev p = *reinterpret_cast<const ProductDev *>(blob + off);
     const E *L = reinterpret_cast<const E *>(blob + tab_off);
     const E *M = L + (1u << p.c0);
@@ -518,7 +520,7 @@ cudaError_t run_passes(const std::vector<Pass> &passes, const uint8_t *dblob, vo
             e = cudaGetLastError();
         } else if (ps.kind == Pass::ROW) {
             e = run_row_pass(dblob, ps.off, ps.off2, ps.row.nitems, elem_bytes, ps.wide, ps.low != 0, ps.real != 0,
-                             ps.row.off_pre != 0 || ps.row.off_post != 0, state, sms, st);
+                             ps.row.off_pre != 0 || ps.row.off_post != 0, state, i > 0, sms, st);
         } else if (ps.kind == Pass::FAST) {
             e = run_fast_tile(dblob, ps.off, ps.off2, ps.geom.ntiles, elem_bytes, state, status, sms, st);
         } else if (ps.kind == Pass::INIT) {
@@ -531,19 +533,19 @@ cudaError_t run_passes(const std::vector<Pass> &passes, const uint8_t *dblob, vo
             void *dst = (i + 1 == passes.size() && last_dst) ? last_dst : state;
             const void *src = (i == 0 && first_src) ? first_src : (dst != state ? state : nullptr);
             e = run_grow(dblob, ps.off, ps.off2, int(ps.gb.regs.size()), ps.gb.dev.nitems, elem_bytes, dst, nullptr,
-                         nullptr, ps.gb.all_real(), ps.prefetch != 0, status, sms, st, src);
+                         nullptr, ps.gb.all_real(), ps.prefetch != 0, status, sms, st, src, i > 0);
         } else if (ps.kind == Pass::AFFINE) {
             void *dst = (i + 1 == passes.size() && last_dst) ? last_dst : state;
             const void *src = (i == 0 && first_src) ? first_src : (dst != state ? state : nullptr);
             e = run_affine(dblob, ps.off, ps.off2, ps.aff->dev.ntiles, elem_bytes, ps.aff->real, dst, src, nullptr,
-                           nullptr, sms, st);
+                           nullptr, i > 0, sms, st);
         } else if (ps.kind == Pass::DIAG) {
             e = run_diag(dblob, ps.off, ps.off2, ps.m, elem_bytes, ps.row_bits, ps.chunk_bits, ps.prefetch != 0, state, status,
                          sms, st);
         } else if (ps.kind == Pass::SPAN) {
             e = run_span(dblob, ps.off, ps.off2, ps.span.ntiles, elem_bytes, ps.low != 0,
                          span_layouts(elem_bytes, ps.span.gates, ps.low != 0, ps.prefetch != 0), ps.prefetch != 0,
-                         ps.real, state, ps.span.rot, ps.span.pos, sms, st);
+                         ps.real, state, ps.span.rot, ps.span.pos, i > 0, sms, st);
         } else if (ps.kind == Pass::WALSH) {
             e = run_walsh(dblob, ps.off, ps.off2, ps.m, uint32_t(ps.row_bits), elem_bytes, state, sms, st);
         } else if (ps.kind == Pass::PAIR) {

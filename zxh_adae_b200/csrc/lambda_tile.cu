@@ -22,6 +22,7 @@
 // it); a term's sign outside the registers is one bit per tile (one parity per term) XOR
 // one per thread.
 #include "adjoint.h"
+#include "chain.cuh"
 #include "core.h"
 #include "dev.cuh"
 
@@ -60,15 +61,17 @@ __device__ __forceinline__ double flip_sign(double c, uint32_t s)
     return __hiloint2double(__double2hiint(c) ^ int(s << 31), __double2loint(c));
 }
 
-// MODE 0: energy only; 1: lam is written; 2: lam is added to.
+// MODE 0: energy only; 1: lam is written; 2: lam is added to. With lam the energy comes from
+// the whole of it, in the last pass (last != 0).
 template <typename E, int MODE>
 __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 2 : 1)
-    lambda_tile_kernel(const E *__restrict__ psi, E *lam, const __grid_constant__ LamPassDev p,
-                       const TermDev *__restrict__ terms, double *energy)
+    lambda_tile_kernel(const E *psi, E *lam, const __grid_constant__ LamPassDev p,
+                       const TermDev *__restrict__ terms, double *energy, int last)
 {
     using R = typename ET<E>::R;
     extern __shared__ __align__(128) unsigned char s_raw[];
     LamSmem<E> &sm = *reinterpret_cast<LamSmem<E> *>(s_raw);
+    chain_trigger();
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t nd = p.nd;
 
@@ -110,6 +113,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 2 : 1)
     double en = 0.0;
     uint32_t turn = 0;
     uint64_t rn = tile_base(blockIdx.x);
+    chain_wait();  // everything above reads only the terms
     for (uint64_t t = blockIdx.x; t < p.ntiles; t += gridDim.x, turn ^= 1u) {
         const uint64_t r0 = rn;
         const uint64_t ra = r0 ^ rt;
@@ -120,9 +124,12 @@ __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 2 : 1)
                 if ((j >> b) & 1) r ^= p.basis[4 + b];
             return r;
         };
-        E x[kLamRegs];
+        E x[kLamRegs], l[kLamRegs];
 #pragma unroll
-        for (int j = 0; j < kLamRegs; j++) x[j] = __ldg(psi + addr(j));
+        for (int j = 0; j < kLamRegs; j++) {
+            x[j] = __ldcg(psi + addr(j));
+            if constexpr (MODE == 2) l[j] = __ldcg(lam + addr(j));
+        }
         if (t + gridDim.x < p.ntiles) {
             rn = tile_base(t + gridDim.x);
             const uint64_t r = (rn ^ rp) & ~uint64_t((1 << kLamRun) - 1);
@@ -142,9 +149,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 2 : 1)
         for (int j = 0; j < kLamRegs; j++) sm.slab[it | uint32_t(j << 4)] = x[j];
         __syncthreads();
 
-        // diagonal part: coefficients by register part, then the transform
-        E l[kLamRegs];
-        if (nd) {
+        // diagonal part (the first pass): coefficients by register part, then the transform
+        if (MODE != 2 && nd) {
             R u[kLamRegs];
             uint32_t word = ~0u, signs = 0;
 #pragma unroll
@@ -173,7 +179,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 2 : 1)
                 l[j].x = u[j] * x[j].x;
                 l[j].y = u[j] * x[j].y;
             }
-        } else {
+        } else if (MODE != 2) {
 #pragma unroll
             for (int j = 0; j < kLamRegs; j++) l[j].x = l[j].y = R(0);
         }
@@ -194,20 +200,17 @@ __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 2 : 1)
 #pragma unroll
             for (int j = 0; j < kLamRegs; j++) l[j] = axpy(c, row[j << 4], l[j]);
         }
+        if (MODE == 0 || last) {
 #pragma unroll
-        for (int j = 0; j < kLamRegs; j++) {
-            en += double(x[j].x) * double(l[j].x) + double(x[j].y) * double(l[j].y);  // Re(conj(psi) lambda)
-            if constexpr (MODE != 0) {
-                E *dst = lam + addr(j);
-                if constexpr (MODE == 2) {
-                    const E old = *dst;
-                    l[j].x += old.x;
-                    l[j].y += old.y;
-                }
-                *dst = l[j];
-            }
+            for (int j = 0; j < kLamRegs; j++)  // Re(conj(psi) lambda)
+                en += double(x[j].x) * double(l[j].x) + double(x[j].y) * double(l[j].y);
+        }
+        if constexpr (MODE != 0) {
+#pragma unroll
+            for (int j = 0; j < kLamRegs; j++) __stcg(lam + addr(j), l[j]);
         }
     }
+    if (MODE != 0 && !last) return;
     en = warp_sum_f64(en);
     if (lane == 0) sm.red[warp] = en;
     __syncthreads();
@@ -219,8 +222,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 2 : 1)
 }
 
 template <typename E, int MODE>
-cudaError_t launch_pass(const E *psi, E *lam, const LamPassDev &p, const TermDev *terms, double *energy, int sms,
-                        cudaStream_t st)
+cudaError_t launch_pass(const E *psi, E *lam, const LamPassDev &p, const TermDev *terms, double *energy, bool last,
+                        bool chained, int sms, cudaStream_t st)
 {
     auto kern = lambda_tile_kernel<E, MODE>;
     const int smem = int(sizeof(LamSmem<E>));
@@ -229,8 +232,7 @@ cudaError_t launch_pass(const E *psi, E *lam, const LamPassDev &p, const TermDev
     int per_sm = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, size_t(smem));
     const unsigned grid = unsigned(std::min<uint64_t>(p.ntiles, uint64_t(sms) * uint64_t(std::max(1, per_sm))));
-    kern<<<grid, kThreads, size_t(smem), st>>>(psi, lam, p, terms, energy);
-    return cudaGetLastError();
+    return launch_chained(chained, kern, grid, kThreads, size_t(smem), st, psi, lam, p, terms, energy, last ? 1 : 0);
 }
 
 template <typename E>
@@ -238,9 +240,10 @@ cudaError_t lambda_tiles_typed(const E *psi, E *lam, const std::vector<LamPassDe
                                double *energy, int sms, cudaStream_t st)
 {
     for (size_t i = 0; i < passes.size(); i++) {
-        const cudaError_t e = !lam   ? launch_pass<E, 0>(psi, lam, passes[i], terms, energy, sms, st)
-                              : i ? launch_pass<E, 2>(psi, lam, passes[i], terms, energy, sms, st)
-                                  : launch_pass<E, 1>(psi, lam, passes[i], terms, energy, sms, st);
+        const bool last = i + 1 == passes.size();
+        const cudaError_t e = !lam ? launch_pass<E, 0>(psi, lam, passes[i], terms, energy, last, i > 0, sms, st)
+                              : i  ? launch_pass<E, 2>(psi, lam, passes[i], terms, energy, last, i > 0, sms, st)
+                                   : launch_pass<E, 1>(psi, lam, passes[i], terms, energy, last, i > 0, sms, st);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

@@ -38,7 +38,8 @@ cudaError_t run_counts(const SamplerScratch &sc, int m, const PermCols &cols, un
                        unsigned long long *uoff, unsigned long long *total, uint64_t *words, uint64_t *hits,
                        int pass, int sms, cudaStream_t st, uint64_t &kernels);
 
-// Pass runner (kernels.cu).
+// Pass runner (kernels.cu). chained, here and below: the launch directly follows another
+// kernel of the run (chain.cuh).
 struct Pass;
 // first_src / last_dst (only where the first / last pass is a general strided
 // pass): that pass reads psi from first_src / writes it to last_dst instead of
@@ -62,7 +63,7 @@ cudaError_t run_fast_tile(const uint8_t *dblob, uint64_t foff, uint64_t toff, ui
 // low: the low pass (lane bits swapped into registers); real: every gate of the
 // pass has a real matrix (both need row_low_ok); win: the pass has a window.
 cudaError_t run_row_pass(const uint8_t *dblob, uint64_t poff, uint64_t toff, uint64_t nitems, int elem_bytes,
-                         int wide, bool low, bool real, bool win, void *state, int sms, cudaStream_t st);
+                         int wide, bool low, bool real, bool win, void *state, bool chained, int sms, cudaStream_t st);
 // Span pass (span.cu): up to T real-rotation gates on a 2^T-amplitude tile per
 // read-modify-write (T = 13 complex64, 12 complex128); low: the tile is real bits
 // 0..T-1; layouts: 2 or 3 (span_layouts); land: the landing form; win: 0 no window,
@@ -70,8 +71,8 @@ cudaError_t run_row_pass(const uint8_t *dblob, uint64_t poff, uint64_t toff, uin
 // pass's rotation coefficients and tile coordinates (host copies of SpanDev::rot and
 // SpanDev::pos, passed to the landing form as a kernel parameter).
 cudaError_t run_span(const uint8_t *dblob, uint64_t soff, uint64_t toff, uint64_t ntiles, int elem_bytes, bool low,
-                     int layouts, bool land, int win, void *state, const double (*rot)[2], const uint8_t *pos, int sms,
-                     cudaStream_t st);
+                     int layouts, bool land, int win, void *state, const double (*rot)[2], const uint8_t *pos,
+                     bool chained, int sms, cudaStream_t st);
 // amplitude 0 := 1 (the rest of an INIT pass is a memset)
 cudaError_t run_set_one(void *state, int elem_bytes, cudaStream_t st);
 // General strided pass (grow.cu): lam == nullptr applies the pass to psi; otherwise
@@ -82,7 +83,7 @@ cudaError_t run_set_one(void *state, int elem_bytes, cudaStream_t st);
 // psi_src: read psi from there (written to psi).
 cudaError_t run_grow(const uint8_t *dblob, uint64_t poff, uint64_t toff, int R, uint64_t nitems, int elem_bytes,
                      void *psi, void *lam, double *grads, bool real, bool staged, DevStatus *status, int sms,
-                     cudaStream_t st, const void *psi_src = nullptr);
+                     cudaStream_t st, const void *psi_src = nullptr, bool chained = false);
 int grow_reg_bits(int elem_bytes, bool adjoint);
 int grow_fixed_bits(int elem_bytes);
 int grow_adjoint_gates();

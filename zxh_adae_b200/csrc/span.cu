@@ -50,6 +50,7 @@
 // windows as one factor per thread times one per register pattern, others with
 // in-tile quadratic terms by a Gray-code walk over the registers (32-bit turns for
 // complex64, the full 64-bit turns for complex128).
+#include "chain.cuh"
 #include "core.h"
 #include "dev.cuh"
 #include "host.h"
@@ -751,6 +752,7 @@ __global__ void __launch_bounds__(kSpanThreads, 2)
     E *half = s_land + (1 << G::T);
     __shared__ SpanShared<G, WIN, EXPS> sh;
 
+    chain_trigger();
     const SpanDev &p = *reinterpret_cast<const SpanDev *>(blob + soff);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     span_setup<G, LS>(sh, p, blob, toff, tid);
@@ -784,12 +786,15 @@ __global__ void __launch_bounds__(kSpanThreads, 2)
         }
         cp_async_commit();
     };
-    issue(blockIdx.x);
 
     for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const uint64_t base = span_tile_base<G, LOW>(tile, kc.pos);
         [[maybe_unused]] SpanWin<E> wpre, wpost;
         span_windows_setup<G, LS>(wpre, wpost, p, blob, sh, g, base, lane, warp);
+        if (tile == blockIdx.x) {  // everything above reads only the program
+            chain_wait();
+            issue(tile);
+        }
         cp_async_wait<0>();  // this thread's copies of the tile have landed
         __syncthreads();     // and everyone's
         E x[NR];
@@ -867,7 +872,7 @@ cudaError_t launch_span(const uint8_t *dblob, uint64_t soff, uint64_t toff, uint
 
 template <class G, bool LOW, bool THREE, int WIN>
 cudaError_t launch_span_land(const uint8_t *dblob, uint64_t soff, uint64_t toff, uint64_t ntiles, void *state,
-                             const double (*rot)[2], const uint8_t *pos, int sms, cudaStream_t st)
+                             const double (*rot)[2], const uint8_t *pos, bool chained, int sms, cudaStream_t st)
 {
     using E = typename G::E;
     SpanConst<E> kc;
@@ -880,14 +885,13 @@ cudaError_t launch_span_land(const uint8_t *dblob, uint64_t soff, uint64_t toff,
     const size_t smem = (sizeof(E) << G::T) + (sizeof(E) << (G::T - 1));  // 64 + 32 KiB
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
-    kern<<<span_grid(kern, smem, ntiles, sms), kSpanThreads, smem, st>>>(dblob, soff, toff, static_cast<E *>(state),
-                                                                         kc);
-    return cudaGetLastError();
+    return launch_chained(chained, kern, span_grid(kern, smem, ntiles, sms), kSpanThreads, smem, st, dblob, soff, toff,
+                          static_cast<E *>(state), kc);
 }
 
 template <int FORM, bool LOW, bool THREE>
 cudaError_t launch_span_win(const uint8_t *dblob, uint64_t soff, uint64_t toff, uint64_t ntiles, int win, void *state,
-                            const double (*rot)[2], const uint8_t *pos, int sms, cudaStream_t st)
+                            const double (*rot)[2], const uint8_t *pos, bool chained, int sms, cudaStream_t st)
 {
     // FORM: 0 register form complex64, 1 register form complex128, 2 landing form
     // complex64, 3 landing form complex128
@@ -897,8 +901,8 @@ cudaError_t launch_span_win(const uint8_t *dblob, uint64_t soff, uint64_t toff, 
         else if constexpr (FORM == 1)
             return launch_span<GeoReg128, LOW, THREE, W>(dblob, soff, toff, ntiles, state, sms, st);
         else if constexpr (FORM == 2)
-            return launch_span_land<GeoLand64, LOW, THREE, W>(dblob, soff, toff, ntiles, state, rot, pos, sms, st);
-        else return launch_span_land<GeoLand128, LOW, THREE, W>(dblob, soff, toff, ntiles, state, rot, pos, sms, st);
+            return launch_span_land<GeoLand64, LOW, THREE, W>(dblob, soff, toff, ntiles, state, rot, pos, chained, sms, st);
+        else return launch_span_land<GeoLand128, LOW, THREE, W>(dblob, soff, toff, ntiles, state, rot, pos, chained, sms, st);
     };
     switch (win) {
     case 0: return go(std::integral_constant<int, 0>{});
@@ -936,29 +940,29 @@ int span_layouts(int elem_bytes, uint32_t gates, bool low, bool land)
 }
 
 cudaError_t run_span(const uint8_t *dblob, uint64_t soff, uint64_t toff, uint64_t ntiles, int elem_bytes, bool low,
-                     int layouts, bool land, int win, void *state, const double (*rot)[2], const uint8_t *pos, int sms,
-                     cudaStream_t st)
+                     int layouts, bool land, int win, void *state, const double (*rot)[2], const uint8_t *pos,
+                     bool chained, int sms, cudaStream_t st)
 {
     if (layouts != 2 && layouts != 3) return cudaErrorInvalidValue;
     const bool three = layouts == 3;
     if (elem_bytes == 16) {
         if (land) {
             if (!three) return cudaErrorInvalidValue;
-            return low ? launch_span_win<3, true, true>(dblob, soff, toff, ntiles, win, state, rot, pos, sms, st)
-                       : launch_span_win<3, false, true>(dblob, soff, toff, ntiles, win, state, rot, pos, sms, st);
+            return low ? launch_span_win<3, true, true>(dblob, soff, toff, ntiles, win, state, rot, pos, chained, sms, st)
+                       : launch_span_win<3, false, true>(dblob, soff, toff, ntiles, win, state, rot, pos, chained, sms, st);
         }
-        if (low) return launch_span_win<1, true, true>(dblob, soff, toff, ntiles, win, state, rot, pos, sms, st);
-        return three ? launch_span_win<1, false, true>(dblob, soff, toff, ntiles, win, state, rot, pos, sms, st)
-                     : launch_span_win<1, false, false>(dblob, soff, toff, ntiles, win, state, rot, pos, sms, st);
+        if (low) return launch_span_win<1, true, true>(dblob, soff, toff, ntiles, win, state, rot, pos, chained, sms, st);
+        return three ? launch_span_win<1, false, true>(dblob, soff, toff, ntiles, win, state, rot, pos, chained, sms, st)
+                     : launch_span_win<1, false, false>(dblob, soff, toff, ntiles, win, state, rot, pos, chained, sms, st);
     }
     if (land) {
-        if (low) return launch_span_win<2, true, true>(dblob, soff, toff, ntiles, win, state, rot, pos, sms, st);
-        return three ? launch_span_win<2, false, true>(dblob, soff, toff, ntiles, win, state, rot, pos, sms, st)
-                     : launch_span_win<2, false, false>(dblob, soff, toff, ntiles, win, state, rot, pos, sms, st);
+        if (low) return launch_span_win<2, true, true>(dblob, soff, toff, ntiles, win, state, rot, pos, chained, sms, st);
+        return three ? launch_span_win<2, false, true>(dblob, soff, toff, ntiles, win, state, rot, pos, chained, sms, st)
+                     : launch_span_win<2, false, false>(dblob, soff, toff, ntiles, win, state, rot, pos, chained, sms, st);
     }
-    if (low) return launch_span_win<0, true, true>(dblob, soff, toff, ntiles, win, state, rot, pos, sms, st);
+    if (low) return launch_span_win<0, true, true>(dblob, soff, toff, ntiles, win, state, rot, pos, chained, sms, st);
     if (three) return cudaErrorInvalidValue;
-    return launch_span_win<0, false, false>(dblob, soff, toff, ntiles, win, state, rot, pos, sms, st);
+    return launch_span_win<0, false, false>(dblob, soff, toff, ntiles, win, state, rot, pos, chained, sms, st);
 }
 
 }  // namespace zxh

@@ -15,6 +15,7 @@
 // the warp. Diagonal windows fused into the pass are evaluated per amplitude as a
 // polynomial in 64-bit fixed-point turns (Gray-code walk over the register bits)
 // and one table-plus-Taylor exp.
+#include "chain.cuh"
 #include "core.h"
 #include "dev.cuh"
 #include "host.h"
@@ -694,6 +695,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pass_kernel(const uint8_t *__
     static_assert(!XP || (R == 4 && sizeof(VT) == 16) || (R == 5 && sizeof(VT) == 8),
                   "the low pass swaps lane bits with 16 rows of 16 bytes or 32 rows of 8 bytes");
     extern __shared__ __align__(128) float4 s_xp[];  // XP: NR x 32 row slots per warp
+    chain_trigger();
 
     const RowPassDev &p = *reinterpret_cast<const RowPassDev *>(blob + poff);
     const FastGateDev *gates = reinterpret_cast<const FastGateDev *>(blob + p.off_gates);
@@ -769,6 +771,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pass_kernel(const uint8_t *__
     }
 
     const uint64_t stride = uint64_t(gridDim.x) * WARPS;
+    chain_wait();  // everything above reads only the program
     for (uint64_t item = uint64_t(blockIdx.x) * WARPS + uint64_t(warp); item < nitems; item += stride) {
         // item bits go to every real bit outside [0, F) and the register bits
         uint64_t base = item << F;
@@ -877,7 +880,7 @@ bool row_low_ok(int elem_bytes, int wide) { return elem_bytes == 8 || row_reg_bi
 
 template <typename E, int W, bool XP, bool REAL, bool WIN>
 static cudaError_t launch_row(const uint8_t *dblob, uint64_t poff, uint64_t toff, uint64_t nitems, void *state,
-                              int sms, cudaStream_t st)
+                              bool chained, int sms, cudaStream_t st)
 {
     auto kern = row_pass_kernel<E, W, XP, REAL, WIN>;
     const size_t smem = XP ? size_t(kThreads / 32) * (size_t(1) << RowCfg<E, W>::R) * 32 * sizeof(typename RowCfg<E, W>::VT) : 0;
@@ -890,40 +893,39 @@ static cudaError_t launch_row(const uint8_t *dblob, uint64_t poff, uint64_t toff
     if (per_sm < 1) per_sm = 1;
     const uint64_t ctas = (nitems + kThreads / 32 - 1) / (kThreads / 32);
     const unsigned grid = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(ctas, uint64_t(sms) * uint64_t(per_sm))));
-    kern<<<grid, kThreads, smem, st>>>(dblob, poff, toff, static_cast<E *>(state));
-    return cudaGetLastError();
+    return launch_chained(chained, kern, grid, kThreads, smem, st, dblob, poff, toff, static_cast<E *>(state));
 }
 
 template <typename E, int W, bool XP, bool REAL>
 static cudaError_t launch_row_win(const uint8_t *dblob, uint64_t poff, uint64_t toff, uint64_t nitems, bool win,
-                                  void *state, int sms, cudaStream_t st)
+                                  void *state, bool chained, int sms, cudaStream_t st)
 {
-    return win ? launch_row<E, W, XP, REAL, true>(dblob, poff, toff, nitems, state, sms, st)
-               : launch_row<E, W, XP, REAL, false>(dblob, poff, toff, nitems, state, sms, st);
+    return win ? launch_row<E, W, XP, REAL, true>(dblob, poff, toff, nitems, state, chained, sms, st)
+               : launch_row<E, W, XP, REAL, false>(dblob, poff, toff, nitems, state, chained, sms, st);
 }
 
 // The low-pass shapes also run with real gates.
 template <typename E, int W>
 static cudaError_t launch_row_low(const uint8_t *dblob, uint64_t poff, uint64_t toff, uint64_t nitems, bool low,
-                                  bool real, bool win, void *state, int sms, cudaStream_t st)
+                                  bool real, bool win, void *state, bool chained, int sms, cudaStream_t st)
 {
-    if (low) return real ? launch_row_win<E, W, true, true>(dblob, poff, toff, nitems, win, state, sms, st)
-                         : launch_row_win<E, W, true, false>(dblob, poff, toff, nitems, win, state, sms, st);
-    return real ? launch_row_win<E, W, false, true>(dblob, poff, toff, nitems, win, state, sms, st)
-                : launch_row_win<E, W, false, false>(dblob, poff, toff, nitems, win, state, sms, st);
+    if (low) return real ? launch_row_win<E, W, true, true>(dblob, poff, toff, nitems, win, state, chained, sms, st)
+                         : launch_row_win<E, W, true, false>(dblob, poff, toff, nitems, win, state, chained, sms, st);
+    return real ? launch_row_win<E, W, false, true>(dblob, poff, toff, nitems, win, state, chained, sms, st)
+                : launch_row_win<E, W, false, false>(dblob, poff, toff, nitems, win, state, chained, sms, st);
 }
 
 cudaError_t run_row_pass(const uint8_t *dblob, uint64_t poff, uint64_t toff, uint64_t nitems, int elem_bytes,
-                         int wide, bool low, bool real, bool win, void *state, int sms, cudaStream_t st)
+                         int wide, bool low, bool real, bool win, void *state, bool chained, int sms, cudaStream_t st)
 {
     // the wide complex64 shape always takes the instance with the window code:
     // ptxas spills far less there (the windows are skipped at run time)
     if (elem_bytes == 8)
-        return wide ? launch_row_low<float2, 1>(dblob, poff, toff, nitems, low, real, true, state, sms, st)
-                    : launch_row_low<float2, 0>(dblob, poff, toff, nitems, low, real, win, state, sms, st);
-    if (wide) return launch_row_low<double2, 1>(dblob, poff, toff, nitems, low, real, win, state, sms, st);
+        return wide ? launch_row_low<float2, 1>(dblob, poff, toff, nitems, low, real, true, state, chained, sms, st)
+                    : launch_row_low<float2, 0>(dblob, poff, toff, nitems, low, real, win, state, chained, sms, st);
+    if (wide) return launch_row_low<double2, 1>(dblob, poff, toff, nitems, low, real, win, state, chained, sms, st);
     if (low || real) return cudaErrorInvalidValue;
-    return launch_row_win<double2, 0, false, false>(dblob, poff, toff, nitems, win, state, sms, st);
+    return launch_row_win<double2, 0, false, false>(dblob, poff, toff, nitems, win, state, chained, sms, st);
 }
 
 }  // namespace zxh
