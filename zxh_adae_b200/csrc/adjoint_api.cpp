@@ -288,8 +288,7 @@ int reverse_program(zxh_sim *s, const std::vector<size_t> &ends, AffineMap A, st
     const int R = std::max(1, std::min(s->pp.adj_regs, zxh::grow_reg_bits(s->elem_bytes, true)));
     const int maxg = zxh::grow_adjoint_gates();
     const bool fuse = N >= F && s->pp.adj_windows;  // diagonal gates ride in the general strided passes
-    // affine tile passes; grow_only is the batch kernel's set, which has none
-    const bool tiles = fuse && s->pp.affine && !s->pp.grow_only && N >= zxh::kAffBits;
+    const bool tiles = fuse && s->pp.affine && (!s->pp.grow_only || s->pp.grow_tiles) && N >= zxh::kAffBits;
     auto all_deltas = [&]() {
         std::vector<uint64_t> d(static_cast<size_t>(N), 0);
         for (int q = 0; q < N; q++) A.solve(q, d[size_t(q)]);

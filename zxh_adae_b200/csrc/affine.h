@@ -72,11 +72,14 @@ struct AffBuild {
     std::vector<AffTermDev> terms[2];
     bool real = true;  // every gate has a real matrix
 
-    // The gates that fit in a pass, in order: at most 8 whose deltas are independent modulo
-    // the low run bits, and those inside the run bits.
+    // The coordinates of a pass: up to 8 deltas independent modulo the run bits (high), up to 4
+    // that are not but are independent of all others (low: inside the run bits, or the sum of
+    // such a vector and of high deltas, as the gates of a CX fan-in have).
     struct Room {
-        std::vector<uint64_t> ech;
-        bool add(uint64_t delta);  // false: it does not fit; nothing changes
+        struct High { uint64_t part, delta; };  // part: delta >> kAffRun reduced by those before it
+        std::vector<High> high;                 // echelon form, largest part first
+        std::vector<uint64_t> low;              // echelon form of the low coordinates' run parts
+        int add(uint64_t delta);  // 1: a high coordinate, 0: a low one, -1: no room (nothing changes)
     };
     bool init(int elem_bytes, int m, const std::vector<U3Op> &gates, const std::vector<uint64_t> &deltas,
               bool adjoint_matrix = false, const std::vector<uint32_t> *gen = nullptr,

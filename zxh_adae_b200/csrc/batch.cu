@@ -196,8 +196,8 @@ __global__ void __launch_bounds__(NT, NT == kThreads && sizeof(E) == 16 ? 1 : 51
                                                              double *grads, double *energies, DevStatus *status,
                                                              long long spin_limit)
 {
-    __shared__ BatchShared<E, NT> sm;
-    extern __shared__ __align__(128) unsigned char s_tile[];
+    extern __shared__ __align__(128) unsigned char s_raw[];  // an op's tables: BatchShared or AffSmem
+    BatchShared<E, NT> &sm = *reinterpret_cast<BatchShared<E, NT> *>(s_raw);
     __shared__ uint32_t s_task, s_abort;
     for (;;) {
         __syncthreads();
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(NT, NT == kThreads && sizeof(E) == 16 ? 1 : 51
         if (s_abort) break;
         const bool grow = op.kind == BOP_GROW || op.kind == BOP_GROW_ADJ;
         run_op_slice<E, REAL, NT>(op, blob, arena, grads, energies, task.begin, task.end, grow ? task.begin : 0,
-                                  grow ? uint64_t(NT / 32) : 0, sm, s_tile);
+                                  grow ? uint64_t(NT / 32) : 0, sm, s_raw);
         __threadfence();
         __syncthreads();
         if (threadIdx.x == 0) atomicSub(&remaining[task.op], 1u);
@@ -239,13 +239,11 @@ cudaError_t persistent_typed(const uint8_t *blob, const BatchOp *ops, const Batc
                              DevStatus *status, long long spin_limit, int sms, cudaStream_t st)
 {
     int per_sm = 1;
-    size_t smem = 0;
-    if (NT == kThreads) {
-        smem = sizeof(adev::AffSmem<E, true>);
-        const cudaError_t e = cudaFuncSetAttribute(batch_kernel<E, REAL, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   int(smem));
-        if (e != cudaSuccess) return e;
-    }
+    size_t smem = sizeof(BatchShared<E, NT>);
+    if (NT == kThreads) smem = std::max(smem, std::max(sizeof(adev::AffSmem<E, true>), sizeof(adev::AffSmem<E, false>)));
+    const cudaError_t e = cudaFuncSetAttribute(batch_kernel<E, REAL, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               int(smem));
+    if (e != cudaSuccess) return e;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel<E, REAL, NT>, NT, smem);
     if (per_sm < 1) per_sm = 1;
     batch_kernel<E, REAL, NT><<<unsigned(sms * per_sm), NT, smem, st>>>(blob, ops, tasks, ntasks, next, remaining, arena,

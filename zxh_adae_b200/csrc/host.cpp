@@ -1317,11 +1317,11 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
         std::vector<std::vector<U3Op>> groups;
         for (const U3Op *u : gs) {
             size_t k = 0;
-            while (k < rooms.size() && !rooms[k].add(u->delta)) k++;
+            while (k < rooms.size() && rooms[k].add(u->delta) < 0) k++;
             if (k == rooms.size()) {
                 rooms.emplace_back();
                 groups.emplace_back();
-                if (!rooms[k].add(u->delta)) return false;
+                if (rooms[k].add(u->delta) < 0) return false;
             }
             groups[k].push_back(*u);
         }
@@ -1657,7 +1657,7 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
         if ((pp.grow || pp.grow_only) && grow_ok(op)) {
             const int mm = op.m;
             const size_t first = out.passes.size();
-            const bool tiles = pp.affine && !pp.grow_only && op.deltas && mm >= kAffBits;
+            const bool tiles = pp.affine && (!pp.grow_only || pp.grow_tiles) && op.deltas && mm >= kAffBits;
             bool done = tiles && emit_affine(op);
             if (!done) {
                 out.passes.resize(first);
