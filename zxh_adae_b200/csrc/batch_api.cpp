@@ -267,18 +267,29 @@ void make_tasks(zxh_batch *b)
     size_t levels = 0;
     for (const auto &ch : b->chain) levels = std::max(levels, ch.size());
     b->rem_init.assign(b->ops.size(), 0);
-    for (size_t L = 0; L < levels; L++)
+    // Units of a task: the knob's, but no more than spread a level's work of that kind over two
+    // tasks an SM (a level runs as long as its longest task: 16 circuits of 12 to 17 qubits
+    // took 3.1 ms in tasks of 8 tiles, 1.4 ms in tasks of 1 or 2), and at least what the
+    // warps of a CTA share. A tile is four strided items' amplitudes; a quarter of their task
+    // measured best where the level is large.
+    enum { ITEMS, TILES, ELEMS, KINDS };
+    auto kind_of = [](const BatchOp &op) {
+        if (op.kind == zxh::BOP_GROW || op.kind == zxh::BOP_GROW_ADJ) return ITEMS;
+        return op.kind == zxh::BOP_AFFINE || op.kind == zxh::BOP_AFFINE_ADJ ? TILES : ELEMS;
+    };
+    const uint64_t knob[KINDS] = {uint64_t(b->task_items), uint64_t(std::max(1, b->task_items / 16)),
+                                  uint64_t(b->task_elems)};
+    const uint64_t least[KINDS] = {8, 1, 2048};
+    for (size_t L = 0; L < levels; L++) {
+        uint64_t units[KINDS] = {0, 0, 0};
+        for (const auto &ch : b->chain)
+            if (L < ch.size()) units[kind_of(b->ops[ch[L]])] += b->ops[ch[L]].units;
         for (size_t c = 0; c < b->chain.size(); c++) {
             if (L >= b->chain[c].size()) continue;
             const uint32_t oi = b->chain[c][L];
             const BatchOp &op = b->ops[oi];
-            const bool grow = op.kind == zxh::BOP_GROW || op.kind == zxh::BOP_GROW_ADJ;
-            const bool tiles = op.kind == zxh::BOP_AFFINE || op.kind == zxh::BOP_AFFINE_ADJ;
-            // a tile is four strided items' amplitudes (complex64, 16 rows); a quarter of their
-            // task keeps a circuit's tiles on more CTAs
-            const uint64_t per = grow    ? uint64_t(b->task_items)
-                                 : tiles ? uint64_t(std::max(1, b->task_items / 16))
-                                         : uint64_t(b->task_elems);
+            const int k = kind_of(op);
+            const uint64_t per = std::min(knob[k], std::max(least[k], units[k] / (2 * uint64_t(b->sms))));
             for (uint64_t s = 0; s < op.units; s += per) {
                 BatchTask t;
                 t.op = oi;
@@ -289,6 +300,7 @@ void make_tasks(zxh_batch *b)
                 b->rem_init[oi]++;
             }
         }
+    }
 }
 
 int upload(zxh_batch *b)
