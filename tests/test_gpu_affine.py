@@ -142,3 +142,72 @@ def test_affine_gradients_against_dense_adjoint(n, links, window, dtype):
     want = ob.oracle_state(n, circ.records(p))
     assert np.max(np.abs(ob.qubit_order(s.get_state(), n) - want)) <= TOL[dtype]  # the forward output stays
     s.close()
+
+
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+def test_affine_rotations_at_the_ends_of_their_forms(dtype):
+    # cosine or sine zero, equal, and sign changes: the coefficient factored out of a rotation
+    n = 12
+    edge = [math.pi, 3 * math.pi, math.pi / 2, -math.pi / 2, 2 * math.pi, 3.0, 1e-3, 0.3]
+    recs = [(H, 0, q) for q in range(n)]
+    for r in range(3):
+        recs += [(CX, i, (i + 1 + r) % n) for i in range(n)]
+        recs += [(U3, 0, q, edge[(q + r) % len(edge)], 0.0, 0.0) for q in range(n)]
+        recs += [(RZ, 0, q, 0.1 * q + r) for q in range(n)]
+    g = as_records(recs)
+    terms = ad.tfim_terms(n)
+    e_ref, g_ref = ob.dense_adjoint(n, g, terms)
+    s = ZXH(n, dtype=dtype)
+    s.push_gates(g)
+    e, grad = s.adjoint_gradient(terms)
+    tol = 2 * n * (1e-12 if dtype == "complex128" else 1e-6)
+    assert abs(e - e_ref) <= tol and np.max(np.abs(grad - g_ref)) <= tol
+    want = ob.oracle_state(n, g)
+    assert np.max(np.abs(ob.qubit_order(s.get_state(), n) - want)) <= TOL[dtype]
+    s.close()
+
+
+@pytest.mark.parametrize("mode", ["persistent", "graph", "sequential"])
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+def test_batched_tiles_against_dense_adjoint(mode, dtype):
+    # circuits below, at and above the tile size, real and complex gates, with CX
+    from zxh_adae_b200.batch import Batch
+
+    circs = []
+    for n, links, window in [(11, "chain", "linear"), (12, "random", "dense"), (14, "chain", "linear"), (9, "random", "dense")]:
+        c = ansatz(n, links, window, seed=n)
+        p = np.random.default_rng(n).uniform(-math.pi, math.pi, c.nparams)
+        circs.append((n, c.records(p), ad.tfim_terms(n, h=0.8)))
+    for n in (12, 13):  # a real queue's circuits (rotations), in the same batch
+        circs.append(workloads.batch_tfim(1, n, n, n, 3)[0][:3])
+    ref = [ob.dense_adjoint(n, r, t) for n, r, t in circs]
+    for which in (circs, circs[-2:]):
+        want = ref if which is circs else ref[-2:]
+        b = Batch(which, dtype=dtype)
+        for threads in (256, 128, 256):
+            b.set("threads", threads)
+            b.set("task_items", 32 if threads == 128 else 512)
+            e, g = b.run(mode)
+            for k, (n, _r, _t) in enumerate(which):
+                tol = 2 * n * (1e-12 if dtype == "complex128" else 1e-6)
+                assert abs(e[k] - want[k][0]) <= tol, (threads, n)
+                assert np.max(np.abs(b.gradients(g)[k] - want[k][1])) <= tol, (threads, n)
+        b.close()
+
+
+@pytest.mark.parametrize("n", [3, 7, 12, 14])
+def test_first_layer_on_expanded_qubits(n):
+    # every qubit expanded and |0>: the first gate of each is part of the product state
+    g = np.concatenate([as_records([(X, 0, 1), (CX, 0, n - 1)]), workloads.u3_layer(n, n),
+                        as_records([(P, 0, q, 0.3 + q) for q in range(n)]), workloads.u3_layer(n, n + 1),
+                        workloads.cx_chain(n), workloads.u3_layer(n, n + 2)])
+    for part in (g, g[: n + 2], g[2:]):
+        o = Oracle(n)
+        o.push(part)
+        o.execute()
+        for dtype in ("complex64", "complex128"):
+            s = ZXH(n, eager_expand_all=True, dtype=dtype)
+            s.push_gates(part)
+            s.execute()
+            assert np.max(np.abs(s.get_state(0).astype(np.complex128) - o.get_state(0))) <= TOL[dtype]
+            s.close()

@@ -288,7 +288,8 @@ int reverse_program(zxh_sim *s, const std::vector<size_t> &ends, AffineMap A, st
     const int R = std::max(1, std::min(s->pp.adj_regs, zxh::grow_reg_bits(s->elem_bytes, true)));
     const int maxg = zxh::grow_adjoint_gates();
     const bool fuse = N >= F && s->pp.adj_windows;  // diagonal gates ride in the general strided passes
-    const bool tiles = fuse && s->pp.affine && (!s->pp.grow_only || s->pp.grow_tiles) && N >= zxh::kAffBits;
+    const bool tiles = fuse && s->pp.affine && (!s->pp.grow_only || s->pp.grow_tiles) && N >= zxh::kAffBits &&
+                       N <= zxh::kAffMaxBits;
     auto all_deltas = [&]() {
         std::vector<uint64_t> d(static_cast<size_t>(N), 0);
         for (int q = 0; q < N; q++) A.solve(q, d[size_t(q)]);
@@ -643,7 +644,7 @@ int zxh_adjoint_gradient(zxh_sim *s, const zxh_term *terms, size_t nterms, size_
             kernels++;
             break;
         case RevStep::AFFINE:
-            CK(s, zxh::run_affine(s->d_adj + L.grow, r.off, r.toff, r.aff->dev.ntiles, s->elem_bytes, r.aff->real,
+            CK(s, zxh::run_affine(s->d_adj + L.grow, r.off, r.toff, r.aff->dev.ntiles, s->elem_bytes, r.aff->form,
                                   s->d_psi, psi_from, s->d_lam, d_grads, chained, s->sms, s->stream),
                "adjoint tile launch");
             psi_from = nullptr;

@@ -20,7 +20,8 @@
 // is a polynomial of degree two in eight bits whose coefficients depend only on the tile
 // and the position in the run: the CTA evaluates the terms 16 times per tile (once per run
 // position) instead of once per thread, and a thread reads the polynomial from shared
-// memory. Gradients of window terms come from the marginals of w = Im(conj(lambda) psi) over
+// memory. Real addresses are 32-bit (states of at most 2^32 amplitudes; larger ones take the
+// general strided passes). Gradients of window terms come from the marginals of w = Im(conj(lambda) psi) over
 // the same bits, reduced once per tile. The slot of tile index i is i ^ (bits 4..7 of i): in
 // every layout the lanes that share a bank cycle cover one 128-byte row.
 #include "affine_dev.cuh"
@@ -34,22 +35,22 @@ namespace {
 
 using namespace adev;
 
-template <typename E, bool ADJ, bool REAL>
+template <typename E, bool ADJ, int FORM>
 __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? (ADJ ? 2 : 3) : (ADJ ? 1 : 2))
     affine_kernel(const uint8_t *__restrict__ blob, uint64_t poff, uint64_t toff, E *psi, const E *src, E *lam,
                   double *grads, uint64_t ntiles)
 {
     extern __shared__ __align__(128) unsigned char s_raw[];
     chain_trigger();
-    affine_body<E, ADJ, REAL>(*reinterpret_cast<AffSmem<E, ADJ> *>(s_raw), blob, poff, toff, psi, src, lam, grads,
-                              blockIdx.x, gridDim.x, ntiles);
+    affine_body<E, ADJ, FORM>(*reinterpret_cast<AffSmem<E, ADJ> *>(s_raw), blob, poff, toff, psi, src, lam, grads,
+                              blockIdx.x, gridDim.x, uint32_t(ntiles));
 }
 
-template <typename E, bool ADJ, bool REAL>
+template <typename E, bool ADJ, int FORM>
 cudaError_t launch_affine(const uint8_t *blob, uint64_t poff, uint64_t toff, uint64_t ntiles, E *psi, const E *src, E *lam,
                           double *grads, bool chained, int sms, cudaStream_t st)
 {
-    auto kern = affine_kernel<E, ADJ, REAL>;
+    auto kern = affine_kernel<E, ADJ, FORM>;
     const int smem = int(sizeof(AffSmem<E, ADJ>));
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
@@ -60,26 +61,33 @@ cudaError_t launch_affine(const uint8_t *blob, uint64_t poff, uint64_t toff, uin
                           src ? src : static_cast<const E *>(psi), lam, grads, ntiles);
 }
 
+template <typename E, bool ADJ, typename... A>
+cudaError_t affine_form(int form, A... args)
+{
+    switch (form) {
+    case 0: return launch_affine<E, ADJ, 0>(args...);
+    case 1: return launch_affine<E, ADJ, 1>(args...);
+    default: return launch_affine<E, ADJ, 2>(args...);
+    }
+}
+
 template <typename E>
-cudaError_t affine_typed(bool real, const uint8_t *blob, uint64_t poff, uint64_t toff, uint64_t ntiles, E *psi, const E *src,
+cudaError_t affine_typed(int form, const uint8_t *blob, uint64_t poff, uint64_t toff, uint64_t ntiles, E *psi, const E *src,
                          E *lam, double *grads, bool chained, int sms, cudaStream_t st)
 {
-    if (lam)
-        return real ? launch_affine<E, true, true>(blob, poff, toff, ntiles, psi, src, lam, grads, chained, sms, st)
-                    : launch_affine<E, true, false>(blob, poff, toff, ntiles, psi, src, lam, grads, chained, sms, st);
-    return real ? launch_affine<E, false, true>(blob, poff, toff, ntiles, psi, src, lam, grads, chained, sms, st)
-                : launch_affine<E, false, false>(blob, poff, toff, ntiles, psi, src, lam, grads, chained, sms, st);
+    return lam ? affine_form<E, true>(form, blob, poff, toff, ntiles, psi, src, lam, grads, chained, sms, st)
+               : affine_form<E, false>(form, blob, poff, toff, ntiles, psi, src, lam, grads, chained, sms, st);
 }
 
 }  // namespace
 
-cudaError_t run_affine(const uint8_t *dblob, uint64_t poff, uint64_t toff, uint64_t ntiles, int elem_bytes, bool real,
+cudaError_t run_affine(const uint8_t *dblob, uint64_t poff, uint64_t toff, uint64_t ntiles, int elem_bytes, int form,
                        void *psi, const void *psi_src, void *lam, double *grads, bool chained, int sms, cudaStream_t st)
 {
     if (elem_bytes == 8)
-        return affine_typed(real, dblob, poff, toff, ntiles, static_cast<float2 *>(psi),
+        return affine_typed(form, dblob, poff, toff, ntiles, static_cast<float2 *>(psi),
                             static_cast<const float2 *>(psi_src), static_cast<float2 *>(lam), grads, chained, sms, st);
-    return affine_typed(real, dblob, poff, toff, ntiles, static_cast<double2 *>(psi),
+    return affine_typed(form, dblob, poff, toff, ntiles, static_cast<double2 *>(psi),
                         static_cast<const double2 *>(psi_src), static_cast<double2 *>(lam), grads, chained, sms, st);
 }
 

@@ -11,6 +11,7 @@
 namespace zxh {
 
 constexpr int kAffBits = 12;      // tile coordinates
+constexpr int kAffMaxBits = 32;   // largest state
 constexpr int kAffRun = 4;        // coordinates 0..3 span the low 4 real bits
 constexpr int kAffHigh = kAffBits - kAffRun;
 constexpr int kAffPairs = kAffHigh * (kAffHigh - 1) / 2;
@@ -23,8 +24,12 @@ __host__ __device__ constexpr int aff_pair(int i, int j) { return i * (2 * kAffH
 
 // The gate on a coordinate: u00, u01, u10, u11 (re, im; U^dagger in adjoint passes), its
 // qubit's selector, the gradient's generator (0 none, 1 Y, 2 X) and slot.
+// Rotation passes: one coefficient of [[c, -s], [s, c]] factored out, rot = s / c and factor c
+// where |c| >= |s|, else (bit of AffDev::mu) rot = c / s and factor s; gscale is the square of
+// the factors of the gates applied before it.
 struct AffGateDev {
     double u[8];
+    double rot, gscale;
     uint32_t sel, gen, slot, pad;
 };
 
@@ -55,7 +60,11 @@ struct AffWinDev {
 };
 
 struct AffDev {
-    uint32_t m, gates, nsel, pad;  // gates: bit k = coordinate k has one
+    uint32_t m, gates, nsel;       // gates: bit k = coordinate k has one
+    uint32_t mu;                   // rotation passes: the gates with rot = c / s
+    double scale;                  // rotation passes: the product of the factors,
+    uint64_t mu_high, mu_low;      // negated by the parity of these selector bits (high coordinates'
+                                   // gates: of the run position; low ones': of the tile)
     uint64_t ntiles;
     uint64_t basis[kAffBits], tr[64];      // tile coordinates; real vectors of the tile bits
     uint64_t alpha[kAffMaxSel], lw[1 << kAffRun];  // selector masks; bit s of lw[l]: f_s of run position l
@@ -70,7 +79,8 @@ struct AffBuild {
     AffDev dev;
     std::vector<AffEntryDev> entries[2];
     std::vector<AffTermDev> terms[2];
-    bool real = true;  // every gate has a real matrix
+    // 0: complex matrices; 1: every gate's is real; 2: every gate is a real rotation (affine_body)
+    int form = 2;
 
     // The coordinates of a pass: up to 8 deltas independent modulo the run bits (high), up to 4
     // that are not but are independent of all others (low: inside the run bits, or the sum of
@@ -98,7 +108,7 @@ struct AffBuild {
 // The pass at poff of the blob over psi (read from psi_src where given); lam != nullptr:
 // the adjoint form, gradients added to grads[slot]. toff: the phase table (unused without
 // windows). chained: directly after another kernel of the run (chain.cuh).
-cudaError_t run_affine(const uint8_t *dblob, uint64_t poff, uint64_t toff, uint64_t ntiles, int elem_bytes, bool real,
+cudaError_t run_affine(const uint8_t *dblob, uint64_t poff, uint64_t toff, uint64_t ntiles, int elem_bytes, int form,
                        void *psi, const void *psi_src, void *lam, double *grads, bool chained, int sms, cudaStream_t st);
 
 }  // namespace zxh

@@ -25,8 +25,11 @@ struct AffSmem {
     E slab[ADJ ? 2 : 1][1 << kAffBits];      // adjoint passes: also the sums and marginals of w
     E exp[1 << kExpTableBits];
     RT u[kAffBits][2][8];  // [1]: the |1> member first
+    RT rot[kAffBits];
+    double gscale[kAffBits];
     uint32_t sel[kAffBits], gen[kAffBits];
-    uint64_t alpha[kAffMaxSel], lw[kRun], basis[kAffBits];
+    uint64_t lw[kRun];
+    uint32_t alpha[kAffMaxSel], basis[kAffBits];
     AffWinDev win[NW];
     AffEntryDev ent[NW][kAffMaxEntries];
     int64_t K[NW][kRun], w[NW][kRun][kAffHigh], q[NW][kRun][kAffPairs];
@@ -78,12 +81,19 @@ __device__ __forceinline__ E cmad2(RT ar, RT ai, E a, RT br, RT bi, E b)  // a-c
     return o;
 }
 
+// a * b + c by components (the real parts of conj(a) b summed over both).
+__device__ __forceinline__ float2 dot2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ double2 dot2(double2 a, double2 b, double2 c)
+{
+    return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
+}
+
 // The gate on register bit RR, m its matrix in the thread's orientation; adjoint passes
 // first add the gradient's share (FP32 over 8 pairs for complex64) to acc.
 template <int RR, bool ADJ, bool REAL, typename E, typename RT>
 __device__ __forceinline__ void gate(E (&x)[kNR], E (&y)[kNR], const RT *m, bool flip, uint32_t gen, double *acc)
 {
-    RT part = 0;
+    [[maybe_unused]] E p0 = {0, 0}, p1 = {0, 0};
     const RT m0 = m[0], m2 = m[2], m4 = m[4], m6 = m[6];
     const RT m1 = REAL ? RT(0) : m[1], m3 = REAL ? RT(0) : m[3], m5 = REAL ? RT(0) : m[5], m7 = REAL ? RT(0) : m[7];
 #pragma unroll
@@ -94,9 +104,11 @@ __device__ __forceinline__ void gate(E (&x)[kNR], E (&y)[kNR], const RT *m, bool
         if constexpr (ADJ) {
             const E llo = y[j], lhi = y[j | B];
             if (gen == 1) {  // Im<l|Y|p> = Re(conj(l1) p0) - Re(conj(l0) p1)
-                part += (lhi.x * lo.x + lhi.y * lo.y) - (llo.x * hi.x + llo.y * hi.y);
+                p0 = dot2(lhi, lo, p0);
+                p1 = dot2(llo, hi, p1);
             } else if (gen == 2) {  // Im<l|X|p> = Im(conj(l0) p1 + conj(l1) p0)
-                part += (llo.x * hi.y - llo.y * hi.x) + (lhi.x * lo.y - lhi.y * lo.x);
+                p0.x += llo.x * hi.y - llo.y * hi.x;
+                p0.y += lhi.x * lo.y - lhi.y * lo.x;
             }
             if constexpr (REAL) {
                 y[j] = rmad2(m0, llo, m2, lhi);
@@ -115,20 +127,93 @@ __device__ __forceinline__ void gate(E (&x)[kNR], E (&y)[kNR], const RT *m, bool
         }
     }
     if constexpr (ADJ) {
-        if (gen) *acc += double(gen == 1 && flip ? -part : part);
+        if (gen == 1) {
+            const double part = (double(p0.x) - double(p1.x)) + (double(p0.y) - double(p1.y));
+            *acc += flip ? -part : part;
+        } else if (gen == 2) {
+            *acc += double(p0.x) + double(p0.y);
+        }
+    }
+}
+
+__device__ __forceinline__ float2 neg(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ double2 neg(double2 a) { return make_double2(-a.x, -a.y); }
+__device__ __forceinline__ float2 axpy(float c, float2 a, float2 b) { return __ffma2_rn(make_float2(c, c), a, b); }
+__device__ __forceinline__ double2 axpy(double c, double2 a, double2 b)
+{
+    return make_double2(fma(c, a.x, b.x), fma(c, a.y, b.y));
+}
+__device__ __forceinline__ float2 scaled(float c, float2 a) { return __fmul2_rn(make_float2(c, c), a); }
+__device__ __forceinline__ double2 scaled(double c, double2 a) { return make_double2(c * a.x, c * a.y); }
+
+// A rotation with one coefficient factored out: half the multiply-adds of gate(). r: its
+// coefficient, negated where the thread's pairs start at the |1> member (flip); with
+// rot = c / s that also negates the factor (AffDev::mu_high, mu_low).
+template <int RR, bool ADJ, typename E, typename RT>
+__device__ __forceinline__ void rotation(E (&x)[kNR], E (&y)[kNR], RT r, bool mu, bool flip, uint32_t gen, double gscale,
+                                         double *acc)
+{
+    constexpr int B = 1 << RR;
+    if constexpr (ADJ) {
+        if (gen) {
+            E p0 = {0, 0}, p1 = {0, 0};
+#pragma unroll
+            for (int j = 0; j < kNR; j++) {
+                if ((j >> RR) & 1) continue;
+                p0 = dot2(y[j | B], x[j], p0);
+                p1 = dot2(y[j], x[j | B], p1);
+            }
+            const double part = (double(p0.x) - double(p1.x)) + (double(p0.y) - double(p1.y));
+            *acc += gscale * (flip ? -part : part);
+        }
+    }
+    if (mu) {  // one branch around each form: inside the loop the compiler computes both
+#pragma unroll
+        for (int j = 0; j < kNR; j++) {
+            if ((j >> RR) & 1) continue;
+            const E lo = x[j], hi = x[j | B];
+            x[j] = axpy(r, lo, neg(hi));
+            x[j | B] = axpy(r, hi, lo);
+            if constexpr (ADJ) {
+                const E llo = y[j], lhi = y[j | B];
+                y[j] = axpy(r, llo, neg(lhi));
+                y[j | B] = axpy(r, lhi, llo);
+            }
+        }
+    } else {
+        const RT nr = -r;
+#pragma unroll
+        for (int j = 0; j < kNR; j++) {
+            if ((j >> RR) & 1) continue;
+            const E lo = x[j], hi = x[j | B];
+            x[j] = axpy(nr, hi, lo);
+            x[j | B] = axpy(r, lo, hi);
+            if constexpr (ADJ) {
+                const E llo = y[j], lhi = y[j | B];
+                y[j] = axpy(nr, lhi, llo);
+                y[j | B] = axpy(r, llo, lhi);
+            }
+        }
     }
 }
 
 // The gates on coordinates K0 .. K0 + 3, the layout's registers; c: the selector bits of
 // the thread (of the tile, in layout C).
-template <int K0, bool ADJ, bool REAL, typename E, typename SM>
-__device__ __forceinline__ void gates(E (&x)[kNR], E (&y)[kNR], uint32_t mask, uint64_t c, SM &sm, uint32_t tid)
+template <int K0, bool ADJ, int FORM, typename E, typename SM>
+__device__ __forceinline__ void gates(E (&x)[kNR], E (&y)[kNR], uint32_t mask, uint32_t mu, uint64_t c, SM &sm,
+                                      uint32_t tid)
 {
     auto one = [&](auto rr) {
         constexpr int RR = decltype(rr)::value, k = K0 + RR;
         if (!((mask >> k) & 1u)) return;
         const bool flip = (c >> sm.sel[k]) & 1;
-        gate<RR, ADJ, REAL>(x, y, sm.u[k][flip], flip, sm.gen[k], ADJ ? &sm.gacc[ADJ ? k : 0][ADJ ? tid : 0] : nullptr);
+        double *acc = ADJ ? &sm.gacc[ADJ ? k : 0][ADJ ? tid : 0] : nullptr;
+        if constexpr (FORM == 2) {
+            const auto r = sm.rot[k];
+            rotation<RR, ADJ>(x, y, flip ? -r : r, (mu >> k) & 1u, flip, sm.gen[k], sm.gscale[k], acc);
+        } else {
+            gate<RR, ADJ, FORM == 1>(x, y, sm.u[k][flip], flip, sm.gen[k], acc);
+        }
     };
     one(std::integral_constant<int, 0>());
     one(std::integral_constant<int, 1>());
@@ -331,16 +416,18 @@ __device__ __forceinline__ void window_grad(const E (&x)[kNR], const E (&y)[kNR]
 // a launch
 // that may have started before the work it follows has ended waits for it here (chain.cuh):
 // nothing but the program is read before that.
-template <typename E, bool ADJ, bool REAL>
+template <typename E, bool ADJ, int FORM>
 __device__ __forceinline__ void affine_body(AffSmem<E, ADJ> &sm, const uint8_t *__restrict__ blob, uint64_t poff,
-                                            uint64_t toff, E *psi, const E *src, E *lam, double *grads, uint64_t first,
-                                            uint64_t step, uint64_t end)
+                                            uint64_t toff, E *psi, const E *src, E *lam, double *grads, uint32_t first,
+                                            uint32_t step, uint32_t end)
 {
     using SM = AffSmem<E, ADJ>;
     using RT = typename ET<E>::R;
     const AffDev &p = *reinterpret_cast<const AffDev *>(blob + poff);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t mask = p.gates, nsel = p.nsel;
+    const uint32_t mask = p.gates, mu = p.mu, nsel = p.nsel;
+    const uint64_t mu_high = p.mu_high, mu_low = p.mu_low;
+    const RT scale = RT(p.scale);
     const AffWinDev &w0 = sm.win[0], &w1 = sm.win[SM::NW - 1];
     const bool win0 = p.win[0].nterms != 0, win1 = !ADJ && p.win[1].nterms != 0;
 
@@ -364,11 +451,13 @@ __device__ __forceinline__ void affine_body(AffSmem<E, ADJ> &sm, const uint8_t *
             sm.u[tid][0][i] = RT(g.u[i]);
             sm.u[tid][1][i] = RT(g.u[i ^ 6]);  // [[u11, u10], [u01, u00]]
         }
+        sm.rot[tid] = RT(g.rot);
+        sm.gscale[tid] = g.gscale;
         sm.sel[tid] = g.sel;
         sm.gen[tid] = g.gen;
-        sm.basis[tid] = p.basis[tid];
+        sm.basis[tid] = uint32_t(p.basis[tid]);
     }
-    if (tid >= 32 && tid < 32 + kAffMaxSel) sm.alpha[tid - 32] = p.alpha[tid - 32];
+    if (tid >= 32 && tid < 32 + kAffMaxSel) sm.alpha[tid - 32] = uint32_t(p.alpha[tid - 32]);
     if (tid >= 96 && tid < 96 + kRun) sm.lw[tid - 96] = p.lw[tid - 96];
     if constexpr (ADJ) {
         const AffTermDev *t = reinterpret_cast<const AffTermDev *>(blob + w0.off_terms);
@@ -388,7 +477,7 @@ __device__ __forceinline__ void affine_body(AffSmem<E, ADJ> &sm, const uint8_t *
     __syncthreads();
 
     // the thread's part of the address in layouts A and B
-    uint64_t ra = 0, rb = 0;
+    uint32_t ra = 0, rb = 0;
 #pragma unroll
     for (int b = 0; b < 5; b++)
         if ((lane >> b) & 1u) {
@@ -401,26 +490,22 @@ __device__ __forceinline__ void affine_body(AffSmem<E, ADJ> &sm, const uint8_t *
             ra ^= sm.basis[9 + b];
             rb ^= sm.basis[5 + b];
         }
-    const uint64_t tr0 = p.tr[lane], tr1 = p.tr[lane + 32u];
+    const uint32_t trl = uint32_t(p.tr[lane]);  // at most 20 tile bits
     const bool need_c = (mask & 0x00fu) != 0, need_b = need_c || (mask & 0xf00u) != 0 || win1;
     const uint64_t lw = sm.lw[lane & 15u], lw0 = sm.lw[0], lwe = sm.lw[tid >> 4];
 
-    auto tile_base = [&](uint64_t t) {
-        const uint64_t rl = (((t >> lane) & 1u) ? tr0 : 0) ^ (((t >> (lane + 32u)) & 1u) ? tr1 : 0);
-        return (uint64_t(__reduce_xor_sync(0xffffffffu, uint32_t(rl >> 32))) << 32) |
-               __reduce_xor_sync(0xffffffffu, uint32_t(rl));
-    };
+    auto tile_base = [&](uint32_t t) { return __reduce_xor_sync(0xffffffffu, ((t >> lane) & 1u) ? trl : 0u); };
     // the run of 16 amplitudes this thread asks L2 for, one tile ahead
-    uint64_t rp = 0;
+    uint32_t rp = 0;
 #pragma unroll
     for (int b = 0; b < kAffHigh; b++)
         if ((tid >> b) & 1u) rp ^= sm.basis[kAffRun + b];
 
-    uint64_t rn = tile_base(first);
+    uint32_t rn = tile_base(first);
     chain_wait();  // everything above reads only the program
-    for (uint64_t t = first; t < end; t += step) {
-        const uint64_t r0 = rn;
-        auto addr = [&](uint64_t base, int k0, int j) {
+    for (uint32_t t = first; t < end; t += step) {
+        const uint32_t r0 = rn;
+        auto addr = [&](uint32_t base, int k0, int j) {
 #pragma unroll
             for (int b = 0; b < 4; b++)
                 if ((j >> b) & 1) base ^= sm.basis[k0 + b];
@@ -429,13 +514,13 @@ __device__ __forceinline__ void affine_body(AffSmem<E, ADJ> &sm, const uint8_t *
         E x[kNR], y[kNR];
 #pragma unroll
         for (int j = 0; j < kNR; j++) {
-            const uint64_t r = addr(r0 ^ ra, 4, j);
+            const uint32_t r = addr(r0 ^ ra, 4, j);
             x[j] = __ldcg(src + r);
             if constexpr (ADJ) y[j] = __ldcg(lam + r);
         }
         if (t + step < end) {
             rn = tile_base(t + step);
-            const uint64_t r = (rn ^ rp) & ~uint64_t(kRun - 1);
+            const uint32_t r = (rn ^ rp) & ~uint32_t(kRun - 1);
 #pragma unroll
             for (int i = 0; i < int(sizeof(E)) / 8; i++) {
                 prefetch_l2(src + r + i * (kRun / 2));
@@ -443,8 +528,8 @@ __device__ __forceinline__ void affine_body(AffSmem<E, ADJ> &sm, const uint8_t *
             }
         }
         // selector bits of the tile: lane s takes selectors s and s + 32
-        const bool b0 = lane < nsel && par64(sm.alpha[lane] & r0);
-        const bool b1 = lane + 32u < nsel && par64(sm.alpha[lane + 32u] & r0);
+        const bool b0 = lane < nsel && (__popc(sm.alpha[lane] & r0) & 1);
+        const bool b1 = lane + 32u < nsel && (__popc(sm.alpha[lane + 32u] & r0) & 1);
         const uint64_t P = uint64_t(__ballot_sync(0xffffffffu, b0)) | (uint64_t(__ballot_sync(0xffffffffu, b1)) << 32);
         const uint64_t c = P ^ lw;
         if (win0 || win1) {
@@ -459,23 +544,31 @@ __device__ __forceinline__ void affine_body(AffSmem<E, ADJ> &sm, const uint8_t *
             if constexpr (ADJ) window_grad(x, y, sm, w0, P, tid);
             window_apply<0, ADJ>(x, y, sm, w0.pairs, 0, lane, warp);
         }
-        gates<4, ADJ, REAL>(x, y, mask, c, sm, tid);
+        gates<4, ADJ, FORM>(x, y, mask, mu, c, sm, tid);
         if (need_c) {
             exchange<0, 2, ADJ ? 2 : 1>(x, y, sm.slab, lane, warp);
-            gates<0, ADJ, REAL>(x, y, mask, P ^ lw0, sm, tid);
+            gates<0, ADJ, FORM>(x, y, mask, mu, P ^ lw0, sm, tid);
             exchange<2, 1, ADJ ? 2 : 1>(x, y, sm.slab, lane, warp);
         } else if (need_b) {
             exchange<0, 1, ADJ ? 2 : 1>(x, y, sm.slab, lane, warp);
         }
-        if (need_b) gates<8, ADJ, REAL>(x, y, mask, c, sm, tid);
+        if (need_b) gates<8, ADJ, FORM>(x, y, mask, mu, c, sm, tid);
         if constexpr (!ADJ) {
             if (win1) window_apply<1, false>(x, y, sm, w1.pairs, 1, lane, warp);
         }
-        const uint64_t rs = r0 ^ (need_b ? rb : ra);
+        if (FORM == 2 && mask) {
+            const RT f = (par64(c & mu_high) ^ par64((P ^ lw0) & mu_low)) ? -scale : scale;
+#pragma unroll
+            for (int j = 0; j < kNR; j++) {
+                x[j] = scaled(f, x[j]);
+                if constexpr (ADJ) y[j] = scaled(f, y[j]);
+            }
+        }
+        const uint32_t rs = r0 ^ (need_b ? rb : ra);
         const int ks = need_b ? 8 : 4;
 #pragma unroll
         for (int j = 0; j < kNR; j++) {
-            const uint64_t r = addr(rs, ks, j);
+            const uint32_t r = addr(rs, ks, j);
             __stcg(psi + r, x[j]);
             if constexpr (ADJ) __stcg(lam + r, y[j]);
         }

@@ -4,6 +4,7 @@
 #include "host.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 namespace zxh {
@@ -55,8 +56,9 @@ bool AffBuild::init(int eb, int mm, const std::vector<U3Op> &gates, const std::v
         entries[d].clear();
         terms[d].clear();
     }
-    real = true;
-    if (m < kAffBits) return false;
+    form = 2;
+    dev.scale = 1.0;
+    if (m < kAffBits || m > kAffMaxBits) return false;
     dev.m = uint32_t(m);
     Room room;
     int nlow = 0, nhigh = 0;
@@ -116,12 +118,32 @@ bool AffBuild::init(int eb, int mm, const std::vector<U3Op> &gates, const std::v
         for (int q = 0; q < 4; q++) {
             d.u[2 * q] = w[q].real();
             d.u[2 * q + 1] = w[q].imag();
-            real = real && w[q].imag() == 0.0;
+            if (w[q].imag() != 0.0) form = 0;
         }
         d.sel = uint32_t(s);
         d.gen = gen ? (*gen)[i] : 0u;
         d.slot = slot ? (*slot)[i] : 0u;
         dev.gates |= 1u << at[i];
+        const double c = w[0].real(), sn = w[2].real();
+        // a product of rotations may miss the form by its rounding; an X generator's gradient
+        // (RX by a multiple of 2 pi is real) takes the general form
+        if (d.gen == 2 || std::fabs(c - w[3].real()) > 1e-15 || std::fabs(sn + w[1].real()) > 1e-15) form = std::min(form, 1);
+        const bool mu = std::fabs(c) < std::fabs(sn);
+        if (mu) {
+            dev.mu |= 1u << at[i];
+            (at[i] < kAffRun ? dev.mu_low : dev.mu_high) |= 1ULL << s;
+        }
+        d.rot = mu ? c / sn : sn / c;
+        dev.scale *= mu ? sn : c;
+    }
+    // the order gates are applied in: layouts A, C, B
+    double before = 1.0;
+    for (int k : {4, 5, 6, 7, 0, 1, 2, 3, 8, 9, 10, 11}) {
+        AffGateDev &d = dev.gate[k];
+        d.gscale = before;
+        if (!((dev.gates >> k) & 1)) continue;
+        const double f = ((dev.mu >> k) & 1) ? d.u[4] : d.u[0];
+        before *= f * f;
     }
     return true;
 }

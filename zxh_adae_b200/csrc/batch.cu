@@ -140,14 +140,24 @@ __device__ __forceinline__ void run_op_slice(const BatchOp &op, const uint8_t *b
     E *lam = arena + op.lam;
     double *gr = grads + op.grad_base;
     if constexpr (NT == kThreads) {  // tile: dynamic shared memory of the affine passes
+        // real queues: rotations, or any real gates
         if (op.kind == BOP_AFFINE) {
-            adev::affine_body<E, false, REAL>(*reinterpret_cast<adev::AffSmem<E, false> *>(tile), ob, op.off0, op.off1, psi,
-                                              psi, nullptr, nullptr, b, 1, e);
+            auto &as = *reinterpret_cast<adev::AffSmem<E, false> *>(tile);
+            if (REAL && op.aux == 2)
+                adev::affine_body<E, false, 2>(as, ob, op.off0, op.off1, psi, psi, nullptr, nullptr, uint32_t(b), 1,
+                                               uint32_t(e));
+            else
+                adev::affine_body<E, false, REAL ? 1 : 0>(as, ob, op.off0, op.off1, psi, psi, nullptr, nullptr, uint32_t(b),
+                                                          1, uint32_t(e));
             return;
         }
         if (op.kind == BOP_AFFINE_ADJ) {
-            adev::affine_body<E, true, REAL>(*reinterpret_cast<adev::AffSmem<E, true> *>(tile), ob, op.off0, op.off1, psi,
-                                             psi, lam, gr, b, 1, e);
+            auto &as = *reinterpret_cast<adev::AffSmem<E, true> *>(tile);
+            if (REAL && op.aux == 2)
+                adev::affine_body<E, true, 2>(as, ob, op.off0, op.off1, psi, psi, lam, gr, uint32_t(b), 1, uint32_t(e));
+            else
+                adev::affine_body<E, true, REAL ? 1 : 0>(as, ob, op.off0, op.off1, psi, psi, lam, gr, uint32_t(b), 1,
+                                                         uint32_t(e));
             return;
         }
     }

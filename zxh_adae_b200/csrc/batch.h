@@ -32,7 +32,8 @@ struct BatchOp {
     uint64_t base;                   // this op's descriptors start at blob + base
     uint64_t off0, off1, off2;       // GROW*, AFFINE*: pass descriptor, phase table; LAMBDA: terms;
                                      // DIAG_ADJ: gates, slots, phase table (all from base)
-    uint32_t aux, m;                 // LAMBDA: terms; DIAG_ADJ: gates; GROW*, AFFINE*: 1 if every gate is real; m: state bits
+    uint32_t aux, m;                 // LAMBDA: terms; DIAG_ADJ: gates; AFFINE*: the form of
+                                     // its gates; GROW*: 1 if every gate is real; m: state bits
     uint64_t psi, lam;               // element offsets of the circuit's states in the arena
     uint32_t grad_base, energy;      // the circuit's first gradient slot and its energy slot
 };

@@ -197,7 +197,7 @@ int compile(zxh_batch *b)
                 op.base = base;
                 op.off0 = ps.off;
                 op.off1 = ps.off2;
-                op.aux = ps.aff->real ? 1u : 0u;
+                op.aux = uint32_t(ps.aff->form);
             } else {
                 return bfail(b, ZXH_ERR_ARG, "circuit " + std::to_string(c) +
                                                  " needs a pass the batched launch does not run (n >= 6 required)");
@@ -243,7 +243,7 @@ int compile(zxh_batch *b)
                 op.base = gbase;
                 op.off0 = r.off;
                 op.off1 = r.toff;
-                op.aux = r.aff->real ? 1u : 0u;
+                op.aux = uint32_t(r.aff->form);
             } else if (r.kind == zxh::adj::RevStep::DIAG) {
                 op.kind = zxh::BOP_DIAG_ADJ;
                 op.units = uint64_t(1) << N;
@@ -375,11 +375,11 @@ int launch_op(zxh_batch *b, const BatchOp &op)
                           op.aux != 0, (zxh::PlanParams().grow_staged & 2) != 0, b->d_status, b->sms, b->stream);
         break;
     case zxh::BOP_AFFINE:
-        e = zxh::run_affine(b->d_blob + op.base, op.off0, op.off1, op.units, b->eb, op.aux != 0, psi, nullptr, nullptr,
+        e = zxh::run_affine(b->d_blob + op.base, op.off0, op.off1, op.units, b->eb, int(op.aux), psi, nullptr, nullptr,
                             nullptr, false, b->sms, b->stream);
         break;
     case zxh::BOP_AFFINE_ADJ:
-        e = zxh::run_affine(b->d_blob + op.base, op.off0, op.off1, op.units, b->eb, op.aux != 0, psi, nullptr, lam, gr,
+        e = zxh::run_affine(b->d_blob + op.base, op.off0, op.off1, op.units, b->eb, int(op.aux), psi, nullptr, lam, gr,
                             false, b->sms, b->stream);
         break;
     case zxh::BOP_LAMBDA:

@@ -955,8 +955,10 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
     int m = start.m;
 
     // 1. Product-state prefix: expansions whose selector is constant on the old
-    //    bits, starting from |0...0>, and diagonal windows made only of P phases on
-    //    existing bits / constant selectors. The prefix is written in one pass.
+    //    bits, starting from |0...0>, batches of gates each on a bit no gate has touched
+    //    (under eager_expand_all the first layer: its passes over a state that is still
+    //    |0...0> would cost as much as any layer's), and diagonal windows made only of P
+    //    phases on existing bits / constant selectors. The prefix is written in one pass.
     if (start.fresh && pp.grow_only) {
         Pass ps;
         ps.kind = Pass::INIT;
@@ -972,9 +974,29 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
             v[b][0] = cd(1.0, 0.0);
             v[b][1] = cd(0.0, 0.0);
         }
+        uint64_t untouched = low_mask(pm);
         size_t j = 0;
         for (; j < ops.size(); j++) {
             const Op &op = ops[j];
+            if (op.kind == Op::U3BATCH) {
+                uint64_t bits = 0;
+                bool ok = op.m == pm;
+                for (const U3Op &u : op.u3) {
+                    ok = ok && !u.has_ctrl && u.delta && single_bit_or_zero(u.delta) && u.sel.alpha == u.delta;
+                    bits |= u.delta;
+                }
+                if (!ok || (bits & ~untouched)) break;
+                untouched &= ~bits;
+                for (const U3Op &u : op.u3) {
+                    // the bit's |0> (its selector 0) is bit value beta
+                    cd *w = v[bit_index(u.delta)];
+                    const int z = u.sel.beta;
+                    const cd a = w[z], b = w[z ^ 1];
+                    w[z] = u.u[0] * a + u.u[1] * b;
+                    w[z ^ 1] = u.u[2] * a + u.u[3] * b;
+                }
+                continue;
+            }
             if (op.kind == Op::EXPAND) {
                 const U3Op &u = op.u3[0];
                 const uint64_t old_alpha = u.sel.alpha & low_mask(pm);
@@ -1657,7 +1679,7 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
         if ((pp.grow || pp.grow_only) && grow_ok(op)) {
             const int mm = op.m;
             const size_t first = out.passes.size();
-            const bool tiles = pp.affine && (!pp.grow_only || pp.grow_tiles) && op.deltas && mm >= kAffBits;
+            const bool tiles = pp.affine && (!pp.grow_only || pp.grow_tiles) && op.deltas && mm >= kAffBits && mm <= kAffMaxBits;
             bool done = tiles && emit_affine(op);
             if (!done) {
                 out.passes.resize(first);

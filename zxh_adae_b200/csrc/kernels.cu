@@ -537,7 +537,7 @@ cudaError_t run_passes(const std::vector<Pass> &passes, const uint8_t *dblob, vo
         } else if (ps.kind == Pass::AFFINE) {
             void *dst = (i + 1 == passes.size() && last_dst) ? last_dst : state;
             const void *src = (i == 0 && first_src) ? first_src : (dst != state ? state : nullptr);
-            e = run_affine(dblob, ps.off, ps.off2, ps.aff->dev.ntiles, elem_bytes, ps.aff->real, dst, src, nullptr,
+            e = run_affine(dblob, ps.off, ps.off2, ps.aff->dev.ntiles, elem_bytes, ps.aff->form, dst, src, nullptr,
                            nullptr, i > 0, sms, st);
         } else if (ps.kind == Pass::DIAG) {
             e = run_diag(dblob, ps.off, ps.off2, ps.m, elem_bytes, ps.row_bits, ps.chunk_bits, ps.prefetch != 0, state, status,

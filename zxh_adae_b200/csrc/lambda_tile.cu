@@ -64,7 +64,7 @@ __device__ __forceinline__ double flip_sign(double c, uint32_t s)
 // MODE 0: energy only; 1: lam is written; 2: lam is added to. With lam the energy comes from
 // the whole of it, in the last pass (last != 0).
 template <typename E, int MODE>
-__global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 2 : 1)
+__global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? (MODE == 0 ? 3 : 2) : 1)
     lambda_tile_kernel(const E *psi, E *lam, const __grid_constant__ LamPassDev p,
                        const TermDev *__restrict__ terms, double *energy, int last)
 {
