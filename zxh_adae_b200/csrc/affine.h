@@ -24,9 +24,10 @@ __host__ __device__ constexpr int aff_pair(int i, int j) { return i * (2 * kAffH
 
 // The gate on a coordinate: u00, u01, u10, u11 (re, im; U^dagger in adjoint passes), its
 // qubit's selector, the gradient's generator (0 none, 1 Y, 2 X) and slot.
-// Rotation passes: one coefficient of [[c, -s], [s, c]] factored out, rot = s / c and factor c
-// where |c| >= |s|, else (bit of AffDev::mu) rot = c / s and factor s; gscale is the square of
-// the factors of the gates applied before it.
+// Factored passes: one coefficient of a rotation [[c, -s], [s, c]] or a reflection [[c, s],
+// [s, -c]] (bit of AffDev::refl) factored out, rot = s / c and factor c where |c| >= |s|, else
+// (bit of AffDev::mu) rot = c / s and factor s; gscale is the square of the factors of the
+// gates applied before it.
 struct AffGateDev {
     double u[8];
     double rot, gscale;
@@ -60,11 +61,11 @@ struct AffWinDev {
 };
 
 struct AffDev {
-    uint32_t m, gates, nsel;       // gates: bit k = coordinate k has one
-    uint32_t mu;                   // rotation passes: the gates with rot = c / s
-    double scale;                  // rotation passes: the product of the factors,
-    uint64_t mu_high, mu_low;      // negated by the parity of these selector bits (high coordinates'
-                                   // gates: of the run position; low ones': of the tile)
+    uint32_t m, gates, nsel, pad;  // gates: bit k = coordinate k has one
+    uint32_t mu, refl;             // factored passes: the gates with rot = c / s, the reflections
+    double scale;                  // the product of the factors, negated by the parity of these
+    uint64_t neg_high, neg_low;    // selector bits (high coordinates' gates: of the run position;
+                                   // low ones': of the tile)
     uint64_t ntiles;
     uint64_t basis[kAffBits], tr[64];      // tile coordinates; real vectors of the tile bits
     uint64_t alpha[kAffMaxSel], lw[1 << kAffRun];  // selector masks; bit s of lw[l]: f_s of run position l
@@ -79,7 +80,7 @@ struct AffBuild {
     AffDev dev;
     std::vector<AffEntryDev> entries[2];
     std::vector<AffTermDev> terms[2];
-    // 0: complex matrices; 1: every gate's is real; 2: every gate is a real rotation (affine_body)
+    // 0: complex matrices; 1: every gate's is real; 2: every gate is a real rotation or reflection
     int form = 2;
 
     // The coordinates of a pass: up to 8 deltas independent modulo the run bits (high), up to 4

@@ -22,6 +22,9 @@ template <typename E, bool ADJ>
 struct AffSmem {
     using RT = typename ET<E>::R;
     static constexpr int NW = ADJ ? 1 : 2;  // windows
+    // The windows' entries: in shared memory, but for complex128 forward passes, where L1 serves
+    // the space better (24-qubit ansatz 2.86 -> 2.64 ms; complex64 1.32 -> 1.36).
+    static constexpr bool ENT = ADJ || sizeof(E) == 8;
     E slab[ADJ ? 2 : 1][1 << kAffBits];      // adjoint passes: also the sums and marginals of w
     E exp[1 << kExpTableBits];
     RT u[kAffBits][2][8];  // [1]: the |1> member first
@@ -31,7 +34,7 @@ struct AffSmem {
     uint64_t lw[kRun];
     uint32_t alpha[kAffMaxSel], basis[kAffBits];
     AffWinDev win[NW];
-    AffEntryDev ent[NW][kAffMaxEntries];
+    AffEntryDev ent[ENT ? NW : 1][ENT ? kAffMaxEntries : 1];
     int64_t K[NW][kRun], w[NW][kRun][kAffHigh], q[NW][kRun][kAffPairs];
     AffTermDev term[ADJ ? kAffMaxTerms : 1];
     uint8_t plist[kAffPairs];
@@ -39,7 +42,10 @@ struct AffSmem {
     double gacc[ADJ ? kAffBits : 1][ADJ ? kThreads : 1];
 };
 
-__device__ __forceinline__ uint32_t slot_of(uint32_t i) { return i ^ ((i >> 4) & 15u); }
+// SWZ: the exchanges of layout C, whose half warps differ in coordinates 4..7; between A and B
+// (coordinates 0..3) the plain index serves, with every register at a constant offset.
+template <bool SWZ>
+__host__ __device__ constexpr uint32_t slot_of(uint32_t i) { return SWZ ? i ^ ((i >> 4) & 15u) : i; }
 
 // Registers j of layout L (0 A, 1 B, 2 C) in tile index bits.
 template <int L>
@@ -55,18 +61,19 @@ __device__ __forceinline__ uint32_t fixed_bits(uint32_t lane, uint32_t warp)
 template <int LA, int LB, int NS, typename E>
 __device__ __forceinline__ void exchange(E (&x)[kNR], E (&y)[kNR], E (*slab)[1 << kAffBits], uint32_t lane, uint32_t warp)
 {
-    const uint32_t a = slot_of(fixed_bits<LA>(lane, warp)), b = slot_of(fixed_bits<LB>(lane, warp));
+    constexpr bool SWZ = LA == 2 || LB == 2;
+    const uint32_t a = slot_of<SWZ>(fixed_bits<LA>(lane, warp)), b = slot_of<SWZ>(fixed_bits<LB>(lane, warp));
     __syncthreads();  // the slab's previous reads are done
 #pragma unroll
     for (int j = 0; j < kNR; j++) {
-        const uint32_t s = a ^ (reg_bits<LA>(j) ^ ((reg_bits<LA>(j) >> 4) & 15u));
+        const uint32_t s = SWZ ? a ^ slot_of<SWZ>(reg_bits<LA>(j)) : a + reg_bits<LA>(j);
         slab[0][s] = x[j];
         if constexpr (NS == 2) slab[1][s] = y[j];
     }
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < kNR; j++) {
-        const uint32_t s = b ^ (reg_bits<LB>(j) ^ ((reg_bits<LB>(j) >> 4) & 15u));
+        const uint32_t s = SWZ ? b ^ slot_of<SWZ>(reg_bits<LB>(j)) : b + reg_bits<LB>(j);
         x[j] = slab[0][s];
         if constexpr (NS == 2) y[j] = slab[1][s];
     }
@@ -146,12 +153,41 @@ __device__ __forceinline__ double2 axpy(double c, double2 a, double2 b)
 __device__ __forceinline__ float2 scaled(float c, float2 a) { return __fmul2_rn(make_float2(c, c), a); }
 __device__ __forceinline__ double2 scaled(double c, double2 a) { return make_double2(c * a.x, c * a.y); }
 
-// A rotation with one coefficient factored out: half the multiply-adds of gate(). r: its
-// coefficient, negated where the thread's pairs start at the |1> member (flip); with
-// rot = c / s that also negates the factor (AffDev::mu_high, mu_low).
+// One half of a factored gate on a state: lo' = a lo + p hi, hi' = q lo + b hi with
+//   rotation   (rot = s / c)  lo - r hi, hi + r lo     (rot = c / s)  r lo - hi, lo + r hi
+//   reflection (rot = s / c)  lo + r hi, r lo - hi     (rot = c / s)  r lo + hi, lo - r hi
+template <int RR, bool MU, bool REFL, typename E, typename RT>
+__device__ __forceinline__ void factored(E (&x)[kNR], RT r)
+{
+    constexpr int B = 1 << RR;
+    const RT nr = -r;
+#pragma unroll
+    for (int j = 0; j < kNR; j++) {
+        if ((j >> RR) & 1) continue;
+        const E lo = x[j], hi = x[j | B];
+        if constexpr (!MU && !REFL) {
+            x[j] = axpy(nr, hi, lo);
+            x[j | B] = axpy(r, lo, hi);
+        } else if constexpr (!REFL) {
+            x[j] = axpy(r, lo, neg(hi));
+            x[j | B] = axpy(r, hi, lo);
+        } else if constexpr (!MU) {
+            x[j] = axpy(r, hi, lo);
+            x[j | B] = axpy(r, lo, neg(hi));
+        } else {
+            x[j] = axpy(r, lo, hi);
+            x[j | B] = axpy(nr, hi, lo);
+        }
+    }
+}
+
+// A rotation or reflection with one coefficient factored out: half the multiply-adds of
+// gate(), and one rounding less. r: its coefficient, negated where the thread's pairs start
+// at the |1> member (flip). One branch per form around whole loops: inside them the compiler
+// computes every form.
 template <int RR, bool ADJ, typename E, typename RT>
-__device__ __forceinline__ void rotation(E (&x)[kNR], E (&y)[kNR], RT r, bool mu, bool flip, uint32_t gen, double gscale,
-                                         double *acc)
+__device__ __forceinline__ void factored_gate(E (&x)[kNR], E (&y)[kNR], RT r, bool mu, bool refl, bool flip, uint32_t gen,
+                                              double gscale, double *acc)
 {
     constexpr int B = 1 << RR;
     if constexpr (ADJ) {
@@ -167,50 +203,35 @@ __device__ __forceinline__ void rotation(E (&x)[kNR], E (&y)[kNR], RT r, bool mu
             *acc += gscale * (flip ? -part : part);
         }
     }
-    if (mu) {  // one branch around each form: inside the loop the compiler computes both
-#pragma unroll
-        for (int j = 0; j < kNR; j++) {
-            if ((j >> RR) & 1) continue;
-            const E lo = x[j], hi = x[j | B];
-            x[j] = axpy(r, lo, neg(hi));
-            x[j | B] = axpy(r, hi, lo);
-            if constexpr (ADJ) {
-                const E llo = y[j], lhi = y[j | B];
-                y[j] = axpy(r, llo, neg(lhi));
-                y[j | B] = axpy(r, lhi, llo);
-            }
-        }
+    auto both = [&](auto m, auto f) {
+        factored<RR, decltype(m)::value, decltype(f)::value>(x, r);
+        if constexpr (ADJ) factored<RR, decltype(m)::value, decltype(f)::value>(y, r);
+    };
+    using T = std::true_type;
+    using F = std::false_type;
+    if (!refl) {
+        if (mu) both(T(), F());
+        else both(F(), F());
     } else {
-        const RT nr = -r;
-#pragma unroll
-        for (int j = 0; j < kNR; j++) {
-            if ((j >> RR) & 1) continue;
-            const E lo = x[j], hi = x[j | B];
-            x[j] = axpy(nr, hi, lo);
-            x[j | B] = axpy(r, lo, hi);
-            if constexpr (ADJ) {
-                const E llo = y[j], lhi = y[j | B];
-                y[j] = axpy(nr, lhi, llo);
-                y[j | B] = axpy(r, llo, lhi);
-            }
-        }
+        if (mu) both(T(), T());
+        else both(F(), T());
     }
 }
 
 // The gates on coordinates K0 .. K0 + 3, the layout's registers; c: the selector bits of
 // the thread (of the tile, in layout C).
 template <int K0, bool ADJ, int FORM, typename E, typename SM>
-__device__ __forceinline__ void gates(E (&x)[kNR], E (&y)[kNR], uint32_t mask, uint32_t mu, uint64_t c, SM &sm,
+__device__ __forceinline__ void gates(E (&x)[kNR], E (&y)[kNR], uint32_t mask, uint32_t mu, uint32_t refl, uint64_t c, SM &sm,
                                       uint32_t tid)
 {
     auto one = [&](auto rr) {
         constexpr int RR = decltype(rr)::value, k = K0 + RR;
         if (!((mask >> k) & 1u)) return;
-        const bool flip = (c >> sm.sel[k]) & 1;
+        const bool flip = (uint32_t(c) >> sm.sel[k]) & 1u;  // the gates' selectors are the first ones
         double *acc = ADJ ? &sm.gacc[ADJ ? k : 0][ADJ ? tid : 0] : nullptr;
         if constexpr (FORM == 2) {
             const auto r = sm.rot[k];
-            rotation<RR, ADJ>(x, y, flip ? -r : r, (mu >> k) & 1u, flip, sm.gen[k], sm.gscale[k], acc);
+            factored_gate<RR, ADJ>(x, y, flip ? -r : r, (mu >> k) & 1u, (refl >> k) & 1u, flip, sm.gen[k], sm.gscale[k], acc);
         } else {
             gate<RR, ADJ, FORM == 1>(x, y, sm.u[k][flip], flip, sm.gen[k], acc);
         }
@@ -224,18 +245,19 @@ __device__ __forceinline__ void gates(E (&x)[kNR], E (&y)[kNR], uint32_t mask, u
 // Window d's polynomial at run position l, by the 16 threads part = 0..15 of that position:
 // all take shares of the entries without a coordinate, thread k < 8 those of coordinate k.
 template <typename SM>
-__device__ __forceinline__ void window_eval(SM &sm, const AffWinDev &wd, int d, uint64_t c, uint32_t part, uint32_t l)
+__device__ __forceinline__ void window_eval(SM &sm, const AffEntryDev *ent, const AffWinDev &wd, int d, uint64_t c,
+                                            uint32_t part, uint32_t l)
 {
     int64_t K = 0;
     for (uint32_t e = part; e < wd.n0; e += 16u) {
-        const AffEntryDev t = sm.ent[d][e];
+        const AffEntryDev t = ent[e];
         const bool on = ((c >> t.s0) & 1) && (t.s1 == 0xff || ((c >> t.s1) & 1));
         if (on) K += t.coef;
     }
     if (part < uint32_t(kAffHigh)) {
         int64_t w = 0;
         for (uint32_t e = wd.ck[part]; e < wd.ck[part + 1]; e++) {
-            const AffEntryDev t = sm.ent[d][e];
+            const AffEntryDev t = ent[e];
             const bool f0 = (c >> t.s0) & 1, f1 = t.s1 != 0xff && ((c >> t.s1) & 1);
             const int64_t slope = f0 ? -t.coef : t.coef;  // S = f + y (1 - 2 f)
             if (t.kind == 3) {
@@ -425,8 +447,8 @@ __device__ __forceinline__ void affine_body(AffSmem<E, ADJ> &sm, const uint8_t *
     using RT = typename ET<E>::R;
     const AffDev &p = *reinterpret_cast<const AffDev *>(blob + poff);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t mask = p.gates, mu = p.mu, nsel = p.nsel;
-    const uint64_t mu_high = p.mu_high, mu_low = p.mu_low;
+    const uint32_t mask = p.gates, mu = p.mu, refl = p.refl, nsel = p.nsel;
+    const uint64_t neg_high = p.neg_high, neg_low = p.neg_low;
     const RT scale = RT(p.scale);
     const AffWinDev &w0 = sm.win[0], &w1 = sm.win[SM::NW - 1];
     const bool win0 = p.win[0].nterms != 0, win1 = !ADJ && p.win[1].nterms != 0;
@@ -438,11 +460,11 @@ __device__ __forceinline__ void affine_body(AffSmem<E, ADJ> &sm, const uint8_t *
     if (win0 || win1) {
         const E *tab = reinterpret_cast<const E *>(blob + toff);
         for (uint32_t i = tid; i < (1u << kExpTableBits); i += kThreads) sm.exp[i] = tab[i];
-        for (int d = 0; d < SM::NW; d++) {
-            const AffWinDev &wd = sm.win[d];
-            const AffEntryDev *e = reinterpret_cast<const AffEntryDev *>(blob + wd.off_entries);
-            for (uint32_t i = tid; i < wd.ck[kAffHigh]; i += kThreads) sm.ent[d][i] = e[i];
-        }
+        if constexpr (SM::ENT)
+            for (int d = 0; d < SM::NW; d++) {
+                const AffEntryDev *e = reinterpret_cast<const AffEntryDev *>(blob + sm.win[d].off_entries);
+                for (uint32_t i = tid; i < sm.win[d].ck[kAffHigh]; i += kThreads) sm.ent[d][i] = e[i];
+            }
     }
     if (tid < kAffBits) {
         const AffGateDev &g = p.gate[tid];
@@ -491,6 +513,11 @@ __device__ __forceinline__ void affine_body(AffSmem<E, ADJ> &sm, const uint8_t *
             rb ^= sm.basis[5 + b];
         }
     const uint32_t trl = uint32_t(p.tr[lane]);  // at most 20 tile bits
+    auto entries = [&](int d) {
+        return SM::ENT ? sm.ent[SM::ENT ? d : 0] : reinterpret_cast<const AffEntryDev *>(blob + sm.win[d].off_entries);
+    };
+    const AffEntryDev *ent0 = entries(0);
+    [[maybe_unused]] const AffEntryDev *ent1 = entries(SM::NW - 1);
     const bool need_c = (mask & 0x00fu) != 0, need_b = need_c || (mask & 0xf00u) != 0 || win1;
     const uint64_t lw = sm.lw[lane & 15u], lw0 = sm.lw[0], lwe = sm.lw[tid >> 4];
 
@@ -505,18 +532,18 @@ __device__ __forceinline__ void affine_body(AffSmem<E, ADJ> &sm, const uint8_t *
     chain_wait();  // everything above reads only the program
     for (uint32_t t = first; t < end; t += step) {
         const uint32_t r0 = rn;
-        auto addr = [&](uint32_t base, int k0, int j) {
-#pragma unroll
-            for (int b = 0; b < 4; b++)
-                if ((j >> b) & 1) base ^= sm.basis[k0 + b];
-            return base;
-        };
         E x[kNR], y[kNR];
+        {
+            // the registers in Gray-code order: one XOR per address
+            const uint32_t g[4] = {sm.basis[4], sm.basis[5], sm.basis[6], sm.basis[7]};
+            uint32_t r = r0 ^ ra;
 #pragma unroll
-        for (int j = 0; j < kNR; j++) {
-            const uint32_t r = addr(r0 ^ ra, 4, j);
-            x[j] = __ldcg(src + r);
-            if constexpr (ADJ) y[j] = __ldcg(lam + r);
+            for (int i = 0; i < kNR; i++) {
+                const int j = i ^ (i >> 1);
+                if (i) r ^= g[ctz_const(i)];
+                x[j] = __ldcg(src + r);
+                if constexpr (ADJ) y[j] = __ldcg(lam + r);
+            }
         }
         if (t + step < end) {
             rn = tile_base(t + step);
@@ -534,9 +561,9 @@ __device__ __forceinline__ void affine_body(AffSmem<E, ADJ> &sm, const uint8_t *
         const uint64_t c = P ^ lw;
         if (win0 || win1) {
             __syncthreads();  // the previous tile's polynomials and sums are read
-            if (win0) window_eval(sm, w0, 0, P ^ lwe, tid & 15u, tid >> 4);
+            if (win0) window_eval(sm, ent0, w0, 0, P ^ lwe, tid & 15u, tid >> 4);
             if constexpr (!ADJ) {
-                if (win1) window_eval(sm, w1, 1, P ^ lwe, tid & 15u, tid >> 4);
+                if (win1) window_eval(sm, ent1, w1, 1, P ^ lwe, tid & 15u, tid >> 4);
             }
             __syncthreads();
         }
@@ -544,33 +571,37 @@ __device__ __forceinline__ void affine_body(AffSmem<E, ADJ> &sm, const uint8_t *
             if constexpr (ADJ) window_grad(x, y, sm, w0, P, tid);
             window_apply<0, ADJ>(x, y, sm, w0.pairs, 0, lane, warp);
         }
-        gates<4, ADJ, FORM>(x, y, mask, mu, c, sm, tid);
+        gates<4, ADJ, FORM>(x, y, mask, mu, refl, c, sm, tid);
         if (need_c) {
             exchange<0, 2, ADJ ? 2 : 1>(x, y, sm.slab, lane, warp);
-            gates<0, ADJ, FORM>(x, y, mask, mu, P ^ lw0, sm, tid);
+            gates<0, ADJ, FORM>(x, y, mask, mu, refl, P ^ lw0, sm, tid);
             exchange<2, 1, ADJ ? 2 : 1>(x, y, sm.slab, lane, warp);
         } else if (need_b) {
             exchange<0, 1, ADJ ? 2 : 1>(x, y, sm.slab, lane, warp);
         }
-        if (need_b) gates<8, ADJ, FORM>(x, y, mask, mu, c, sm, tid);
+        if (need_b) gates<8, ADJ, FORM>(x, y, mask, mu, refl, c, sm, tid);
         if constexpr (!ADJ) {
             if (win1) window_apply<1, false>(x, y, sm, w1.pairs, 1, lane, warp);
         }
         if (FORM == 2 && mask) {
-            const RT f = (par64(c & mu_high) ^ par64((P ^ lw0) & mu_low)) ? -scale : scale;
+            const RT f = (par64(c & neg_high) ^ par64((P ^ lw0) & neg_low)) ? -scale : scale;
 #pragma unroll
             for (int j = 0; j < kNR; j++) {
                 x[j] = scaled(f, x[j]);
                 if constexpr (ADJ) y[j] = scaled(f, y[j]);
             }
         }
-        const uint32_t rs = r0 ^ (need_b ? rb : ra);
-        const int ks = need_b ? 8 : 4;
+        {
+            const uint32_t *gb = sm.basis + (need_b ? 8 : 4);
+            const uint32_t g[4] = {gb[0], gb[1], gb[2], gb[3]};
+            uint32_t r = r0 ^ (need_b ? rb : ra);
 #pragma unroll
-        for (int j = 0; j < kNR; j++) {
-            const uint32_t r = addr(rs, ks, j);
-            __stcg(psi + r, x[j]);
-            if constexpr (ADJ) __stcg(lam + r, y[j]);
+            for (int i = 0; i < kNR; i++) {
+                const int j = i ^ (i >> 1);
+                if (i) r ^= g[ctz_const(i)];
+                __stcg(psi + r, x[j]);
+                if constexpr (ADJ) __stcg(lam + r, y[j]);
+            }
         }
     }
     if constexpr (ADJ) {

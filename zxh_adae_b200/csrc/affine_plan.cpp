@@ -20,6 +20,9 @@ uint64_t reduced(uint64_t v, const std::vector<uint64_t> &ech)
     return v;
 }
 
+// What a product of rotations, or exp(i pi) in an H, may miss its form by.
+constexpr double kRound = 1e-15;
+
 void insert(uint64_t v, std::vector<uint64_t> &ech)
 {
     ech.push_back(v);
@@ -118,21 +121,22 @@ bool AffBuild::init(int eb, int mm, const std::vector<U3Op> &gates, const std::v
         for (int q = 0; q < 4; q++) {
             d.u[2 * q] = w[q].real();
             d.u[2 * q + 1] = w[q].imag();
-            if (w[q].imag() != 0.0) form = 0;
+            if (std::fabs(w[q].imag()) > kRound) form = 0;
         }
         d.sel = uint32_t(s);
         d.gen = gen ? (*gen)[i] : 0u;
         d.slot = slot ? (*slot)[i] : 0u;
         dev.gates |= 1u << at[i];
         const double c = w[0].real(), sn = w[2].real();
-        // a product of rotations may miss the form by its rounding; an X generator's gradient
-        // (RX by a multiple of 2 pi is real) takes the general form
-        if (d.gen == 2 || std::fabs(c - w[3].real()) > 1e-15 || std::fabs(sn + w[1].real()) > 1e-15) form = std::min(form, 1);
+        const bool rot = std::fabs(c - w[3].real()) <= kRound && std::fabs(sn + w[1].real()) <= kRound;
+        const bool refl = std::fabs(c + w[3].real()) <= kRound && std::fabs(sn - w[1].real()) <= kRound;
+        // an X generator's gradient (RX by a multiple of 2 pi is real) takes the general form
+        if (d.gen == 2 || !(rot || refl)) form = std::min(form, 1);
         const bool mu = std::fabs(c) < std::fabs(sn);
-        if (mu) {
-            dev.mu |= 1u << at[i];
-            (at[i] < kAffRun ? dev.mu_low : dev.mu_high) |= 1ULL << s;
-        }
+        if (mu) dev.mu |= 1u << at[i];
+        if (!rot) dev.refl |= 1u << at[i];
+        // from the other member of a pair the factor changes sign: a rotation's s, a reflection's c
+        if (mu == rot) (at[i] < kAffRun ? dev.neg_low : dev.neg_high) |= 1ULL << s;
         d.rot = mu ? c / sn : sn / c;
         dev.scale *= mu ? sn : c;
     }
