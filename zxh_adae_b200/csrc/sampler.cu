@@ -384,15 +384,17 @@ __global__ void __launch_bounds__(kThreads) small_draw_kernel(const double *mass
     }
 }
 
-// segments hit by at most kWarpMax shots; a warp takes `group` (at most 32) consecutive
-// segments. Registers are capped so that 4 CTAs fit an SM in complex64.
+// Segments hit by at most kWarpMax shots. Warp w takes segments w, w + W, w + 2 W, ... (W
+// warps in all): neighbouring segments of a state tend to have like masses, and a warp with 28
+// of them in a row held up the others (10^6 shots from an uneven product state of 29 qubits).
+// Registers are capped so that 4 CTAs fit an SM in complex64.
 template <typename E>
 __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 4 : 3) resolve_warp_kernel(const E *__restrict__ state, uint64_t nseg,
                                                                 uint32_t seglen, const unsigned long long *counts,
                                                                 const unsigned long long *offsets, uint64_t stream2,
                                                                 uint64_t *__restrict__ real_out,
                                                                 uint32_t *heavy_list, uint32_t *heavy_count,
-                                                                const double *parts, uint32_t group)
+                                                                const double *parts)
 {
     chain_trigger();
     chain_wait();
@@ -400,16 +402,16 @@ __global__ void __launch_bounds__(kThreads, sizeof(E) == 8 ? 4 : 3) resolve_warp
     const uint64_t gwarp = (uint64_t(blockIdx.x) * kThreads + threadIdx.x) >> 5;
     const uint64_t nwarps = (uint64_t(gridDim.x) * kThreads) >> 5;
     const uint32_t per_lane = (seglen + 31) / 32;  // amplitudes owned by a lane
-    for (uint64_t g0 = gwarp * group; g0 < nseg; g0 += nwarps * group) {
-        const uint64_t gl = g0 + uint64_t(lane);
-        const unsigned long long cl = gl < nseg && uint32_t(lane) < group ? counts[gl] : 0ULL;
+    for (uint64_t g0 = gwarp; g0 < nseg; g0 += nwarps * 32) {
+        const uint64_t gl = g0 + uint64_t(lane) * nwarps;
+        const unsigned long long cl = gl < nseg ? counts[gl] : 0ULL;
         unsigned todo = __ballot_sync(0xffffffffu, cl != 0);
         if (cl > kWarpMax) heavy_list[atomicAdd(heavy_count, 1u)] = uint32_t(gl);
         todo &= __ballot_sync(0xffffffffu, cl <= kWarpMax);
         while (todo) {
             const int src = __ffs(todo) - 1;
             todo &= todo - 1;
-            const uint64_t g = g0 + uint64_t(src);
+            const uint64_t g = g0 + uint64_t(src) * nwarps;
             const unsigned long long cnt = __shfl_sync(0xffffffffu, cl, src);
             const unsigned long long off = offsets[g];
             const E *seg = state + g * seglen;
@@ -876,7 +878,10 @@ cudaError_t draw(const E *state, int m, uint64_t shots, uint64_t stream_seed, ui
         seg_mass_kernel<E><<<grid((nseg * 32 + kThreads - 1) / kThreads), kThreads, 0, st>>>(state, nseg, seglen, sc.segcdf,
                                                                                           sc.parts);
     kernels++;
-    if (nblk == 1 && shots <= kSmallShots) {
+    // Only a small draw's launches are chained (chain.cuh): in a large one the next kernel's
+    // waiting CTAs take room from the one that runs (10^6 shots at 27 qubits 0.54 instead of 0.49 ms).
+    const bool small = nblk == 1 && shots <= kSmallShots;
+    if (small) {
         const cudaError_t e = launch_chained(true, small_draw_kernel, 1, kThreads, 0, st, sc.segcdf, nseg, stream_seed,
                                              shots, sc.counts, sc.offsets, sc.heavy_count);
         if (e != cudaSuccess) return e;
@@ -897,24 +902,20 @@ cudaError_t draw(const E *state, int m, uint64_t shots, uint64_t stream_seed, ui
                                                                                          sc.offsets);
         kernels += 7;
     }
-    // Segments per warp: as few as give every warp that fits on the chip (4 CTAs an SM) one
-    // group, so that a small state's segments are not queued behind one another (20 qubits:
-    // 256 segments on 8 warps, 120 us) and a large one's fill the chip.
-    const uint64_t warps = uint64_t(sms) * 4 * (kThreads / 32);
-    const uint32_t group = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(32, (nseg + warps - 1) / warps)));
-    const uint64_t groups = (nseg + group - 1) / group;
-    cudaError_t e = launch_chained(true, resolve_warp_kernel<E>, grid((groups * 32 + kThreads - 1) / kThreads), kThreads, 0,
-                                   st, state, nseg, seglen, sc.counts, sc.offsets, stream2, real_out, sc.heavy_list,
-                                   sc.heavy_count, sc.parts, group);
+    // a warp per segment, as many warps as fit on the chip (4 CTAs an SM); 32 segments queued
+    // on each warp left a 20-qubit state's 256 to 8 warps (120 us)
+    const uint64_t ctas = std::min<uint64_t>((nseg * 32 + kThreads - 1) / kThreads, uint64_t(sms) * 4);
+    cudaError_t e = launch_chained(small, resolve_warp_kernel<E>, grid(ctas), kThreads, 0, st, state, nseg, seglen, sc.counts,
+                                   sc.offsets, stream2, real_out, sc.heavy_list, sc.heavy_count, sc.parts);
     kernels++;
     if (e == cudaSuccess && shots > kWarpMax) {  // fewer cannot make a segment heavy
         const size_t smem = size_t(seglen + seglen / 16 + 1) * 8;
-        e = launch_chained(true, resolve_cta_kernel<E>, grid(std::min<uint64_t>(nseg, uint64_t(sms) * 2)), kThreads, smem, st,
+        e = launch_chained(small, resolve_cta_kernel<E>, grid(std::min<uint64_t>(nseg, uint64_t(sms) * 2)), kThreads, smem, st,
                            state, seglen, sc.counts, sc.offsets, stream2, real_out, sc.heavy_list, sc.heavy_count);
         kernels++;
     }
     if (e == cudaSuccess && words) {
-        e = launch_chained(true, map_kernel, grid((shots + kThreads - 1) / kThreads), kThreads, 0, st, real_out, shots, cols,
+        e = launch_chained(small, map_kernel, grid((shots + kThreads - 1) / kThreads), kThreads, 0, st, real_out, shots, cols,
                            words);
         kernels++;
     }
