@@ -288,10 +288,13 @@ int zxh_batch_gradient_offsets(const zxh_batch *batch, size_t *offsets);
  * that launch from a CUDA graph captured on first use. */
 int zxh_batch_run(zxh_batch *batch, int mode, double *energies, double *grads, size_t ngrads);
 /* Knobs: grow_regs (1..4, gates with high deltas per general strided pass),
- * adj_regs (1..3, the same for the reverse passes), task_items (pass items per
- * task), task_elems (amplitudes per task of the element-wise passes); setting
- * one of these recompiles the batch. threads (64, 128 or 256): threads per CTA
- * of the persistent kernel, i.e. the warps that work on one task.
+ * adj_regs (1..3, the same for the reverse passes), task_items (most pass items per
+ * task; a sixteenth of it in tiles), task_elems (most amplitudes per task of the
+ * element-wise passes; a level of the queue is cut into smaller tasks where these
+ * leave fewer than two an SM); setting one of these recompiles the batch. threads
+ * (64, 128 or 256): threads per CTA of the persistent kernel, i.e. the warps that
+ * work on one task; only 256 runs affine tile passes (circuits of 12 to 32
+ * qubits), so a change to or from it recompiles the batch.
  * wait_limit_log2 (0..31, default 31): a persistent task waits at most
  * 2^wait_limit_log2 SM clocks for the previous pass of its circuit, then the run
  * ends early and zxh_batch_run returns ZXH_ERR_TIMEOUT; the handle stays usable
@@ -338,8 +341,9 @@ int zxh_optimize_gates(size_t n, int level, const zxh_gate *gates, size_t count,
  * diag_row_bits_c64, diag_row_bits_c128 (log2 rows of its warp tile), grow (1:
  * U3 batches whose pair deltas span several bits use the general strided pass,
  * 0: the TMA tile / global pair passes), affine (1: such batches, and the adjoint
- * sweep, run as affine tile passes on states of at least 2^12 amplitudes with
- * every qubit expanded, 0: the register-row form of the general strided pass), grow_regs (1..4: gates with high deltas per
+ * sweep, run as affine tile passes on states of 2^12 to 2^32 amplitudes with
+ * every qubit expanded, 0: the register-row form of the general strided pass,
+ * the only one grow_regs, adj_regs and grow_staged act on), grow_regs (1..4: gates with high deltas per
  * general strided pass), grow_only (1: plan every batch and window as general
  * strided passes after a |0...0> init, the pass set of the batched launch; needs
  * eager_expand_all), adj_windows (1: the adjoint sweep undoes diagonal gates

