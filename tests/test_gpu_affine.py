@@ -167,6 +167,25 @@ def test_affine_rotations_at_the_ends_of_their_forms(dtype):
     s.close()
 
 
+@pytest.mark.parametrize("turn", [9e-16, 2e-16, 5e-17])
+def test_affine_gates_next_to_a_rotation_keep_their_phase(turn):
+    # complex128: real amplitudes, then U3 gates whose imaginary parts are a fraction of
+    # an ulp of 1; the state's imaginary part is their sum and carries no other error than
+    # its own rounding (a relative 2^-53 per gate and amplitude; 1e-12 is 4500 of them)
+    n = 12
+    g = as_records([(U3, 0, q, 0.4 + 0.1 * q, 0.0, 0.0) for q in range(n)] + [(CX, i, i + 1) for i in range(n - 1)] +
+                   [(U3, 0, q, 1.1 + 0.1 * q, turn, 0.0) for q in range(n)])
+    o = Oracle(n)
+    o.push(g)
+    o.execute()
+    want = o.get_state(0).imag
+    s = ZXH(n, dtype="complex128")
+    s.push_gates(g)
+    s.execute()
+    assert np.linalg.norm(s.get_state(0).imag - want) <= 1e-12 * np.linalg.norm(want)
+    s.close()
+
+
 @pytest.mark.parametrize("mode", ["persistent", "graph", "sequential"])
 @pytest.mark.parametrize("dtype", ["complex64", "complex128"])
 def test_batched_tiles_against_dense_adjoint(mode, dtype):

@@ -20,8 +20,16 @@ uint64_t reduced(uint64_t v, const std::vector<uint64_t> &ech)
     return v;
 }
 
-// What a product of rotations, or exp(i pi) in an H, may miss its form by.
-constexpr double kRound = 1e-15;
+// H as u3_matrix rounds it: exp(i pi) leaves imaginary parts of 8.7e-17 that the gate has not.
+bool is_h(const cd u[4])
+{
+    static const std::vector<cd> h = [] {
+        std::vector<cd> m(4);
+        u3_matrix(std::acos(-1.0) / 2.0, std::acos(-1.0), 0.0, m.data());
+        return m;
+    }();
+    return std::equal(h.begin(), h.end(), u);
+}
 
 void insert(uint64_t v, std::vector<uint64_t> &ech)
 {
@@ -61,6 +69,10 @@ bool AffBuild::init(int eb, int mm, const std::vector<U3Op> &gates, const std::v
     }
     form = 2;
     dev.scale = 1.0;
+    // What a matrix may miss its form by. complex128 takes exact forms and H only: a phase of
+    // 1e-15 dropped from every gate of a deep circuit adds up. In complex64 the amplitudes
+    // round at 6e-8, and products of H with rotations keep their form.
+    const double round = elem_bytes == 8 ? 1e-15 : 0.0;
     if (m < kAffBits || m > kAffMaxBits) return false;
     dev.m = uint32_t(m);
     Room room;
@@ -118,18 +130,20 @@ bool AffBuild::init(int eb, int mm, const std::vector<U3Op> &gates, const std::v
             w[2] = std::conj(g.u[1]);
             w[3] = std::conj(g.u[3]);
         }
+        if (is_h(g.u))
+            for (cd &x : w) x = x.real();
         for (int q = 0; q < 4; q++) {
             d.u[2 * q] = w[q].real();
             d.u[2 * q + 1] = w[q].imag();
-            if (std::fabs(w[q].imag()) > kRound) form = 0;
+            if (!(std::fabs(w[q].imag()) <= round)) form = 0;
         }
         d.sel = uint32_t(s);
         d.gen = gen ? (*gen)[i] : 0u;
         d.slot = slot ? (*slot)[i] : 0u;
         dev.gates |= 1u << at[i];
         const double c = w[0].real(), sn = w[2].real();
-        const bool rot = std::fabs(c - w[3].real()) <= kRound && std::fabs(sn + w[1].real()) <= kRound;
-        const bool refl = std::fabs(c + w[3].real()) <= kRound && std::fabs(sn - w[1].real()) <= kRound;
+        const bool rot = std::fabs(c - w[3].real()) <= round && std::fabs(sn + w[1].real()) <= round;
+        const bool refl = std::fabs(c + w[3].real()) <= round && std::fabs(sn - w[1].real()) <= round;
         // an X generator's gradient (RX by a multiple of 2 pi is real) takes the general form
         if (d.gen == 2 || !(rot || refl)) form = std::min(form, 1);
         const bool mu = std::fabs(c) < std::fabs(sn);
