@@ -1,0 +1,57 @@
+"""What the host side launches, without a GPU: the library's objects linked with a CUDA
+runtime that only logs (fake_cuda.cpp), the package run on it in a child process."""
+import os
+import subprocess
+import sys
+import textwrap
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parent.parent
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    objs = sorted((ROOT / "zxh_adae_b200" / "csrc" / "_build").glob("*.o"))
+    if not objs:
+        pytest.skip("no object files: the library was not built in this tree")
+    out = tmp_path_factory.mktemp("fake") / "libfake.so"
+    subprocess.run(["g++", "-shared", "-fPIC", "-O1", "-std=c++17", f"-I{CUDA}/include", "-Wl,-Bsymbolic", "-Wl,--no-undefined",
+                    "-o", str(out), str(ROOT / "tests" / "fake_cuda.cpp"), *map(str, objs)], check=True)
+    return out
+
+
+PRELUDE = """
+import ctypes, sys
+import numpy as np
+from zxh_adae_b200 import ZXH, workloads as wl, records as rc
+from zxh_adae_b200 import adjoint as ad
+from zxh_adae_b200.batch import Batch
+from zxh_adae_b200._core import _lib
+_lib.fake_take_log.restype = ctypes.c_char_p
+_lib.fake_fail_malloc.argtypes = [ctypes.c_long]
+def launches():  # (chained, grid, kernel) since the last call
+    out = [l.split(" ", 2) for l in _lib.fake_take_log().decode().splitlines()]
+    short = lambda k: k.replace("(anonymous namespace)::", "").replace("zxh::", "").replace("void ", "").split("(")[0]
+    return [(c == "1", int(g), short(k)) for c, g, k in out]
+"""
+
+
+def run(fake, body):
+    env = dict(os.environ, ZXH_B200_LIB=str(fake), PYTHONPATH=str(ROOT))
+    r = subprocess.run([sys.executable, "-c", PRELUDE + textwrap.dedent(body)], env=env, capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return r.stdout
+
+
+
+def test_batch_tasks_hold_whole_shares_of_a_cta(fake):
+    # 256 circuits of 11 qubits: 16 strided items an op (complex64) are one task of two
+    # rounds of the CTA's 8 warps, not 13 items and 3
+    run(fake, """
+    b = Batch([c[:3] for c in wl.batch_tfim(256, 5, 11, 11, 10)])
+    ops, tasks, _ = b.stats()
+    assert tasks == ops, (ops, tasks)
+    """)

@@ -269,8 +269,10 @@ void make_tasks(zxh_batch *b)
     b->rem_init.assign(b->ops.size(), 0);
     // Units of a task: the knob's, but no more than spread a level's work of that kind over two
     // tasks an SM (a level runs as long as its longest task: 16 circuits of 12 to 17 qubits
-    // took 3.1 ms in tasks of 8 tiles, 1.4 ms in tasks of 1 or 2), and at least what the
-    // warps of a CTA share. A tile is four strided items' amplitudes; a quarter of their task
+    // took 3.1 ms in tasks of 8 tiles, 1.4 ms in tasks of 1 or 2), in whole shares of the
+    // CTA's warps: of 13 strided items, five are a second round that leaves three warps idle,
+    // and the op's other three another task (256 circuits of 11 qubits, complex64: 0.66 ms, 0.60
+    // in whole shares). A tile is four strided items' amplitudes; a quarter of their task
     // measured best where the level is large.
     enum { ITEMS, TILES, ELEMS, KINDS };
     auto kind_of = [](const BatchOp &op) {
@@ -279,7 +281,7 @@ void make_tasks(zxh_batch *b)
     };
     const uint64_t knob[KINDS] = {uint64_t(b->task_items), uint64_t(std::max(1, b->task_items / 16)),
                                   uint64_t(b->task_elems)};
-    const uint64_t least[KINDS] = {8, 1, 2048};
+    const uint64_t share[KINDS] = {8, 1, 2048};
     for (size_t L = 0; L < levels; L++) {
         uint64_t units[KINDS] = {0, 0, 0};
         for (const auto &ch : b->chain)
@@ -289,7 +291,8 @@ void make_tasks(zxh_batch *b)
             const uint32_t oi = b->chain[c][L];
             const BatchOp &op = b->ops[oi];
             const int k = kind_of(op);
-            const uint64_t per = std::min(knob[k], std::max(least[k], units[k] / (2 * uint64_t(b->sms))));
+            const uint64_t even = units[k] / (2 * uint64_t(b->sms));
+            const uint64_t per = std::min(knob[k], std::max<uint64_t>(1, (even + share[k] - 1) / share[k]) * share[k]);
             for (uint64_t s = 0; s < op.units; s += per) {
                 BatchTask t;
                 t.op = oi;
