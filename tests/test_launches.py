@@ -55,3 +55,22 @@ def test_batch_tasks_hold_whole_shares_of_a_cta(fake):
     ops, tasks, _ = b.stats()
     assert tasks == ops, (ops, tasks)
     """)
+
+
+def test_batch_kernel_without_tiles(fake):
+    # circuits below 12 qubits have no tile passes: their queue runs the form of the kernel
+    # that leaves room for two CTAs an SM, but where there is one task an SM in complex128
+    run(fake, """
+    def form(cnt, n, dtype, threads=256):
+        b = Batch([c[:3] for c in wl.batch_tfim(cnt, 5, n, n, 4)], dtype=dtype)
+        b.set("threads", threads)
+        launches(); b.run("persistent")
+        (k,) = [k for _, _, k in launches() if "batch_kernel" in k]
+        return k
+    for dtype, e in (("complex64", "float2"), ("complex128", "double2")):
+        assert form(512, 7, dtype) == f"batch_kernel<{e}, true, 256, false>"
+        assert form(4, 7, dtype) == f"batch_kernel<{e}, true, 256, {'true' if e == 'double2' else 'false'}>"
+        assert form(2, 12, dtype) == f"batch_kernel<{e}, true, 256, true>"
+        for t in (64, 128):
+            assert form(2, 12, dtype, t) == f"batch_kernel<{e}, true, {t}, false>"
+    """)

@@ -130,7 +130,7 @@ __device__ __forceinline__ void diag_adj_body(E *psi, E *lam, uint64_t b, uint64
     }
 }
 
-template <typename E, bool REAL, int NT>
+template <typename E, bool REAL, int NT, bool TILES>
 __device__ __forceinline__ void run_op_slice(const BatchOp &op, const uint8_t *blob, E *arena, double *grads,
                                              double *energies, uint64_t b, uint64_t e, uint64_t first, uint64_t step,
                                              BatchShared<E, NT> &sm, unsigned char *tile)
@@ -139,7 +139,7 @@ __device__ __forceinline__ void run_op_slice(const BatchOp &op, const uint8_t *b
     E *psi = arena + op.psi;
     E *lam = arena + op.lam;
     double *gr = grads + op.grad_base;
-    if constexpr (NT == kThreads) {  // tile: dynamic shared memory of the affine passes
+    if constexpr (TILES) {  // tile: dynamic shared memory of the affine passes
         // real queues: rotations, or any real gates
         if (op.kind == BOP_AFFINE) {
             auto &as = *reinterpret_cast<adev::AffSmem<E, false> *>(tile);
@@ -196,10 +196,13 @@ __device__ __forceinline__ void run_op_slice(const BatchOp &op, const uint8_t *b
 }
 
 // NT threads per CTA, 512 / NT resident CTAs per SM at 128 registers: 16 warps per SM
-// whatever NT is. The 256-thread complex128 form runs affine passes whose two states fill
-// an SM's shared memory: one CTA per SM, at twice the registers.
-template <typename E, bool REAL, int NT>
-__global__ void __launch_bounds__(NT, NT == kThreads && sizeof(E) == 16 ? 1 : 512 / NT) batch_kernel(const uint8_t *__restrict__ blob,
+// whatever NT is. TILES: the queue holds affine tile passes (NT = 256). Their two complex128
+// states fill an SM's shared memory, one CTA per SM at twice the registers; a queue without
+// them (circuits below 12 qubits) keeps two where it has tasks for both: 256 circuits of 11
+// qubits 0.88 -> 0.59 ms, 512 of 6 to 8 qubits 0.82 -> 0.45. In complex64 the form without
+// tiles spills less: 32 circuits of 11 qubits 0.520 -> 0.498 ms.
+template <typename E, bool REAL, int NT, bool TILES>
+__global__ void __launch_bounds__(NT, TILES && sizeof(E) == 16 ? 1 : 512 / NT) batch_kernel(const uint8_t *__restrict__ blob,
                                                              const BatchOp *__restrict__ ops,
                                                              const BatchTask *__restrict__ tasks, uint32_t ntasks,
                                                              uint32_t *next, uint32_t *remaining, E *arena,
@@ -235,7 +238,7 @@ __global__ void __launch_bounds__(NT, NT == kThreads && sizeof(E) == 16 ? 1 : 51
         __syncthreads();
         if (s_abort) break;
         const bool grow = op.kind == BOP_GROW || op.kind == BOP_GROW_ADJ;
-        run_op_slice<E, REAL, NT>(op, blob, arena, grads, energies, task.begin, task.end, grow ? task.begin : 0,
+        run_op_slice<E, REAL, NT, TILES>(op, blob, arena, grads, energies, task.begin, task.end, grow ? task.begin : 0,
                                   grow ? uint64_t(NT / 32) : 0, sm, s_raw);
         __threadfence();
         __syncthreads();
@@ -243,51 +246,55 @@ __global__ void __launch_bounds__(NT, NT == kThreads && sizeof(E) == 16 ? 1 : 51
     }
 }
 
-template <typename E, bool REAL, int NT>
+template <typename E, bool REAL, int NT, bool TILES>
 cudaError_t persistent_typed(const uint8_t *blob, const BatchOp *ops, const BatchTask *tasks, uint32_t ntasks,
                              uint32_t *next, uint32_t *remaining, E *arena, double *grads, double *energies,
                              DevStatus *status, long long spin_limit, int sms, cudaStream_t st)
 {
     int per_sm = 1;
     size_t smem = sizeof(BatchShared<E, NT>);
-    if (NT == kThreads) smem = std::max(smem, std::max(sizeof(adev::AffSmem<E, true>), sizeof(adev::AffSmem<E, false>)));
-    const cudaError_t e = cudaFuncSetAttribute(batch_kernel<E, REAL, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (TILES) smem = std::max(smem, std::max(sizeof(adev::AffSmem<E, true>), sizeof(adev::AffSmem<E, false>)));
+    const cudaError_t e = cudaFuncSetAttribute(batch_kernel<E, REAL, NT, TILES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                int(smem));
     if (e != cudaSuccess) return e;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel<E, REAL, NT>, NT, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel<E, REAL, NT, TILES>, NT, smem);
     if (per_sm < 1) per_sm = 1;
-    batch_kernel<E, REAL, NT><<<unsigned(sms * per_sm), NT, smem, st>>>(blob, ops, tasks, ntasks, next, remaining, arena,
+    batch_kernel<E, REAL, NT, TILES><<<unsigned(sms * per_sm), NT, smem, st>>>(blob, ops, tasks, ntasks, next, remaining, arena,
                                                                      grads, energies, status, spin_limit);
     return cudaGetLastError();
 }
 
 template <typename E, bool REAL>
-cudaError_t persistent_threads(int threads, const uint8_t *blob, const BatchOp *ops, const BatchTask *tasks,
+cudaError_t persistent_threads(int threads, bool wide, const uint8_t *blob, const BatchOp *ops, const BatchTask *tasks,
                                uint32_t ntasks, uint32_t *next, uint32_t *remaining, E *arena, double *grads,
                                double *energies, DevStatus *status, long long spin_limit, int sms, cudaStream_t st)
 {
+    if (wide)
+        return threads != kThreads ? cudaErrorInvalidValue
+                                   : persistent_typed<E, REAL, kThreads, true>(blob, ops, tasks, ntasks, next, remaining, arena,
+                                                                               grads, energies, status, spin_limit, sms, st);
     switch (threads) {
     case 64:
-        return persistent_typed<E, REAL, 64>(blob, ops, tasks, ntasks, next, remaining, arena, grads, energies,
+        return persistent_typed<E, REAL, 64, false>(blob, ops, tasks, ntasks, next, remaining, arena, grads, energies,
                                              status, spin_limit, sms, st);
     case 128:
-        return persistent_typed<E, REAL, 128>(blob, ops, tasks, ntasks, next, remaining, arena, grads, energies,
+        return persistent_typed<E, REAL, 128, false>(blob, ops, tasks, ntasks, next, remaining, arena, grads, energies,
                                               status, spin_limit, sms, st);
     case 256:
-        return persistent_typed<E, REAL, 256>(blob, ops, tasks, ntasks, next, remaining, arena, grads, energies,
+        return persistent_typed<E, REAL, 256, false>(blob, ops, tasks, ntasks, next, remaining, arena, grads, energies,
                                               status, spin_limit, sms, st);
     default: return cudaErrorInvalidValue;
     }
 }
 
 template <typename E>
-cudaError_t persistent_real(bool real, int threads, const uint8_t *blob, const BatchOp *ops, const BatchTask *tasks,
+cudaError_t persistent_real(bool real, int threads, bool wide, const uint8_t *blob, const BatchOp *ops, const BatchTask *tasks,
                             uint32_t ntasks, uint32_t *next, uint32_t *remaining, E *arena, double *grads,
                             double *energies, DevStatus *status, long long spin_limit, int sms, cudaStream_t st)
 {
-    return real ? persistent_threads<E, true>(threads, blob, ops, tasks, ntasks, next, remaining, arena, grads,
+    return real ? persistent_threads<E, true>(threads, wide, blob, ops, tasks, ntasks, next, remaining, arena, grads,
                                               energies, status, spin_limit, sms, st)
-                : persistent_threads<E, false>(threads, blob, ops, tasks, ntasks, next, remaining, arena, grads,
+                : persistent_threads<E, false>(threads, wide, blob, ops, tasks, ntasks, next, remaining, arena, grads,
                                                energies, status, spin_limit, sms, st);
 }
 
@@ -295,14 +302,14 @@ cudaError_t persistent_real(bool real, int threads, const uint8_t *blob, const B
 
 cudaError_t run_batch_persistent(const uint8_t *blob, const BatchOp *ops, const BatchTask *tasks, uint32_t ntasks,
                                  uint32_t *next, uint32_t *remaining, void *arena, double *grads, double *energies,
-                                 DevStatus *status, int elem_bytes, bool real, int threads, int wait_limit_log2,
+                                 DevStatus *status, int elem_bytes, bool real, int threads, bool wide, int wait_limit_log2,
                                  int sms, cudaStream_t st)
 {
     const long long spin_limit = 1LL << wait_limit_log2;
     if (elem_bytes == 8)
-        return persistent_real(real, threads, blob, ops, tasks, ntasks, next, remaining, static_cast<float2 *>(arena),
+        return persistent_real(real, threads, wide, blob, ops, tasks, ntasks, next, remaining, static_cast<float2 *>(arena),
                                grads, energies, status, spin_limit, sms, st);
-    return persistent_real(real, threads, blob, ops, tasks, ntasks, next, remaining, static_cast<double2 *>(arena),
+    return persistent_real(real, threads, wide, blob, ops, tasks, ntasks, next, remaining, static_cast<double2 *>(arena),
                            grads, energies, status, spin_limit, sms, st);
 }
 

@@ -46,12 +46,13 @@ struct BatchTask {
 // Runs every task of the queue; counters: `next` (queue head, zeroed) and
 // `remaining[op]` (tasks of each op, preset). grid = resident CTAs. real: every
 // strided op of the queue has real gates (the kernel's real-gate form). threads:
-// 64, 128 or 256 per CTA (the warps that work on one task). A task waits at most
+// 64, 128 or 256 per CTA (the warps that work on one task). wide: the form with
+// affine tile passes (256 threads only), for queues that hold some. A task waits at most
 // 2^wait_limit_log2 SM clocks for its op's predecessor; then it records a timeout
 // in the status word and its CTA ends.
 cudaError_t run_batch_persistent(const uint8_t *blob, const BatchOp *ops, const BatchTask *tasks, uint32_t ntasks,
                                  uint32_t *next, uint32_t *remaining, void *arena, double *grads, double *energies,
-                                 DevStatus *status, int elem_bytes, bool real, int threads, int wait_limit_log2,
+                                 DevStatus *status, int elem_bytes, bool real, int threads, bool wide, int wait_limit_log2,
                                  int sms, cudaStream_t st);
 
 }  // namespace zxh

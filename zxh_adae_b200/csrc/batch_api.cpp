@@ -66,6 +66,8 @@ struct zxh_batch {
     int wait_limit_log2 = 31;  // a task's wait for its predecessor: 2^31 SM clocks (about a second)
     uint64_t bytes = 0;  // algorithmic state bytes of one run
     bool real = false;   // every strided op has real gates: the persistent kernel's real-gate form
+    bool tiles = false;  // some op is an affine tile pass
+    bool wide = false;   // the persistent kernel's form with tiles (batch.h)
     float last_ms = 0.0f;
 };
 
@@ -257,6 +259,13 @@ int compile(zxh_batch *b)
             push(op);
         }
     }
+    b->real = true;
+    b->tiles = false;
+    for (const BatchOp &op : b->ops) {
+        const bool tile = op.kind == zxh::BOP_AFFINE || op.kind == zxh::BOP_AFFINE_ADJ;
+        if ((op.kind == zxh::BOP_GROW || op.kind == zxh::BOP_GROW_ADJ || tile) && !op.aux) b->real = false;
+        b->tiles = b->tiles || tile;
+    }
     return ZXH_OK;
 }
 
@@ -304,6 +313,11 @@ void make_tasks(zxh_batch *b)
             }
         }
     }
+    // Without tile passes that form still serves complex128 queues that leave the SMs one task
+    // each: one CTA at twice the registers finishes it sooner (32 circuits of 11 qubits 0.46
+    // against 0.49 ms; 128 of 10 qubits, 163 tasks a level, 0.45 against 0.42).
+    const bool one_each = b->tasks.size() <= levels * size_t(b->sms);
+    b->wide = b->tiles || (b->eb == 16 && b->threads == 256 && one_each);
 }
 
 int upload(zxh_batch *b)
@@ -354,7 +368,7 @@ int enqueue_persistent(zxh_batch *b)
         "reset counters");
     BCK(b, zxh::run_batch_persistent(b->d_blob, b->d_ops, b->d_tasks, uint32_t(b->tasks.size()), b->d_next, b->d_rem,
                                      b->d_arena, b->d_grads, b->d_energy, b->d_status, b->eb, b->real,
-                                     b->threads, b->wait_limit_log2, b->sms, b->stream),
+                                     b->threads, b->wide, b->wait_limit_log2, b->sms, b->stream),
         "batch launch");
     return ZXH_OK;
 }
@@ -409,10 +423,6 @@ int launch_op(zxh_batch *b, const BatchOp &op)
 int build(zxh_batch *b)
 {
     if (int rc = compile(b)) return rc;
-    b->real = true;
-    for (const BatchOp &op : b->ops)
-        if ((op.kind == zxh::BOP_GROW || op.kind == zxh::BOP_GROW_ADJ || op.kind == zxh::BOP_AFFINE ||
-             op.kind == zxh::BOP_AFFINE_ADJ) && !op.aux) b->real = false;
     make_tasks(b);
     return upload(b);
 }
