@@ -298,7 +298,10 @@ int zxh_batch_run(zxh_batch *batch, int mode, double *energies, double *grads, s
  * wait_limit_log2 (0..31, default 31): a persistent task waits at most
  * 2^wait_limit_log2 SM clocks for the previous pass of its circuit, then the run
  * ends early and zxh_batch_run returns ZXH_ERR_TIMEOUT; the handle stays usable
- * (the next run starts from scratch). Small values exist to test that path. */
+ * (the next run starts from scratch). Small values exist to test that path.
+ * A setting whose program cannot be compiled or placed on the device is taken back;
+ * zxh_batch_run returns ZXH_ERR_STATE if the program of the old one could not be
+ * placed again either (until a setting succeeds). */
 int zxh_batch_set(zxh_batch *batch, const char *name, int value);
 int zxh_batch_get(const zxh_batch *batch, const char *name, int *value);
 /* Times the persistent launch (reps timed runs per setting after one warm-up)

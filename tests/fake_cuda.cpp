@@ -1,7 +1,7 @@
 // fake_cuda.cpp -- a CUDA runtime without a GPU for tests of the host side: linked with
 // the library's objects in place of the static runtime (fakecuda.py). Device memory is
 // addresses only, copies and memsets move nothing, launches are written to a log by
-// kernel name, and a test can make an allocation fail.
+// kernel name, and a test can make allocations fail.
 #include <cuda_runtime.h>
 #include <cxxabi.h>
 
@@ -20,7 +20,7 @@ std::map<const void *, std::string> &names()
 }
 
 std::string g_log;
-long g_fail_in = -1;  // cudaMalloc calls until one fails, < 0: none
+long g_fail = 0;  // cudaMalloc calls that fail from now on
 uintptr_t g_next = uintptr_t(1) << 40;
 struct Config { dim3 grid, block; size_t smem; cudaStream_t st; } g_config;
 
@@ -44,7 +44,7 @@ const char *fake_take_log()
     g_log.clear();
     return out.c_str();
 }
-void fake_fail_malloc(long in) { g_fail_in = in; }
+void fake_fail_malloc(long calls) { g_fail = calls; }
 
 void **__cudaRegisterFatBinary(void *) { static void *h; return &h; }
 void __cudaRegisterFatBinaryEnd(void **) {}
@@ -84,7 +84,7 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void
 cudaError_t cudaMalloc(void **p, size_t n)
 {
     *p = nullptr;
-    if (g_fail_in >= 0 && g_fail_in-- == 0) return cudaErrorMemoryAllocation;
+    if (g_fail > 0 && g_fail--) return cudaErrorMemoryAllocation;
     *p = reinterpret_cast<void *>(g_next);
     g_next += (n + 511) & ~size_t(511);
     return cudaSuccess;

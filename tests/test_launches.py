@@ -74,3 +74,31 @@ def test_batch_kernel_without_tiles(fake):
         for t in (64, 128):
             assert form(2, 12, dtype, t) == f"batch_kernel<{e}, true, {t}, false>"
     """)
+
+
+def test_batch_after_a_failed_rebuild(fake):
+    # another thread count is another pass set: where it cannot be placed, the handle goes
+    # back to the one it had, or, where that fails too, refuses to run
+    run(fake, """
+    b = Batch([c[:3] for c in wl.batch_tfim(2, 5, 12, 12, 4)])
+    before = b.stats()[:2]
+    for failures in (1, 100):
+        _lib.fake_fail_malloc(failures)
+        try:
+            b.set("threads", 64)
+            raise SystemExit("the rebuild did not fail")
+        except MemoryError:
+            pass
+        assert b.get("threads") == 256
+        launches()
+        try:
+            b.run("persistent")
+            ran = True
+        except RuntimeError:
+            ran = False
+        assert ran == (failures == 1) and ran == any("batch_kernel" in k for _, _, k in launches())
+        assert not ran or b.stats()[:2] == before
+    _lib.fake_fail_malloc(0)
+    b.set("threads", 256)  # a later setting builds the program again
+    b.run("persistent")
+    """)

@@ -68,6 +68,7 @@ struct zxh_batch {
     bool real = false;   // every strided op has real gates: the persistent kernel's real-gate form
     bool tiles = false;  // some op is an affine tile pass
     bool wide = false;   // the persistent kernel's form with tiles (batch.h)
+    bool ready = false;  // the device holds the program of the settings: false after a failed rebuild
     float last_ms = 0.0f;
 };
 
@@ -125,6 +126,7 @@ uint64_t append(std::vector<uint8_t> &blob, const void *p, size_t n)
 // Host compile of every circuit into ops, tasks and one descriptor blob.
 int compile(zxh_batch *b)
 {
+    b->ready = false;
     b->ops.clear();
     b->rem_init.clear();
     b->blob.clear();
@@ -323,6 +325,7 @@ void make_tasks(zxh_batch *b)
 int upload(zxh_batch *b)
 {
     drop_graph(b);
+    b->ready = false;
     const size_t ngr = b->grad_off.back();
     if (int rc = grow_dev(b, reinterpret_cast<void **>(&b->d_blob), b->cap_blob, b->blob.size(), "cudaMalloc(batch blob)"))
         return rc;
@@ -353,6 +356,7 @@ int upload(zxh_batch *b)
                            cudaMemcpyHostToDevice, b->stream),
         "upload counters");
     BCK(b, cudaStreamSynchronize(b->stream), "upload");
+    b->ready = true;
     return ZXH_OK;
 }
 
@@ -525,6 +529,7 @@ int zxh_batch_run(zxh_batch *b, int mode, double *energies, double *grads, size_
     if ((ngr && !grads) || !energies) return bfail(b, ZXH_ERR_ARG, "output is null");
     if (ngrads < ngr) return bfail(b, ZXH_ERR_ARG, "grads holds fewer entries than the batch's recorded gates");
     if (mode < ZXH_BATCH_SEQUENTIAL || mode > ZXH_BATCH_GRAPH) return bfail(b, ZXH_ERR_ARG, "unknown batch mode");
+    if (!b->ready) return bfail(b, ZXH_ERR_STATE, "the batch has no program: its last rebuild failed");
     BCK(b, cudaSetDevice(b->device), "cudaSetDevice");
     if (mode == ZXH_BATCH_GRAPH && !b->gexec) {
         BCK(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
@@ -585,15 +590,24 @@ int zxh_batch_set(zxh_batch *b, const char *name, int value)
                                          (field == &b->threads ? " and one of 64, 128, 256" : ""));
     // only 256-thread CTAs run affine tile passes: another pass set on either side
     const bool other_passes = field == &b->threads && (b->threads == 256) != (value == 256);
-    *field = value;
     BCK(b, cudaSetDevice(b->device), "cudaSetDevice");
-    if (field == &b->wait_limit_log2 || (field == &b->threads && !other_passes)) {
+    const int old = *field;
+    *field = value;
+    if (b->ready && (field == &b->wait_limit_log2 || (field == &b->threads && !other_passes))) {
         // launch parameters: only the captured graph holds the old value
         BCK(b, cudaStreamSynchronize(b->stream), "sync");
         drop_graph(b);
         return ZXH_OK;
     }
-    return (field == &b->grow_regs || field == &b->adj_regs || other_passes) ? build(b) : retask(b);
+    const bool passes = field == &b->grow_regs || field == &b->adj_regs || other_passes;
+    const int rc = passes || !b->ready ? build(b) : retask(b);
+    if (rc) {  // back to the setting the handle had, with its program if that can still be placed
+        const std::string msg = b->err;
+        *field = old;
+        build(b);
+        b->err = msg;
+    }
+    return rc;
 }
 
 int zxh_batch_get(const zxh_batch *b, const char *name, int *value)
