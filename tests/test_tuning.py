@@ -30,3 +30,14 @@ def test_cache_round_trip_and_bad_files(tmp_path):
     path.write_text(json.dumps({"x": {"grow_regs": 3}}))  # missing knobs: not used
     assert TuneCache(path).get("x") is None
     assert set(KNOBS) == set(s)
+
+
+def test_settings_timed_on_other_passes_are_not_used(tmp_path):
+    # 64 threads were a choice of task size once; now they give up the tile passes
+    path = tmp_path / "tune.json"
+    s = {"grow_regs": 3, "adj_regs": 2, "task_items": 512, "task_elems": 524288, "threads": 64}
+    path.write_text(json.dumps({"old": s, "other": {**s, "pass_set": 1}}))
+    c = TuneCache(path)
+    assert c.get("old") is None and c.get("other") is None
+    c.put("old", s)
+    assert c.get("old") == s

@@ -4,8 +4,9 @@
 ``TuneCache`` keeps the winning settings on disk so later batches of the same
 shape on the same GPU model start from them without re-timing. A key is
 (dtype, the circuits' qubit-count range, the number of circuits rounded up to a
-power of two, GPU name, SM count); the value is the knob settings. The file is
-JSON, written atomically (a temporary file renamed over it).
+power of two, GPU name, SM count); the value is the knob settings and the pass set they
+were timed on. The file is JSON, written atomically (a temporary file renamed
+over it).
 
 Pure Python: importing this module loads no native code.
 """
@@ -17,6 +18,10 @@ import tempfile
 from pathlib import Path
 
 KNOBS = ("grow_regs", "adj_regs", "task_items", "task_elems", "threads")
+# The passes a setting chooses between: raised whenever these change, so that settings
+# timed on others are timed again. 2: only 256 threads run affine tile passes, and
+# task_items is an upper limit.
+PASS_SET = 2
 
 
 def batch_key(nqubits, dtype: str, gpu_name: str, sms: int) -> str:
@@ -46,13 +51,13 @@ class TuneCache:
 
     def get(self, key: str):
         v = self.load().get(key)
-        if not isinstance(v, dict) or any(k not in v for k in KNOBS):
+        if not isinstance(v, dict) or any(k not in v for k in KNOBS) or v.get("pass_set") != PASS_SET:
             return None
         return {k: int(v[k]) for k in KNOBS}
 
     def put(self, key: str, settings: dict) -> None:
         data = self.load()
-        data[key] = {k: int(settings[k]) for k in KNOBS}
+        data[key] = {**{k: int(settings[k]) for k in KNOBS}, "pass_set": PASS_SET}
         self.path.parent.mkdir(parents=True, exist_ok=True)
         fd, tmp = tempfile.mkstemp(dir=str(self.path.parent), prefix=self.path.name, suffix=".tmp")
         try:
