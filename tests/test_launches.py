@@ -102,3 +102,23 @@ def test_batch_after_a_failed_rebuild(fake):
     b.set("threads", 256)  # a later setting builds the program again
     b.run("persistent")
     """)
+
+
+def test_chained_kernels_take_states_without_restrict():
+    # a kernel that may start before its predecessor has ended must not promise that nobody
+    # else writes its state: loads through such a pointer may move above the wait. Tables that
+    # were uploaded before the run, the state a draw only reads, and outputs may be __restrict__
+    import re
+
+    seen = 0
+    for src in sorted((ROOT / "zxh_adae_b200" / "csrc").glob("*.cu")):
+        for m in re.finditer(r"__global__[^;{]*?(\w+)\(((?:const uint8_t|const E|const uint64_t|const double|E )[^{;]*)\)\s*\{", src.read_text()):
+            name, params, body = m[1], m[2], src.read_text()[m.end():]
+            body = body[: body.index("\n}\n")]
+            if "chain_wait()" not in body and "affine_body" not in body:
+                continue
+            seen += 1
+            held = set(re.findall(r"__restrict__ (\w+)", params))
+            assert held <= {"blob", "terms", "counts", "offsets", "real_out", "words"} | (
+                {"state"} if src.name == "sampler.cu" else set()), (src.name, name, held)
+    assert seen >= 8

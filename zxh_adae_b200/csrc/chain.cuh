@@ -6,10 +6,11 @@
 // therefore run before its predecessor has ended, and touches nothing that earlier work
 // writes until chain_wait() returns: that waits for the predecessor's end, and its writes
 // are visible then. What a kernel reads before it (its tables in the program blob, kernel
-// parameters) was uploaded before the first kernel of the run; what the predecessor wrote is
-// read through pointers that are not const __restrict__, whose loads may move above the wait. On states whose passes last
-// as long as their setup (10 to 16 us a pass up to 20 qubits) the setup and the launch
-// latency of a pass then overlap the pass before it.
+// parameters) was uploaded before the first kernel of the run. What the predecessor wrote is
+// read through pointers that are not __restrict__: of those the compiler may take it that
+// nothing else writes there, the wait's memory clobber included, and move their loads above it.
+// On states whose passes last as long as their setup (10 to 16 us a pass up to 20 qubits) the
+// setup and the launch latency of a pass then overlap the pass before it.
 #pragma once
 
 #include <cuda_runtime.h>

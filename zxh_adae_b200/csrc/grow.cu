@@ -45,8 +45,8 @@ using namespace gdev;
 // staged form (next item's rows copied into shared memory during the current one).
 template <typename E, int R, bool ADJ, bool REAL, bool PF>
 __global__ void __launch_bounds__(kThreads, (ADJ && R == 4) ? 1 : 2)
-    grow_kernel(const uint8_t *__restrict__ blob, uint64_t poff, uint64_t toff, E *__restrict__ psi,
-                E *__restrict__ lam, double *grads, uint64_t nitems, DevStatus *status, const E *psi_src)
+    grow_kernel(const uint8_t *__restrict__ blob, uint64_t poff, uint64_t toff, E *psi, E *lam,
+                double *grads, uint64_t nitems, DevStatus *status, const E *psi_src)
 {
     __shared__ GrowShared<E> sm;
     extern __shared__ __align__(128) uint8_t stage[];

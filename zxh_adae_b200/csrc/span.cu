@@ -739,7 +739,7 @@ struct SpanConst {
 // copies of the CTA's next tile into the landing slab, and work on this one.
 template <class G, bool LOW, bool THREE, int WIN>
 __global__ void __launch_bounds__(kSpanThreads, 2)
-    span_land_kernel(const uint8_t *__restrict__ blob, uint64_t soff, uint64_t toff, typename G::E *__restrict__ state,
+    span_land_kernel(const uint8_t *__restrict__ blob, uint64_t soff, uint64_t toff, typename G::E *state,
                      const __grid_constant__ SpanConst<typename G::E> kc)
 {
     using E = typename G::E;

@@ -682,7 +682,7 @@ __device__ __forceinline__ void lane_row_transpose(VT (&x)[NR], void *tbv, int l
 // with one read and one write of every amplitude.
 template <typename E, int W, bool XP, bool REAL, bool WIN>
 __global__ void __launch_bounds__(kThreads, 2) row_pass_kernel(const uint8_t *__restrict__ blob, uint64_t poff,
-                                                            uint64_t toff, E *__restrict__ state)
+                                                            uint64_t toff, E *state)
 {
     using VT = typename RowCfg<E, W>::VT;
     using RT = typename ET<E>::R;
