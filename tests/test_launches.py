@@ -122,3 +122,24 @@ def test_chained_kernels_take_states_without_restrict():
             assert held <= {"blob", "terms", "counts", "offsets", "real_out", "words"} | (
                 {"state"} if src.name == "sampler.cu" else set()), (src.name, name, held)
     assert seen >= 8
+
+
+@pytest.mark.parametrize("n,chained", [(20, True), (21, False), (28, False)])
+def test_passes_behind_a_span_pass(fake, n, chained):
+    # CX from every other qubit to the last: the RY layer is span passes, then affine tile passes
+    # (strided ones with affine = 0); the first of these starts before the span pass has ended
+    # on small states only, the others always
+    run(fake, f"""
+    n = {n}
+    g = np.concatenate([wl.h_all(n), rc.as_records([(rc.CX, q, n - 1) for q in range(0, n - 1, 2)]),
+                        rc.as_records([(rc.U3, 0, q, 0.3 + q, 0.0, 0.0) for q in range(n)])])
+    for affine, kind in ((1, "affine_kernel"), (0, "grow_kernel")):
+        s = ZXH(n)
+        s.set_param("affine", affine)
+        s.push_gates(g)
+        launches(); s.execute()
+        ks = launches()
+        behind = [i for i in range(1, len(ks)) if ks[i][2].startswith(kind) and "span_land" in ks[i - 1][2]]
+        assert len(behind) == 1, ks
+        assert [c for c, _, _ in ks[1:]] == [i not in behind or {chained} for i in range(1, len(ks))], ks
+    """)

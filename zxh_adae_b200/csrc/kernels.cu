@@ -502,7 +502,12 @@ cudaError_t run_passes(const std::vector<Pass> &passes, const uint8_t *dblob, vo
         cudaError_t e = cudaSuccess;
         // Chained below 32 qubits: 16 q complex64 (20 U3 + cz layers) 0.43 -> 0.26 ms, 24 q 3.67 -> 3.46,
         // 30 q equal within 0.2 %; at 32 q complex64 chained passes take 1051 ms and unchained ones 931.
-        const bool chained = i > 0 && ps.m < 32;
+        // Not chained from 21 qubits up: an affine tile or strided pass behind a span pass, whose
+        // waiting CTAs cost the batch 2 to 5 % (tiles) or 5 to 9 % (strided) at every size measured,
+        // 22 to 28 q: the CX fan-in circuit at 28 q complex128 7.62 ms chained, 7.32 not. At 20 q
+        // complex128 chaining them gains 2 to 7 %.
+        const bool behind_span = i > 0 && passes[i - 1].kind == Pass::SPAN && ps.kind != Pass::SPAN && ps.m > 20;
+        const bool chained = i > 0 && ps.m < 32 && !behind_span;
         if (ps.kind == Pass::PRODUCT) {
             const uint64_t nvec = std::max<uint64_t>(1, (1ULL << ps.m) / (16 / elem_bytes));
             const unsigned grid = unsigned(std::max<uint64_t>(1, std::min<uint64_t>((nvec + kThreads - 1) / kThreads,
