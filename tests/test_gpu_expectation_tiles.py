@@ -58,3 +58,21 @@ def test_expectation_tiles(n, kind, which, dtype):
     scale = max(1.0, float(np.sum(np.abs(terms["coef"]))))
     assert abs(s.expectation(terms) - ob.oracle_energy(n, gates, terms)) <= TOL[dtype] * scale
     s.close()
+
+
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+@pytest.mark.parametrize("n", [12, 18, 19])
+def test_expectation_of_few_terms(n, dtype):
+    # both sides of the lines between one gather per X term and tiles: Z terms alone, one, two
+    # and three X terms, up to and above the counts that take the gathers
+    gates = circuit(n, "chain", n)
+    rng = np.random.default_rng(n)
+    s = ZXH(n, dtype=dtype)
+    s.push_gates(gates)
+    s.execute()
+    for nx, nd in [(0, 1), (0, 4), (0, 5), (0, 12), (0, 13), (0, 33), (1, 0), (1, 8), (1, 9), (1, 33), (2, 12), (2, 13), (3, 0)]:
+        terms = as_terms([(TERM_X, int(q), 0, 0.4) for q in rng.permutation(n)[:nx]] +
+                         [(TERM_ZZ, int(a), int(b), 0.3) for a, b in rng.integers(0, n, (nd, 2))])
+        scale = max(1.0, float(np.sum(np.abs(terms["coef"]))))
+        assert abs(s.expectation(terms) - ob.oracle_energy(n, gates, terms)) <= TOL[dtype] * scale, (nx, nd)
+    s.close()

@@ -143,3 +143,21 @@ def test_passes_behind_a_span_pass(fake, n, chained):
         assert len(behind) == 1, ks
         assert [c for c, _, _ in ks[1:]] == [i not in behind or {chained} for i in range(1, len(ks))], ks
     """)
+
+
+def test_few_terms_take_the_gathers(fake):
+    # expectations of a few terms: one kernel that gathers; tiles where these are the faster
+    run(fake, """
+    def kernels(n, dtype, nx, nd):
+        s = ZXH(n, dtype=dtype)
+        s.push_gates(wl.h_all(n)); s.execute(); launches()
+        s.expectation(rc.as_terms([(rc.TERM_X, q, 0, 1.0) for q in range(nx)] + [(rc.TERM_ZZ, i % n, (i + 3) % n, 1.0) for i in range(nd)]))
+        return {k.split("<")[0] for _, _, k in launches()}
+    gather, tile = {"lambda_kernel"}, {"lambda_tile_kernel"}
+    for dtype, most in (("complex64", 4), ("complex128", 12)):
+        assert kernels(24, dtype, 0, 1) == kernels(28, dtype, 0, most) == gather
+        assert kernels(24, dtype, 0, most + 1) == kernels(24, dtype, 1, 0) == tile
+        assert kernels(16, dtype, 2, 12) == kernels(18, dtype, 0, 32) == gather
+        assert kernels(16, dtype, 16, 15) == kernels(18, dtype, 3, 0) == tile
+    assert kernels(22, "complex128", 1, 4) == gather and kernels(22, "complex64", 1, 4) == tile
+    """)

@@ -59,9 +59,9 @@ struct LamPassDev {
     double xc[12];
     uint32_t xmask, nd, diag0, goff[17];
 };
-// Passes for H over 2^m amplitudes, none below 2^12 (run_lambda then). Reorders the Z and
-// ZZ terms; call it before the terms are uploaded.
-std::vector<LamPassDev> plan_lambda(std::vector<TermDev> &terms, int m);
+// Passes for H over 2^m amplitudes; none below 2^12 and for few terms (run_lambda then).
+// Reorders the Z and ZZ terms; call it before the terms are uploaded.
+std::vector<LamPassDev> plan_lambda(std::vector<TermDev> &terms, int m, int elem_bytes);
 // run_lambda by the planned passes.
 cudaError_t run_lambda_tiles(const void *psi, void *lam, int elem_bytes, const std::vector<LamPassDev> &passes,
                              const TermDev *dterms, double *energy, int sms, cudaStream_t st);

@@ -505,7 +505,7 @@ int zxh_expectation(zxh_sim *s, const zxh_term *terms, size_t nterms, double *va
     if (int rc = flush_pending(s)) return rc;
     std::vector<TermDev> dt;
     if (int rc = compile_terms(s, terms, nterms, s->ws.map, s->ws.m, true, dt)) return rc;
-    const std::vector<zxh::LamPassDev> hpasses = zxh::plan_lambda(dt, s->ws.m);
+    const std::vector<zxh::LamPassDev> hpasses = zxh::plan_lambda(dt, s->ws.m, s->elem_bytes);
     const AdjLayout L(0, dt.size());
     if (int rc = ensure_dev(s, reinterpret_cast<void **>(&s->d_adj), s->adj_cap, L.total, "cudaMalloc(adjoint)"))
         return rc;
@@ -569,7 +569,7 @@ int zxh_adjoint_gradient(zxh_sim *s, const zxh_term *terms, size_t nterms, size_
     AffineMap A = s->ws.map;
     std::vector<TermDev> dt;
     if (int rc = compile_terms(s, terms, nterms, A, N, false, dt)) return rc;
-    const std::vector<zxh::LamPassDev> hpasses = zxh::plan_lambda(dt, N);
+    const std::vector<zxh::LamPassDev> hpasses = zxh::plan_lambda(dt, N, s->elem_bytes);
     std::vector<RevStep> steps;
     std::vector<AdjDiagGate> dgates;
     std::vector<uint32_t> dslots;

@@ -1,5 +1,5 @@
 // lambda_tile.cu -- lambda = H psi and <psi|H|psi> over tiles held in shared memory
-// (sm_100a), for states of at least 2^12 amplitudes.
+// (sm_100a), for states of at least 2^12 amplitudes and all but a few terms.
 //
 // H is a sum of Z, ZZ and X terms (lambda_dev.cuh has the real-address forms). An X term
 // reads psi[r ^ delta]; done as one gather per term over the whole state that is one more
@@ -254,14 +254,29 @@ int top_bit(uint64_t x) { return 63 - __builtin_clzll(x); }
 
 }  // namespace
 
-std::vector<LamPassDev> plan_lambda(std::vector<TermDev> &terms, int m)
+// Where lambda_kernel's one gather per X term and one parity per amplitude and Z term beat the
+// tiles, whose tables, slab and barriers cost the same for one term as for many. A few Z terms
+// of 28 qubits: complex128 1 term 0.59 against 1.09 ms, 4 terms 0.65 / 1.43, 12 terms 1.47 / 1.66,
+// 16 terms 1.87 / 1.69; complex64 1 term 0.51 / 0.65, 4 terms 0.68 / 0.71, 6 terms 0.83 / 0.73.
+// One X term more is a read of the state (28 qubits complex64 0.82 / 0.44), but nothing while
+// the setup bounds both: at 16 qubits 1 X and 8 Z terms take 10 against 13 us, 3 X and 12 Z 11.5
+// and 12; at 22 qubits complex128 1 X and 4 Z 34 against 40.
+static bool gather_terms(size_t nx, size_t nd, int m, int elem_bytes)
+{
+    if (m <= 18) return nx <= 1 ? nd <= 32 : nx == 2 && nd <= 12;
+    if (nx == 0) return nd <= (elem_bytes == 8 ? 4 : 12);
+    return elem_bytes == 16 && m <= 22 && nx == 1 && nd >= 1 && nd <= 4;
+}
+
+std::vector<LamPassDev> plan_lambda(std::vector<TermDev> &terms, int m, int elem_bytes)
 {
     std::vector<LamPassDev> out;
-    if (m < kLamT) return out;  // lambda_kernel: no tile fits
+    size_t nx = 0;
+    while (nx < terms.size() && terms[nx].kind == 3) nx++;
+    if (m < kLamT || gather_terms(nx, terms.size() - nx, m, elem_bytes)) return out;
     struct Flip { uint64_t delta; double coef; };
     std::vector<Flip> flips;
-    size_t nx = 0;
-    while (nx < terms.size() && terms[nx].kind == 3) {
+    for (nx = 0; nx < terms.size() && terms[nx].kind == 3;) {
         const TermDev &t = terms[nx++];
         auto same = std::find_if(flips.begin(), flips.end(), [&](const Flip &f) { return f.delta == t.delta; });
         if (same != flips.end()) same->coef += t.coef;
