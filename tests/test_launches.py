@@ -161,3 +161,28 @@ def test_few_terms_take_the_gathers(fake):
         assert kernels(16, dtype, 16, 15) == kernels(18, dtype, 3, 0) == tile
     assert kernels(22, "complex128", 1, 4) == gather and kernels(22, "complex64", 1, 4) == tile
     """)
+
+
+def test_batches_of_few_gates(fake):
+    # complex128 batches after CX transport that one strided pass serves faster, and windows
+    # that only a strided pass can take (one pass, not a tile pass and a diagonal one)
+    run(fake, """
+    def kernels(n, dtype, gates, window):
+        s = ZXH(n, dtype=dtype)
+        g = [wl.h_all(n), wl.cx_chain(n), rc.as_records([(rc.U3, 0, 2 * q + 5, 0.3, 0.2, 0.1) for q in range(gates)])]
+        if window: g.append(rc.as_records([(rc.RZ, 0, 2 * q + 5, 0.3, 0.0, 0.0) for q in range(gates)]))
+        s.push_gates(np.concatenate(g)); launches(); s.execute()
+        return [k.split("<")[0] for _, _, k in launches()][1:]
+    tile, strided = ["affine_kernel"], ["grow_kernel"]
+    for n, gates, window, want in ((21, 4, 1, tile), (22, 1, 1, strided), (22, 4, 0, tile), (23, 2, 1, tile), (23, 3, 1, strided),
+                                   (24, 3, 0, tile), (24, 4, 0, strided), (28, 4, 0, strided), (28, 8, 0, tile)):
+        assert kernels(n, "complex128", gates, window) == want, (n, gates, window)
+        assert kernels(n, "complex64", gates, window) == tile, (n, gates, window)
+    # a CP window whose selectors flip with several coordinates of the next batch's tiles
+    g = [wl.h_all(12)]
+    for a, b, q, c, d in ((6, 7, 4, 7, 10), (10, 4, 6, 3, 10)):
+        g.append(rc.as_records([(rc.CX, a, b), (rc.U3, 0, q, 0.3, 0.2, 0.1), (rc.CP, c, d, 0.3)]))
+    s = ZXH(12); s.push_gates(np.concatenate(g)); launches(); s.execute()
+    ks = [k.split("<")[0] for _, _, k in launches()]
+    assert ks[1:] and "diag_kernel" not in ks and ks[-1] == "grow_kernel", ks
+    """)

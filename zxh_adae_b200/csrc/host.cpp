@@ -1358,6 +1358,20 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
         return true;
     };
 
+    // Whether a batch of few gates is faster as one strided pass than as one affine tile pass: in
+    // complex128 on states that L2 does not hold, where a tile's exchanges and windows (two CTAs
+    // an SM) cost more than a strided item's, from 4 gates on, 3 with a window (with fewer the
+    // strided pass's warps hold fewer rows: 28 qubits, 1 gate 1.85 against 1.55 ms; 3 gates are 4 %
+    // better or worse by their deltas). 28 qubits, 4 gates: 1.45 against 1.77 ms, with a window
+    // 1.64 / 1.95; 24 qubits, 10 batches of 3 gates and a window 1.18 / 1.41 ms. With a window any
+    // number of gates at 22 qubits, where L2 holds the state and issue bounds both: 10 batches of 2
+    // gates 0.32 / 0.37. Above 6 gates (low bits' gates ride along) not measured.
+    auto strided_is_faster = [&](const Op &op, bool window) {
+        if (elem_bytes != 16 || op.u3.size() > 6) return false;
+        if (window && op.m == 22) return true;
+        return window ? op.u3.size() >= 3 && op.m >= 23 : op.u3.size() >= 4 && op.m >= 24;
+    };
+
     for (; i < ops.size(); i++) {
         const Op &op = ops[i];
         const std::vector<DiagTerm> *wd = op.kind == Op::DIAG ? &op.diag : nullptr;  // this op's window
@@ -1675,20 +1689,38 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
             continue;
         }
         // U3BATCH with multi-bit deltas: affine tile passes (affine.cu), or general strided
-        // passes (grow.cu) for small states and while qubits are unexpanded
+        // passes (grow.cu) for small states, while qubits are unexpanded, and where one of
+        // these is faster or takes a window that no tile pass can
         if ((pp.grow || pp.grow_only) && grow_ok(op)) {
             const int mm = op.m;
             const size_t first = out.passes.size();
             const bool tiles = pp.affine && (!pp.grow_only || pp.grow_tiles) && op.deltas && mm >= kAffBits && mm <= kAffMaxBits;
+            auto take_held = [&]() {  // the pending window as the first pass's
+                Pass &p0 = out.passes[first];
+                return p0.kind == Pass::AFFINE ? p0.aff->add_window(0, *held) : p0.gb.add_window(0, *held);
+            };
             bool done = tiles && emit_affine(op);
+            bool taken = done && held && take_held();
+            const bool window = held || (i + 1 < ops.size() && ops[i + 1].kind == Op::DIAG && ops[i + 1].m == mm);
+            if (done && !pp.grow_only && ((held && !taken) || strided_is_faster(op, window))) {
+                std::vector<Pass> affine(out.passes.begin() + long(first), out.passes.end());
+                out.passes.resize(first);
+                const bool one = emit_grow(op) && out.passes.size() == first + 1 && (!held || take_held());
+                if (one) {
+                    taken = held != nullptr;
+                } else {
+                    out.passes.resize(first);
+                    out.passes.insert(out.passes.end(), affine.begin(), affine.end());
+                }
+            }
             if (!done) {
                 out.passes.resize(first);
                 done = emit_grow(op);
+                taken = done && held && take_held();
             }
             if (done) {
                 if (held) {
-                    Pass &p0 = out.passes[first];
-                    if (p0.kind == Pass::AFFINE ? p0.aff->add_window(0, *held) : p0.gb.add_window(0, *held)) {
+                    if (taken) {
                         ensure_exp();
                         out.passes[first].off2 = exp_off;
                     } else {
