@@ -178,11 +178,18 @@ def test_batches_of_few_gates(fake):
                                    (24, 3, 0, tile), (24, 4, 0, strided), (28, 4, 0, strided), (28, 8, 0, tile)):
         assert kernels(n, "complex128", gates, window) == want, (n, gates, window)
         assert kernels(n, "complex64", gates, window) == tile, (n, gates, window)
-    # a CP window whose selectors flip with several coordinates of the next batch's tiles
-    g = [wl.h_all(12)]
-    for a, b, q, c, d in ((6, 7, 4, 7, 10), (10, 4, 6, 3, 10)):
-        g.append(rc.as_records([(rc.CX, a, b), (rc.U3, 0, q, 0.3, 0.2, 0.1), (rc.CP, c, d, 0.3)]))
-    s = ZXH(12); s.push_gates(np.concatenate(g)); launches(); s.execute()
-    ks = [k.split("<")[0] for _, _, k in launches()]
-    assert ks[1:] and "diag_kernel" not in ks and ks[-1] == "grow_kernel", ks
+    # windows whose selectors flip with several coordinates of the batch's tiles, before and after
+    # it: one strided pass on small states, a diagonal pass of their own beside tiles on large ones
+    def ks(n, dtype, before, after):
+        g = [wl.h_all(n), wl.u3_layer(n, 1)]
+        if before: g.append(rc.as_records([(rc.RZ, 0, q, 0.3, 0.0, 0.0) for q in range(n)]))
+        g += [wl.cx_chain(n), rc.as_records([(rc.U3, 0, 5, 0.3, 0.2, 0.1)])]
+        if after: g += [wl.cx_chain(n), rc.as_records([(rc.RZ, 0, q, 0.3, 0.0, 0.0) for q in range(n)])]
+        s = ZXH(n, dtype=dtype); s.push_gates(np.concatenate(g)); launches(); s.execute()
+        return [k.split("<")[0] for _, _, k in launches()]
+    for dtype in ("complex64", "complex128"):
+        for before, after in ((0, 1), (1, 0), (1, 1)):
+            small, large = ks(16, dtype, before, after), ks(24, dtype, before, after)
+            assert small[-1] == "grow_kernel" and not {"affine_kernel", "diag_kernel", "walsh_kernel"} & set(small), small
+            assert "grow_kernel" not in large and "affine_kernel" in large, large
     """)

@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <deque>
+#include <functional>
 #include <cmath>
 #include <map>
 #include <memory>
@@ -1366,10 +1367,51 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
     // 1.64 / 1.95; 24 qubits, 10 batches of 3 gates and a window 1.18 / 1.41 ms. With a window any
     // number of gates at 22 qubits, where L2 holds the state and issue bounds both: 10 batches of 2
     // gates 0.32 / 0.37. Above 6 gates (low bits' gates ride along) not measured.
-    auto strided_is_faster = [&](const Op &op, bool window) {
-        if (elem_bytes != 16 || op.u3.size() > 6) return false;
-        if (window && op.m == 22) return true;
-        return window ? op.u3.size() >= 3 && op.m >= 23 : op.u3.size() >= 4 && op.m >= 24;
+    auto strided_is_faster = [&](const Op &op, const std::function<bool()> &window) {
+        const size_t k = op.u3.size();
+        if (elem_bytes != 16 || op.m < 22 || k > 6) return false;
+        if (k >= 4 && op.m >= 24) return true;
+        return (op.m == 22 || k >= 3) && window();
+    };
+
+    // Whether a window whose selectors flip with several coordinates of the batch's tiles is better
+    // taken by one strided pass in their place than by a diagonal pass of its own. The strided pass
+    // evaluates every term for every thread's few amplitudes: it saves a launch on small states, is
+    // up to 3 times as slow on large ones (24 qubits complex64, one gate beside a CP chain 1.36
+    // against 0.46 ms), and wins at any size with one CP, which is a slow diagonal pass. Its time over
+    // the pair's, one gate and
+    //   n RZ      complex64 0.94 at 14 and 16 qubits, 0.91 at 18, 1.32 at 20; complex128 0.69, 0.78, 0.86, 1.18
+    //   3 RZ      complex64 0.8 up to 18, 0.94 at 20, 1.18 at 24; complex128 0.7, 0.88, and 1.04 at 24 (2 gates 0.73)
+    //   1 CP      complex64 0.3, 0.40, 0.82 at 24 (1.12 in another circuit, 4 gates 0.7); complex128 0.4 to 0.75
+    // With four gates and n RZ complex64 0.94 at 12, 1.02 at 16; complex128 0.9 to 0.97 up to 26 qubits.
+    auto strided_takes = [&](const Op &op, const std::vector<DiagTerm> &w) {
+        const size_t k = op.u3.size(), t = w.size();
+        if (elem_bytes == 16)
+            return t <= 2 || (op.m <= 18 && k <= 4) || (t <= 3 && (op.m <= 20 || k >= 2)) || (op.m > 18 && k >= 3 && k <= 6);
+        return (t <= 2 && (op.m <= 22 || k >= 2)) || op.m <= 14 || (op.m <= 18 && (k <= 2 || t <= 3));
+    };
+    // The batch of the last pass, where that is one affine tile pass, and the window it took.
+    struct {
+        const Op *op = nullptr;
+        std::vector<DiagTerm> held;
+    } lone;
+    // The window after it, by one strided pass in its place.
+    auto strided_epilogue = [&](const std::vector<DiagTerm> &w) -> bool {
+        if (last_tile_pass < 0 || out.passes[last_tile_pass].kind != Pass::AFFINE || !lone.op || pp.grow_only ||
+            lone.op->m != m || out.passes[last_tile_pass].aff->dev.win[1].nterms || !strided_takes(*lone.op, w))
+            return false;
+        const Pass keep = out.passes.back();
+        out.passes.pop_back();
+        const size_t first = out.passes.size();
+        if (emit_grow(*lone.op) && out.passes.size() == first + 1 &&
+            (lone.held.empty() || out.passes[first].gb.add_window(0, lone.held)) && out.passes[first].gb.add_window(1, w)) {
+            ensure_exp();
+            out.passes[first].off2 = exp_off;
+            return true;
+        }
+        out.passes.resize(first);
+        out.passes.push_back(keep);
+        return false;
     };
 
     for (; i < ops.size(); i++) {
@@ -1658,6 +1700,8 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
                 last_tile_pass = -1;  // keep one epilogue window per pass
             } else if (next_u3) {
                 held = wd;
+            } else if (strided_epilogue(*wd)) {
+                last_tile_pass = -1;
             } else {
                 standalone_diag(op.m, *wd);
                 last_tile_pass = -1;
@@ -1701,8 +1745,13 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
             };
             bool done = tiles && emit_affine(op);
             bool taken = done && held && take_held();
-            const bool window = held || (i + 1 < ops.size() && ops[i + 1].kind == Op::DIAG && ops[i + 1].m == mm);
-            if (done && !pp.grow_only && ((held && !taken) || strided_is_faster(op, window))) {
+            auto window = [&]() {  // a tile pass of the batch has one
+                if (taken) return true;
+                if (i + 1 >= ops.size() || ops[i + 1].kind != Op::DIAG || ops[i + 1].m != mm) return false;
+                AffBuild last = *out.passes.back().aff;
+                return last.add_window(1, ops[i + 1].diag);
+            };
+            if (done && !pp.grow_only && (held && !taken ? strided_takes(op, *held) : strided_is_faster(op, window))) {
                 std::vector<Pass> affine(out.passes.begin() + long(first), out.passes.end());
                 out.passes.resize(first);
                 const bool one = emit_grow(op) && out.passes.size() == first + 1 && (!held || take_held());
@@ -1719,6 +1768,8 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
                 taken = done && held && take_held();
             }
             if (done) {
+                const size_t batch_passes = out.passes.size() - first;
+                const std::vector<DiagTerm> *pending = held;
                 if (held) {
                     if (taken) {
                         ensure_exp();
@@ -1732,6 +1783,9 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
                     held = nullptr;
                 }
                 last_tile_pass = int(out.passes.size()) - 1;
+                lone.op = batch_passes == 1 ? &op : nullptr;
+                lone.held.clear();
+                if (lone.op && pending && taken) lone.held = *pending;
                 m = mm;
                 continue;
             }
