@@ -193,3 +193,19 @@ def test_batches_of_few_gates(fake):
             assert small[-1] == "grow_kernel" and not {"affine_kernel", "diag_kernel", "walsh_kernel"} & set(small), small
             assert "grow_kernel" not in large and "affine_kernel" in large, large
     """)
+
+
+def test_gradients_on_a_map_that_is_not_onto(fake):
+    # CX of a qubit on itself leaves 11 pair deltas of 12 qubits, fewer than a tile needs: the
+    # sweep's gates run as strided passes, which the batch kernel has too
+    run(fake, """
+    n = 12
+    rest = [q for q in range(n) if q != 7]
+    g = rc.as_records([(rc.H, 0, q) for q in rest] + [(rc.CX, 7, 7)] + [(rc.U3, 0, q, 0.3, 0.0, 0.0) for q in rest])
+    t = rc.as_terms([(rc.TERM_Z, 0, 0, 1.0)])
+    for dtype in ("complex64", "complex128"):
+        Batch([(n, g, t)], dtype=dtype).run("persistent")
+        s = ZXH(n, dtype=dtype); s.push_gates(g); launches(); s.adjoint_gradient(t)
+        ks = {k.split("<")[0] for _, _, k in launches()}
+        assert "grow_kernel" in ks and "adj_pair_kernel" not in ks, ks
+    """)

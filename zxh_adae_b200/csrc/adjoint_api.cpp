@@ -300,8 +300,8 @@ int reverse_program(zxh_sim *s, const std::vector<size_t> &ends, AffineMap A, st
     // gates of the group collected next, so that group's pass undoes them first.
     std::vector<zxh::DiagTerm> pw;
     std::vector<uint32_t> pwk, pws;
-    auto pair_steps = [&]() {  // one global pair pass per gate
-        for (const PairGroup::G &g : pg.gates) {
+    auto pair_steps = [&](const PairGroup &grp) {  // one global pair pass per gate
+        for (const PairGroup::G &g : grp.gates) {
             RevStep p;
             p.kind = RevStep::PAIR;
             std::memset(&p.pair, 0, sizeof(p.pair));
@@ -333,6 +333,21 @@ int reverse_program(zxh_sim *s, const std::vector<size_t> &ends, AffineMap A, st
         }
         return true;
     };
+    // The gates as one general strided pass, or as pair passes; with the pending window where the
+    // pass takes it.
+    auto strided_steps = [&](const PairGroup &grp, bool with_window) -> bool {
+        std::vector<uint64_t> regs;
+        for (const PairGroup::G &g : grp.gates)
+            if (g.op.delta >> F) regs.push_back(g.op.delta);
+        RevStep r;
+        r.kind = RevStep::GROW;
+        bool ok = fuse && r.gb.init(s->elem_bytes, N, regs);
+        for (const PairGroup::G &g : grp.gates) ok = ok && r.gb.add_gate(g.op, g.gen, g.slot, true);
+        if (with_window && (!ok || !r.gb.add_window(1, pw, &pwk, &pws, true))) return false;
+        if (ok) steps.push_back(r);
+        else pair_steps(grp);
+        return true;
+    };
     auto close_group = [&]() -> int {
         if (pg.gates.empty() && pw.empty()) return ZXH_OK;
         if (tiles) {
@@ -350,33 +365,28 @@ int reverse_program(zxh_sim *s, const std::vector<size_t> &ends, AffineMap A, st
             const bool fused = ok && (pw.empty() || r.aff->add_window(0, pw, &pwk, &pws, true));
             if (!fused && !pw.empty() && !window_steps())
                 return fail(s, ZXH_ERR_STATE, "adjoint sweep: window not placeable");
-            if (ok && (fused || !pg.gates.empty())) steps.push_back(r);
-            else if (!ok) pair_steps();
+            if (ok && (fused || !pg.gates.empty())) {
+                steps.push_back(r);
+            } else if (!ok) {  // a map that is no longer onto: fewer deltas than a tile needs
+                PairGroup part;
+                for (const PairGroup::G &g : pg.gates) {
+                    if (!part.fits(g, F, R, N, maxg)) {
+                        strided_steps(part, false);
+                        part = PairGroup();
+                    }
+                    part.add(g, F);
+                }
+                if (!part.gates.empty()) strided_steps(part, false);
+            }
             pg = PairGroup();
             pw.clear();
             pwk.clear();
             pws.clear();
             return ZXH_OK;
         }
-        std::vector<uint64_t> regs;
-        for (const PairGroup::G &g : pg.gates)
-            if (g.op.delta >> F) regs.push_back(g.op.delta);
-        RevStep r;
-        r.kind = RevStep::GROW;
-        bool ok = fuse && r.gb.init(s->elem_bytes, N, regs);
-        for (const PairGroup::G &g : pg.gates) ok = ok && r.gb.add_gate(g.op, g.gen, g.slot, true);
-        if (ok && (pw.empty() || r.gb.add_window(1, pw, &pwk, &pws, true))) {
-            steps.push_back(r);
-        } else {
-            if (!pw.empty() && !window_steps()) return fail(s, ZXH_ERR_STATE, "adjoint sweep: window not placeable");
-            if (!pg.gates.empty()) {
-                RevStep r2;
-                r2.kind = RevStep::GROW;
-                bool ok2 = fuse && r2.gb.init(s->elem_bytes, N, regs);
-                for (const PairGroup::G &g : pg.gates) ok2 = ok2 && r2.gb.add_gate(g.op, g.gen, g.slot, true);
-                if (ok2) steps.push_back(r2);
-                else pair_steps();
-            }
+        if (!strided_steps(pg, !pw.empty())) {
+            if (!window_steps()) return fail(s, ZXH_ERR_STATE, "adjoint sweep: window not placeable");
+            if (!pg.gates.empty()) strided_steps(pg, false);
         }
         pg = PairGroup();
         pw.clear();
