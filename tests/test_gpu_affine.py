@@ -12,7 +12,6 @@ from oracle import observables as ob
 from oracle.bridge import Oracle
 from zxh_adae_b200 import ZXH, workloads
 from zxh_adae_b200 import adjoint as ad
-from zxh_adae_b200._core import plan_stats
 from zxh_adae_b200.records import CP, CX, H, P, RX, RZ, U3, X, Z, as_records
 
 pytestmark = pytest.mark.gpu
@@ -60,7 +59,6 @@ def circuit(n, links, gates, window, seed, layers=4):
                                            (14, "chain", "h"), (15, "random", "complex"), (16, "back", "real")])
 def test_affine_passes_against_oracle(n, links, gates, window, dtype):
     g = circuit(n, links, gates, window, seed=n)
-    assert plan_stats(n, g, dtype=dtype)["grow"] > 0
     o = Oracle(n)
     o.push(g)
     o.execute()
@@ -93,7 +91,7 @@ def test_affine_layers_applied_one_by_one(dtype):
     s.close()
 
 
-def ansatz(n, links, window, seed):
+def ansatz(n, links, window, seed, layers=3):
     rng = np.random.default_rng(seed)
     recs, par = [], []
 
@@ -101,7 +99,7 @@ def ansatz(n, links, window, seed):
         recs.append(rec)
         par.append(sum(p >= 0 for p in par) if parameter else -1)
 
-    for _ in range(3):
+    for _ in range(layers):
         for q in rng.permutation(n):
             add((U3, 0, int(q), 0.0, 0.0, 0.0) if rng.random() < 0.7 else (RX, 0, int(q), 0.0), True)
         add((H, 0, int(rng.integers(n))), False)
@@ -135,10 +133,12 @@ def test_affine_gradients_against_dense_adjoint(n, links, window, dtype):
     s.push_gates(circ.records(p))
     # energies and gradients are sums of 2 n unit terms of the state's relative error
     tol = 2 * n * (1e-12 if dtype == "complex128" else 1e-6)
-    for every in (0, 7):
-        e, g = s.adjoint_gradient(terms, every)
-        assert abs(e - e_ref) <= tol
-        assert np.max(np.abs(g - g_ref)) <= tol
+    for affine in (0, 1):
+        s.set_param("affine", affine)
+        for every in (0, 7):
+            e, g = s.adjoint_gradient(terms, every)
+            assert abs(e - e_ref) <= tol, affine
+            assert np.max(np.abs(g - g_ref)) <= tol, affine
     want = ob.oracle_state(n, circ.records(p))
     assert np.max(np.abs(ob.qubit_order(s.get_state(), n) - want)) <= TOL[dtype]  # the forward output stays
     s.close()
@@ -230,3 +230,75 @@ def test_first_layer_on_expanded_qubits(n):
             s.execute()
             assert np.max(np.abs(s.get_state(0).astype(np.complex128) - o.get_state(0))) <= TOL[dtype]
             s.close()
+
+
+# 2^22 amplitudes are 1024 tiles, on two or three CTAs an SM (296 or 444 on 148 SMs, 148 for the
+# complex128 adjoint): every CTA takes several. Against the strided passes, whose own error has
+# the same bound.
+SEVERAL = 22
+
+
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+@pytest.mark.parametrize("links,window", [("random", "dense"), ("chain", "chain"), ("back", "linear")])
+@pytest.mark.parametrize("gates", ["complex", "real", "h"])
+def test_affine_ctas_with_several_tiles(gates, links, window, dtype):
+    g = circuit(SEVERAL, links, gates, window, seed=3, layers=2)
+    states = []
+    for affine in (0, 1):
+        s = ZXH(SEVERAL, dtype=dtype)
+        s.set_param("affine", affine)
+        s.push_gates(g)
+        s.execute()
+        states.append(s.get_state(0))
+        s.close()
+    assert np.max(np.abs(states[0].astype(np.complex128) - states[1])) <= 2 * TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+@pytest.mark.parametrize("links,window", [("random", "dense"), ("chain", "linear")])
+@pytest.mark.parametrize("form", ["complex", "real", "rotations"])
+def test_adjoint_ctas_with_several_tiles(form, links, window, dtype):
+    # RX by an angle is complex, by zero real but not taken as a rotation (its generator is X)
+    n = SEVERAL
+    circ = ansatz(n, links, window, seed=5, layers=2)
+    recs = circ.records(np.random.default_rng(n).uniform(-math.pi, math.pi, circ.nparams))
+    rx = recs["type"] == RX
+    if form == "real":
+        recs["theta"][rx] = 0.0
+    elif form == "rotations":
+        recs["type"][rx] = U3
+    terms = ad.tfim_terms(n, h=0.6)
+    tol = 2 * 2 * n * (1e-12 if dtype == "complex128" else 1e-6)
+    s = ZXH(n, dtype=dtype)
+    s.push_gates(recs)
+    s.set_param("affine", 0)
+    e_ref, g_ref = s.adjoint_gradient(terms)
+    s.set_param("affine", 1)
+    for every in (0, 20):
+        e, g = s.adjoint_gradient(terms, every)
+        assert abs(e - e_ref) <= tol and np.max(np.abs(g - g_ref)) <= tol, every
+    s.close()
+
+
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+def test_batch_tasks_of_several_tiles(dtype):
+    # a queue whose levels are one circuit's 1024 tiles, in tasks of 3 or 4: a real queue, and one with
+    # complex gates and CX chains
+    from zxh_adae_b200.batch import Batch
+
+    n = SEVERAL
+    real = workloads.batch_tfim(1, n, n, n, 2)[0][:3]
+    c = ansatz(n, "chain", "dense", seed=7, layers=2)
+    mixed = (n, c.records(np.random.default_rng(7).uniform(-math.pi, math.pi, c.nparams)), ad.tfim_terms(n))
+    tol = 2 * 2 * n * (1e-12 if dtype == "complex128" else 1e-6)
+    for which in (real, mixed):
+        s = ZXH(n, dtype=dtype)
+        s.set_param("affine", 0)
+        s.push_gates(which[1])
+        e_ref, g_ref = s.adjoint_gradient(which[2])
+        s.close()
+        b = Batch([which], dtype=dtype)
+        for mode in ("persistent", "graph"):
+            e, g = b.run(mode)
+            assert abs(e[0] - e_ref) <= tol and np.max(np.abs(b.gradients(g)[0] - g_ref)) <= tol, mode
+        b.close()

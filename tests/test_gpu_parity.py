@@ -130,6 +130,7 @@ def test_general_strided_pass_after_cx_transport(dtype, n, seed):
     assert max_err(s2, o) <= TOL[dtype]
     for staged in (0, 7):  # rows loaded straight into registers / staged one item ahead in shared memory
         s3 = zx.ZXH(n, dtype=dtype)
+        s3.set_param("affine", 0)  # tile passes have no staged form
         s3.set_param("grow_staged", staged)
         s3.push_gates(gates)
         s3.execute()
@@ -589,19 +590,21 @@ def _mixed_case(n, seed):
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_u3_batches_mixing_single_and_multi_bit_deltas(n, mixed, dtype):
     # knob span_mixed: the single-bit gates of a mixed batch run as span passes
-    # first, the others as general strided passes after them (1), or the whole
-    # batch as general strided passes (0)
+    # first, the others as affine tile or general strided passes after them (1), or the
+    # whole batch as such (0)
     gates = _mixed_case(n, 900 + n)
     st = plan_stats(n, gates, dtype=dtype)
     assert st["span"] > 0 and st["grow"] > 0
     o = Oracle(n)
     o.push(gates)
     o.execute()
-    s = zx.ZXH(n, dtype=dtype)
-    s.set_param("span_mixed", mixed)
-    s.push_gates(gates)
-    s.execute()
-    assert max_err(s, o) <= TOL[dtype]
+    for affine in (1, 0):  # the others as affine tile passes or as strided passes
+        s = zx.ZXH(n, dtype=dtype)
+        s.set_param("span_mixed", mixed)
+        s.set_param("affine", affine)
+        s.push_gates(gates)
+        s.execute()
+        assert max_err(s, o) <= TOL[dtype], affine
 
 
 @pytest.mark.parametrize("dtype", DTYPES)

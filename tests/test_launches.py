@@ -209,3 +209,27 @@ def test_gradients_on_a_map_that_is_not_onto(fake):
         ks = {k.split("<")[0] for _, _, k in launches()}
         assert "grow_kernel" in ks and "adj_pair_kernel" not in ks, ks
     """)
+
+
+def test_the_affine_tests_run_affine_passes(fake):
+    # the circuits of test_gpu_affine.py: tile passes forward and in the sweep, none with affine = 0
+    run(fake, """
+    from tests.test_gpu_affine import ansatz, circuit, SEVERAL
+    def kinds(n, g, affine, grad=False):
+        s = ZXH(n); s.set_param("affine", affine); s.push_gates(g); launches()
+        s.adjoint_gradient(ad.tfim_terms(n)) if grad else s.execute()
+        ks = launches()
+        tiles = [grid for _, grid, k in ks if k.startswith("affine_kernel")]
+        return tiles, sum(k.startswith("grow_kernel") for _, _, k in ks)
+    for n, links, gates in [(12, "chain", "complex"), (12, "random", "real"), (13, "back", "complex"), (14, "chain", "h"),
+                            (15, "random", "complex"), (16, "back", "real"), (SEVERAL, "random", "h")]:
+        for window in ("none", "linear", "chain", "dense"):
+            g = circuit(n, links, gates, window, seed=n)
+            tiles, strided = kinds(n, g, 1)
+            assert tiles and max(tiles) <= 1 << (n - 12), (n, links, gates, window)
+            assert n < SEVERAL or 2 * max(tiles) < 1 << (n - 12)  # several tiles a CTA
+            assert kinds(n, g, 0)[0] == [] and kinds(n, g, 0)[1] > 0
+    for n, links, window in [(12, "chain", "linear"), (15, "chain", "dense")]:
+        g = ansatz(n, links, window, n).records(np.zeros(ansatz(n, links, window, n).nparams))
+        assert len(kinds(n, g, 1, True)[0]) > 3 and kinds(n, g, 0, True)[0] == []
+    """)
