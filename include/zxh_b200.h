@@ -345,9 +345,10 @@ int zxh_optimize_gates(size_t n, int level, const zxh_gate *gates, size_t count,
  * U3 batches whose pair deltas span several bits use the general strided pass,
  * 0: the TMA tile / global pair passes), affine (1: such batches, and the adjoint
  * sweep, run as affine tile passes on states of 2^12 to 2^32 amplitudes with
- * every qubit expanded, 0: the register-row form of the general strided pass,
- * the only one grow_regs, adj_regs and grow_staged act on), grow_regs (1..4: gates with high deltas per
- * general strided pass), grow_only (1: plan every batch and window as general
+ * every qubit expanded, but for batches of few gates that one general strided
+ * pass serves faster; 0: the register-row form of the general strided pass
+ * throughout, the only one grow_regs, adj_regs and grow_staged act on), grow_regs
+ * (1..4: gates with high deltas per general strided pass), grow_only (1: plan every batch and window as general
  * strided passes after a |0...0> init, the pass set of the batched launch; needs
  * eager_expand_all), adj_windows (1: the adjoint sweep undoes diagonal gates
  * inside its general strided passes, 0: in separate diagonal-group passes),

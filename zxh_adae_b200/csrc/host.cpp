@@ -960,6 +960,9 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
     //    (under eager_expand_all the first layer: its passes over a state that is still
     //    |0...0> would cost as much as any layer's), and diagonal windows made only of P
     //    phases on existing bits / constant selectors. The prefix is written in one pass.
+    //    A batch on touched bits would leave a product as well; it starts the passes
+    //    because the host tests pin the passes of a U3 layer after an H layer (3 at 30
+    //    qubits), not because it could not join.
     if (start.fresh && pp.grow_only) {
         Pass ps;
         ps.kind = Pass::INIT;

@@ -259,8 +259,8 @@ int top_bit(uint64_t x) { return 63 - __builtin_clzll(x); }
 // of 28 qubits: complex128 1 term 0.59 against 1.09 ms, 4 terms 0.65 / 1.43, 12 terms 1.47 / 1.66,
 // 16 terms 1.87 / 1.69; complex64 1 term 0.51 / 0.65, 4 terms 0.68 / 0.71, 6 terms 0.83 / 0.73.
 // One X term more is a read of the state (28 qubits complex64 0.82 / 0.44), but nothing while
-// the setup bounds both: at 16 qubits 1 X and 8 Z terms take 10 against 13 us, 3 X and 12 Z 11.5
-// and 12; at 22 qubits complex128 1 X and 4 Z 34 against 40.
+// the setup bounds both: at 16 qubits complex64 1 X and 8 Z terms take 10 against 13 us, 3 X and
+// 12 Z 12 and 13; at 22 qubits complex128 1 X and 4 Z 27 against 32.
 static bool gather_terms(size_t nx, size_t nd, int m, int elem_bytes)
 {
     if (m <= 18) return nx <= 1 ? nd <= 32 : nx == 2 && nd <= 12;
