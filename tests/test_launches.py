@@ -233,3 +233,20 @@ def test_the_affine_tests_run_affine_passes(fake):
         g = ansatz(n, links, window, n).records(np.zeros(ansatz(n, links, window, n).nparams))
         assert len(kinds(n, g, 1, True)[0]) > 3 and kinds(n, g, 0, True)[0] == []
     """)
+
+
+def test_forms_of_real_gates(fake):
+    # after CX transport: rotations, H and their products run with a factored coefficient in both
+    # types; a phase of 1e-16 makes a complex128 gate complex
+    run(fake, """
+    def form(dtype, *gates):
+        g = np.concatenate([wl.h_all(13), wl.cx_chain(13)] + [rc.as_records([(*x[:1], 0, q, *x[1:]) for q in range(13)]) for x in gates])
+        s = ZXH(13, dtype=dtype); s.push_gates(g); launches(); s.execute()
+        return {k.split(", ")[2][0] for _, _, k in launches() if k.startswith("affine")}
+    ry, h = (rc.U3, 0.3, 0.0, 0.0), (rc.H,)
+    for dtype in ("complex64", "complex128"):
+        for gates in ((ry,), (h,), (ry, ry), (h, ry), (ry, h, ry, h, ry), ((rc.U3, np.pi / 2, np.pi, 0.0), ry)):
+            assert form(dtype, *gates) == {"2"}, (dtype, gates)
+        assert form(dtype, ry, (rc.U3, 0.3, 0.2, 0.1)) == {"0"}
+    assert form("complex128", (rc.U3, 0.3, 1e-16, 0.0)) == {"0"} and form("complex64", (rc.U3, 0.3, 1e-16, 0.0)) == {"2"}
+    """)

@@ -468,6 +468,7 @@ int reverse_program(zxh_sim *s, const std::vector<size_t> &ends, AffineMap A, st
             pgt.op.sel = A.selector(int(g.q));
             if (g.type == zxh::G_H) zxh::u3_matrix(kPi / 2.0, kPi, 0.0, pgt.op.u);
             else zxh::u3_matrix(g.theta, g.lambda, g.phi, pgt.op.u);
+            pgt.op.real = zxh::real_factor(pgt.op.u);
             pgt.gen = pair_generator(g);
             pgt.slot = uint32_t(gi);
             pgt.q = int(g.q);

@@ -20,17 +20,6 @@ uint64_t reduced(uint64_t v, const std::vector<uint64_t> &ech)
     return v;
 }
 
-// H as u3_matrix rounds it: exp(i pi) leaves imaginary parts of 8.7e-17 that the gate has not.
-bool is_h(const cd u[4])
-{
-    static const std::vector<cd> h = [] {
-        std::vector<cd> m(4);
-        u3_matrix(std::acos(-1.0) / 2.0, std::acos(-1.0), 0.0, m.data());
-        return m;
-    }();
-    return std::equal(h.begin(), h.end(), u);
-}
-
 void insert(uint64_t v, std::vector<uint64_t> &ech)
 {
     ech.push_back(v);
@@ -69,9 +58,9 @@ bool AffBuild::init(int eb, int mm, const std::vector<U3Op> &gates, const std::v
     }
     form = 2;
     dev.scale = 1.0;
-    // What a matrix may miss its form by. complex128 takes exact forms and H only: a phase of
-    // 1e-15 dropped from every gate of a deep circuit adds up. In complex64 the amplitudes
-    // round at 6e-8, and products of H with rotations keep their form.
+    // What a matrix may miss its form by, but for what is known to be real. Nothing in
+    // complex128: a phase of 1e-15 dropped from every gate of a deep circuit adds up. In
+    // complex64 the amplitudes round at 6e-8.
     const double round = elem_bytes == 8 ? 1e-15 : 0.0;
     if (m < kAffBits || m > kAffMaxBits) return false;
     dev.m = uint32_t(m);
@@ -130,7 +119,7 @@ bool AffBuild::init(int eb, int mm, const std::vector<U3Op> &gates, const std::v
             w[2] = std::conj(g.u[1]);
             w[3] = std::conj(g.u[3]);
         }
-        if (is_h(g.u))
+        if (g.real)
             for (cd &x : w) x = x.real();
         for (int q = 0; q < 4; q++) {
             d.u[2 * q] = w[q].real();

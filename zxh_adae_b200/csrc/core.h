@@ -95,6 +95,7 @@ struct U3Op {
     uint64_t delta = 0;
     Sel sel;            // pair (i, i^delta) with S(i) == 0 is "even"
     cd u[4];            // u00, u01, u10, u11
+    bool real = false;  // a product of real matrices (real_factor): imaginary parts are rounding
     bool has_ctrl = false;
     Sel ctrl;           // explicit CX: act only where ctrl(i) == 1
 };

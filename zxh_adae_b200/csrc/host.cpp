@@ -7,6 +7,7 @@
 #include "host.h"
 
 #include <algorithm>
+#include <array>
 #include <deque>
 #include <functional>
 #include <cmath>
@@ -124,8 +125,24 @@ void build_u3(double th, double la, double ph, cd u[4])
     u[3] = epl * c;
 }
 
+}  // namespace
+
+bool real_factor(const cd u[4])
+{
+    static const std::array<cd, 4> h = [] {
+        std::array<cd, 4> m;
+        build_u3(kPi / 2.0, kPi, 0.0, m.data());
+        return m;
+    }();
+    return (u[0].imag() == 0.0 && u[1].imag() == 0.0 && u[2].imag() == 0.0 && u[3].imag() == 0.0) ||
+           std::equal(h.begin(), h.end(), u);
+}
+
+namespace {
+
 struct Acc {
     bool active = false;
+    bool real = true;  // every factor is real (real_factor)
     cd u[4] = {cd(1, 0), cd(0, 0), cd(0, 0), cd(1, 0)};
 };
 
@@ -140,6 +157,7 @@ bool is_identity(const Acc &a)
 void acc_reset(Acc &a)
 {
     a.active = false;
+    a.real = true;
     a.u[0] = cd(1, 0);
     a.u[1] = cd(0, 0);
     a.u[2] = cd(0, 0);
@@ -154,6 +172,7 @@ void left_mul(Acc &a, const cd n[4])
     a.u[1] = n[0] * o01 + n[1] * o11;
     a.u[2] = n[2] * o00 + n[3] * o10;
     a.u[3] = n[2] * o01 + n[3] * o11;
+    a.real = a.real && real_factor(n);
     a.active = !is_identity(a);
 }
 
@@ -201,6 +220,7 @@ int walk(const Gate *gates, size_t count, bool disable_x, int M, WalkState &ws, 
             u.delta &= low_mask(ws.m);
             u.sel = A.selector(q);
             for (int k = 0; k < 4; k++) u.u[k] = pend[q].u[k];
+            u.real = pend[q].real;
             op.u3.push_back(u);
         }
         for (int q = 0; q < N; q++) acc_reset(pend[q]);

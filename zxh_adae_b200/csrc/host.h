@@ -23,6 +23,9 @@ int walk(const Gate *gates, size_t count, bool disable_x, int M, WalkState &ws, 
 // U3(theta, lambda, phi) as the walk builds it (build_u3_matrix, zxh.cpp:101-113):
 // u00, u01, u10, u11.
 void u3_matrix(double theta, double lambda, double phi, cd u[4]);
+// Whether a gate's matrix is real: exactly, or H as u3_matrix rounds it (exp(i pi) leaves
+// imaginary parts of 8.7e-17 that the gate has not).
+bool real_factor(const cd u[4]);
 
 // theta / (2 pi) as a 64-bit fixed-point fraction of a turn (wraps modulo 2^64).
 int64_t phase_turns(double theta);
