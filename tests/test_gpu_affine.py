@@ -302,3 +302,51 @@ def test_batch_tasks_of_several_tiles(dtype):
             e, g = b.run(mode)
             assert abs(e[0] - e_ref) <= tol and np.max(np.abs(b.gradients(g)[0] - g_ref)) <= tol, mode
         b.close()
+
+
+def few_gates(n, gates, before, after, seed):
+    # a U3 layer, a window, CX, a few U3, their window, CX, a window in another map
+    rng = np.random.default_rng(seed)
+
+    def window(terms):
+        recs = [(RZ, 0, int(q), rng.uniform(0, 6)) for q in rng.permutation(n)[:terms]]
+        return as_records(recs + [(CP, int(a), int(b), rng.uniform(0, 6)) for a, b in rng.integers(0, n, (terms, 2))])
+
+    u3 = [(U3, 0, int(q), *rng.uniform(0, 6, 3)) for q in rng.permutation(n)[:gates]]
+    parts = [workloads.h_all(n), workloads.u3_layer(n, seed), window(before), workloads.cx_chain(n), as_records(u3),
+             as_records([(RZ, 0, q, rng.uniform(0, 6)) for _, _, q, *_ in u3]), workloads.cx_chain(n), window(after)]
+    return np.concatenate([p for p in parts if len(p)])
+
+
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+@pytest.mark.parametrize("n", [12, 14, 15, 18])
+def test_few_gates_beside_windows(n, dtype):
+    # batches that fit one strided pass, beside windows that no tile pass takes: both sides of the
+    # lines between one strided pass and a tile pass with a diagonal one
+    for gates in (1, 2, 3, 5):
+        for before, after in ((1, 0), (0, 1), (3, 2), (n, 0), (0, n)):
+            g = few_gates(n, gates, before, after, seed=n + gates)
+            o = Oracle(n)
+            o.push(g)
+            o.execute()
+            s = ZXH(n, dtype=dtype)
+            s.push_gates(g)
+            s.execute()
+            assert np.max(np.abs(s.get_state(0).astype(np.complex128) - o.get_state(0))) <= TOL[dtype], (gates, before, after)
+            s.close()
+
+
+@pytest.mark.parametrize("n", [22, 23, 24])
+def test_few_complex128_gates_on_large_states(n):
+    for gates in (1, 3, 4, 7):
+        for before, after in ((0, 0), (2, 2)):
+            g = few_gates(n, gates, before, after, seed=n + gates)
+            states = []
+            for affine in (0, 1):
+                s = ZXH(n, dtype="complex128")
+                s.set_param("affine", affine)
+                s.push_gates(g)
+                s.execute()
+                states.append(s.get_state(0))
+                s.close()
+            assert np.max(np.abs(states[0] - states[1])) <= 2 * TOL["complex128"], (gates, before, after)

@@ -633,3 +633,19 @@ def test_span_pass_through_apply_round_trip(dtype):
     st = torch.as_tensor(_CAI(), device="cuda").to(torch.complex128) * complex(g)
     want = 2.0 ** (-n / 2)
     assert float((st - want).abs().max()) < TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_window_on_a_single_amplitude(dtype):
+    # X alone expands no qubit: the state is one amplitude, and the window a phase on it
+    n = 4
+    parts = [zx.as_records([(zx._core.X, 0, 1), (zx._core.X, 0, 3)]),
+             zx.as_records([(zx._core.P, 0, 1, 0.3), (zx._core.CP, 1, 3, 0.7), (zx._core.RZ, 0, 0, 0.2), (zx._core.P, 0, 2, 0.9)])]
+    o = Oracle(n)
+    o.push(np.concatenate(parts))
+    o.execute()
+    s = zx.ZXH(n, dtype=dtype)
+    s.push_gates(parts[0])
+    s.execute()
+    s.apply(parts[1])
+    assert max_err(s, o) <= TOL[dtype]

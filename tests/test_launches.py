@@ -250,3 +250,17 @@ def test_forms_of_real_gates(fake):
         assert form(dtype, ry, (rc.U3, 0.3, 0.2, 0.1)) == {"0"}
     assert form("complex128", (rc.U3, 0.3, 1e-16, 0.0)) == {"0"} and form("complex64", (rc.U3, 0.3, 1e-16, 0.0)) == {"2"}
     """)
+
+
+def test_windows_on_a_single_amplitude(fake):
+    # no qubit expanded: 8 bytes of complex64 state, below the 16 of a bulk copy
+    run(fake, """
+    for dtype, n in (("complex64", 0), ("complex64", 1), ("complex128", 0)):
+        s = ZXH(4, dtype=dtype)
+        s.push_gates(rc.as_records([(rc.X, 0, 1)] + [(rc.H, 0, 2)] * n)); s.execute(); launches()
+        assert s.state_view()[1] == n
+        s.apply(rc.as_records([(rc.P, 0, 1, 0.3, 0.0, 0.0), (rc.CP, 1, 0, 0.3, 0.0, 0.0)])); s.flush()
+        (k,) = [k for _, _, k in launches() if k.startswith("diag_kernel")]
+        staged = k.split(", ")[2] == "true"
+        assert staged == (dtype == "complex64" and n == 1), k
+    """)

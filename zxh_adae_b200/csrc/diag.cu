@@ -423,6 +423,9 @@ cudaError_t launch_diag_pf(const uint8_t *dblob, uint64_t doff, uint64_t toff, i
                            E *state, DevStatus *status, int sms, cudaStream_t st)
 {
     const bool full = m >= (ET<E>::V == 2 ? 6 : 5) + ROWB;
+    // a bulk copy moves whole 16 bytes: one complex64 amplitude (no qubit expanded yet) is read
+    // and written directly, as half of a vector (states are allocated with at least 256 bytes)
+    pf = pf && (size_t(sizeof(E)) << m) >= 16;
     if (full)
         return pf ? launch_diag<E, ROWB, true, true>(dblob, doff, toff, m, chunk_bits, state, status, sms, st)
                   : launch_diag<E, ROWB, false, true>(dblob, doff, toff, m, chunk_bits, state, status, sms, st);

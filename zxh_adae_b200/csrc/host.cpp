@@ -1420,7 +1420,8 @@ int plan(const std::vector<Op> &ops_in, int elem_bytes, const PlanParams &pp, co
     } lone;
     // The window after it, by one strided pass in its place.
     auto strided_epilogue = [&](const std::vector<DiagTerm> &w) -> bool {
-        if (last_tile_pass < 0 || out.passes[last_tile_pass].kind != Pass::AFFINE || !lone.op || pp.grow_only ||
+        if (last_tile_pass < 0 || last_tile_pass + 1 != int(out.passes.size()) ||
+            out.passes[last_tile_pass].kind != Pass::AFFINE || !lone.op || pp.grow_only ||
             lone.op->m != m || out.passes[last_tile_pass].aff->dev.win[1].nterms || !strided_takes(*lone.op, w))
             return false;
         const Pass keep = out.passes.back();
