@@ -254,19 +254,25 @@ def test_affine_ctas_with_several_tiles(gates, links, window, dtype):
     assert np.max(np.abs(states[0].astype(np.complex128) - states[1])) <= 2 * TOL[dtype]
 
 
+def formed(n, links, window, form):
+    circ = ansatz(n, links, window, seed=5, layers=2)
+    recs = circ.records(np.random.default_rng(n).uniform(-math.pi, math.pi, circ.nparams))
+    rx = (recs["type"] == U3) & (recs["lam"] != 0.0)
+    assert rx.any()
+    if form == "real":
+        recs["theta"][rx] = 0.0
+    elif form == "rotations":
+        recs["lam"][rx] = recs["phi"][rx] = 0.0
+    return recs
+
+
 @pytest.mark.parametrize("dtype", ["complex64", "complex128"])
 @pytest.mark.parametrize("links,window", [("random", "dense"), ("chain", "linear")])
 @pytest.mark.parametrize("form", ["complex", "real", "rotations"])
 def test_adjoint_ctas_with_several_tiles(form, links, window, dtype):
     # RX by an angle is complex, by zero real but not taken as a rotation (its generator is X)
     n = SEVERAL
-    circ = ansatz(n, links, window, seed=5, layers=2)
-    recs = circ.records(np.random.default_rng(n).uniform(-math.pi, math.pi, circ.nparams))
-    rx = recs["type"] == RX
-    if form == "real":
-        recs["theta"][rx] = 0.0
-    elif form == "rotations":
-        recs["type"][rx] = U3
+    recs = formed(n, links, window, form)
     terms = ad.tfim_terms(n, h=0.6)
     tol = 2 * 2 * n * (1e-12 if dtype == "complex128" else 1e-6)
     s = ZXH(n, dtype=dtype)

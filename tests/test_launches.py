@@ -214,7 +214,7 @@ def test_gradients_on_a_map_that_is_not_onto(fake):
 def test_the_affine_tests_run_affine_passes(fake):
     # the circuits of test_gpu_affine.py: tile passes forward and in the sweep, none with affine = 0
     run(fake, """
-    from tests.test_gpu_affine import ansatz, circuit, SEVERAL
+    from tests.test_gpu_affine import ansatz, circuit, formed, SEVERAL
     def kinds(n, g, affine, grad=False):
         s = ZXH(n); s.set_param("affine", affine); s.push_gates(g); launches()
         s.adjoint_gradient(ad.tfim_terms(n)) if grad else s.execute()
@@ -232,6 +232,12 @@ def test_the_affine_tests_run_affine_passes(fake):
     for n, links, window in [(12, "chain", "linear"), (15, "chain", "dense")]:
         g = ansatz(n, links, window, n).records(np.zeros(ansatz(n, links, window, n).nparams))
         assert len(kinds(n, g, 1, True)[0]) > 3 and kinds(n, g, 0, True)[0] == []
+    for form, want in (("complex", "0"), ("real", "1"), ("rotations", "2")):
+        for dtype in ("complex64", "complex128"):
+            s = ZXH(SEVERAL, dtype=dtype); s.push_gates(formed(SEVERAL, "chain", "linear", form)); launches()
+            s.adjoint_gradient(ad.tfim_terms(SEVERAL))
+            sweep = {k.split(", ")[2][0] for _, _, k in launches() if k.startswith("affine_kernel") and ", true, " in k}
+            assert want in sweep and min(sweep) == want, (form, dtype, sweep)
     """)
 
 
