@@ -287,30 +287,25 @@ cudaError_t persistent_threads(int threads, bool wide, const uint8_t *blob, cons
     }
 }
 
+}  // namespace
+
 template <typename E>
-cudaError_t persistent_real(bool real, int threads, bool wide, const uint8_t *blob, const BatchOp *ops, const BatchTask *tasks,
-                            uint32_t ntasks, uint32_t *next, uint32_t *remaining, E *arena, double *grads,
-                            double *energies, DevStatus *status, long long spin_limit, int sms, cudaStream_t st)
+cudaError_t run_batch_persistent(const uint8_t *blob, const BatchOp *ops, const BatchTask *tasks, uint32_t ntasks,
+                                 uint32_t *next, uint32_t *remaining, void *arena, double *grads, double *energies,
+                                 DevStatus *status, bool real, int threads, bool wide, int wait_limit_log2, int sms,
+                                 cudaStream_t st)
 {
-    return real ? persistent_threads<E, true>(threads, wide, blob, ops, tasks, ntasks, next, remaining, arena, grads,
+    const long long spin_limit = 1LL << wait_limit_log2;
+    auto *states = static_cast<E *>(arena);
+    return real ? persistent_threads<E, true>(threads, wide, blob, ops, tasks, ntasks, next, remaining, states, grads,
                                               energies, status, spin_limit, sms, st)
-                : persistent_threads<E, false>(threads, wide, blob, ops, tasks, ntasks, next, remaining, arena, grads,
+                : persistent_threads<E, false>(threads, wide, blob, ops, tasks, ntasks, next, remaining, states, grads,
                                                energies, status, spin_limit, sms, st);
 }
 
-}  // namespace
-
-cudaError_t run_batch_persistent(const uint8_t *blob, const BatchOp *ops, const BatchTask *tasks, uint32_t ntasks,
-                                 uint32_t *next, uint32_t *remaining, void *arena, double *grads, double *energies,
-                                 DevStatus *status, int elem_bytes, bool real, int threads, bool wide, int wait_limit_log2,
-                                 int sms, cudaStream_t st)
-{
-    const long long spin_limit = 1LL << wait_limit_log2;
-    if (elem_bytes == 8)
-        return persistent_real(real, threads, wide, blob, ops, tasks, ntasks, next, remaining, static_cast<float2 *>(arena),
-                               grads, energies, status, spin_limit, sms, st);
-    return persistent_real(real, threads, wide, blob, ops, tasks, ntasks, next, remaining, static_cast<double2 *>(arena),
-                           grads, energies, status, spin_limit, sms, st);
-}
+// One element type per object file: the sixteen kernels take six minutes in one.
+template cudaError_t run_batch_persistent<ZXH_BATCH_ELEM>(const uint8_t *, const BatchOp *, const BatchTask *, uint32_t,
+                                                          uint32_t *, uint32_t *, void *, double *, double *, DevStatus *,
+                                                          bool, int, bool, int, int, cudaStream_t);
 
 }  // namespace zxh

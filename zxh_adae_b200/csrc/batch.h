@@ -50,9 +50,10 @@ struct BatchTask {
 // affine tile passes (256 threads only), for queues that hold some. A task waits at most
 // 2^wait_limit_log2 SM clocks for its op's predecessor; then it records a timeout
 // in the status word and its CTA ends.
+template <typename E>  // float2 or double2: the states' elements
 cudaError_t run_batch_persistent(const uint8_t *blob, const BatchOp *ops, const BatchTask *tasks, uint32_t ntasks,
                                  uint32_t *next, uint32_t *remaining, void *arena, double *grads, double *energies,
-                                 DevStatus *status, int elem_bytes, bool real, int threads, bool wide, int wait_limit_log2,
-                                 int sms, cudaStream_t st);
+                                 DevStatus *status, bool real, int threads, bool wide, int wait_limit_log2, int sms,
+                                 cudaStream_t st);
 
 }  // namespace zxh

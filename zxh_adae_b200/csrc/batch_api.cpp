@@ -370,9 +370,9 @@ int enqueue_persistent(zxh_batch *b)
     BCK(b, cudaMemcpyAsync(b->d_rem, b->d_rem_init, b->ops.size() * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
                            b->stream),
         "reset counters");
-    BCK(b, zxh::run_batch_persistent(b->d_blob, b->d_ops, b->d_tasks, uint32_t(b->tasks.size()), b->d_next, b->d_rem,
-                                     b->d_arena, b->d_grads, b->d_energy, b->d_status, b->eb, b->real,
-                                     b->threads, b->wide, b->wait_limit_log2, b->sms, b->stream),
+    auto run = b->eb == 8 ? &zxh::run_batch_persistent<float2> : &zxh::run_batch_persistent<double2>;
+    BCK(b, run(b->d_blob, b->d_ops, b->d_tasks, uint32_t(b->tasks.size()), b->d_next, b->d_rem, b->d_arena, b->d_grads,
+               b->d_energy, b->d_status, b->real, b->threads, b->wide, b->wait_limit_log2, b->sms, b->stream),
         "batch launch");
     return ZXH_OK;
 }
